@@ -48,6 +48,53 @@ def test_batched_posv(gpu):
         np.testing.assert_allclose(L, np.linalg.cholesky(a0s[i]), rtol=1e-10, atol=1e-12)
 
 
+@pytest.mark.parametrize("nrhs", [0, 1, 8, 9, 20])
+def test_batched_posv_tile_edges(gpu, nrhs):
+    """Orders at the edges of the 16 x 16 tiles and of the size buckets, leading
+    dimensions above the order, right-hand sides across the block rows of
+    eight; nothing outside the lower triangle and B's n rows is written.
+    Bounds: |A - L L^T| <= (n + 1) u |L||L^T| and the solve's residual
+    (3 n + 1) u |L||L^T||x| componentwise (Higham, Accuracy and Stability,
+    theorems 10.3 and 10.4), u = 2^-53, doubled for the reciprocal diagonal."""
+    import torch
+    rng = np.random.default_rng(nrhs)
+    ns = [1, 2, 15, 16, 17, 33, 48, 49, 112, 113, 176, 177, 240, 255, 256, 0]
+    u = 2.0 ** -53
+    As, Bs, a0s, b0s, lda, ldb = [], [], [], [], [], []
+    for n in ns:
+        la, lb = n + 3, n + 5
+        g = rng.standard_normal((n, n))
+        a = np.full((max(n, 1), la), 7.0)             # row = column of the matrix
+        a[:n, :n] = g @ g.T + n * np.eye(n)
+        b = np.full((max(nrhs, 1), lb), 9.0)
+        b[:, :n] = rng.uniform(-1, 1, (max(nrhs, 1), n))
+        a0s.append(a)
+        b0s.append(b)
+        lda.append(la)
+        ldb.append(lb)
+        As.append(torch.tensor(a, device="cuda"))
+        Bs.append(torch.tensor(b, device="cuda"))
+    count = len(ns)
+    info = np.full(count, -1, dtype=np.int32)
+    assert AB.atlb_dposv_batched(count, _int_array(ns), _ptr_array(As), _int_array(lda), _ptr_array(Bs),
+                                 _int_array(ldb), _int_array([nrhs] * count), info) == 0
+    assert np.all(info == 0)
+    for i, n in enumerate(ns):
+        a, b = As[i].cpu().numpy(), Bs[i].cpu().numpy()
+        assert np.array_equal(a[:, n:], a0s[i][:, n:]) and np.array_equal(b[:, n:], b0s[i][:, n:])
+        if n == 0:
+            continue
+        low = np.triu(a[:n, :n]).T                    # rows of `a` are columns of L
+        assert np.array_equal(np.tril(a[:n, :n], -1), np.tril(a0s[i][:n, :n], -1))
+        mag = np.abs(low) @ np.abs(low.T)
+        assert np.all(np.abs(low @ low.T - a0s[i][:n, :n]) <= 2 * (n + 2) * u * mag)
+        for r in range(nrhs):
+            x = b[r, :n]
+            assert np.all(np.abs(a0s[i][:n, :n] @ x - b0s[i][r, :n]) <= 2 * (3 * n + 2) * u * (mag @ np.abs(x)))
+        if nrhs == 0:
+            assert np.array_equal(b, b0s[i])
+
+
 def test_batched_posv_reports_indefinite(gpu):
     import torch
     ns = np.array([20, 150], dtype=np.int32)
