@@ -4,40 +4,39 @@
 // Driver: the reference's recursion (src/lapack/ATL_potrfL.c:204-263,
 // ATL_potrfU.c:199-257): factor the leading half, TRSM the off-diagonal block
 // against it, SYRK-update the trailing half (the DMMA GEMM restricted to one
-// triangle), factor the trailing half.  Leaves of <= 128 columns are factored
-// by one CTA in shared memory (blocked: 16-column panels and register-tiled
-// updates of the trailing triangle); the upper case is factored as the
-// transpose of the lower one (U = L^T), so a single leaf kernel serves both.
+// triangle), factor the trailing half.  Leaves (FP64 <= 256 columns, FP32 <=
+// 128) are factored by one CTA in shared memory; the upper case is factored
+// as the transpose of the lower one (U = L^T).
 #include <algorithm>
 #include <cmath>
 #include <vector>
 #include "common.cuh"
 #include "kernels.h"
 #include "chol_blocks.cuh"
+#include "chol_tiles.cuh"
 
 namespace atlb {
 namespace {
 
-constexpr int CLEAF = 128;
+constexpr int CLEAF = 128;   // columns of a recursion leaf
 
-// Factor the n x n (n <= 128) diagonal block at A in place in shared memory
-// (cholb::chol_smem: 16-column panels, the trailing triangle updated on the
-// FP64 tensor cores for double, with 4 x 4 register tiles for float); the
-// upper case is loaded transposed (U = L^T).  A first non-positive pivot j lowers *dinfo to ioff + j + 1; the
-// block is then left partly factored.
-template <typename T>
+// Factor the n x n (n <= 128) FP32 diagonal block at A in place in shared
+// memory (cholb::chol_smem: 16-column panels, the trailing triangle updated
+// with 4 x 4 register tiles); the upper case is loaded transposed (U = L^T).
+// A first non-positive pivot j lowers *dinfo to ioff + j + 1; the block is
+// then left partly factored.
 __global__ void __launch_bounds__(256)
-potrf_leaf_kernel(int n, T *A, long lda, int upper, int *dinfo, int ioff) {
+potrf_leaf_kernel(int n, float *A, long lda, int upper, int *dinfo, int ioff) {
   extern __shared__ __align__(16) unsigned char leaf_smem[];
-  T *S = reinterpret_cast<T *>(leaf_smem);
+  float *S = reinterpret_cast<float *>(leaf_smem);
   const int lds = cholb::ld_for(n);
   const int nn = n * n, tid = threadIdx.x;
   for (int base = 0; base < nn; base += 256 * 8) {  // eight loads in flight per thread
-    T v[8];
+    float v[8];
 #pragma unroll
     for (int u = 0; u < 8; u++) {
       const int idx = base + u * 256 + tid, i = idx % n, k = idx / n;
-      v[u] = (idx < nn && i >= k) ? (upper ? A[k + (long)i * lda] : A[i + (long)k * lda]) : T(0);
+      v[u] = (idx < nn && i >= k) ? (upper ? A[k + (long)i * lda] : A[i + (long)k * lda]) : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < 8; u++) {
@@ -56,16 +55,50 @@ potrf_leaf_kernel(int n, T *A, long lda, int upper, int *dinfo, int ioff) {
   }
 }
 
-template <typename T>
-void potrf_leaf(int n, T *Ad, long lda, int upper, int *dinfo, int ioff, cudaStream_t st) {
-  const size_t smem = sizeof(T) * (size_t)n * cholb::ld_for(n);
+void potrf_leaf(int n, float *Ad, long lda, int upper, int *dinfo, int ioff, cudaStream_t st) {
+  const size_t smem = sizeof(float) * (size_t)n * cholb::ld_for(n);
   static bool configured = false;
   if (!configured) {
-    ATLB_CUDA_CHECK(cudaFuncSetAttribute(potrf_leaf_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(sizeof(T) * CLEAF * cholb::ld_for(CLEAF))));
+    ATLB_CUDA_CHECK(cudaFuncSetAttribute(potrf_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(sizeof(float) * CLEAF * cholb::ld_for(CLEAF))));
     configured = true;
   }
-  potrf_leaf_kernel<T><<<1, 256, smem, st>>>(n, Ad, lda, upper, dinfo, ioff);
+  potrf_leaf_kernel<<<1, 256, smem, st>>>(n, Ad, lda, upper, dinfo, ioff);
+  ATLB_CUDA_CHECK(cudaGetLastError());
+}
+
+// The FP64 diagonal block (n <= 256): the left-looking tile factorization
+// (chol_tiles.cuh), one CTA.  128 columns take 30 us; with the right-looking
+// panels above, where the whole CTA waits for each 16 x 16 diagonal block,
+// they took 49 us.  Up to 256 columns go in one launch: two leaves with the
+// TRSM and SYRK between them cost more launches and more time.
+struct TileSmem {
+  cholt::Shared<cholt::MAXNB> S;
+  double pool[cholt::pool_tiles_upto(cholt::MAXNB, false) * cholt::TILE];
+};
+template <bool UP>
+__global__ void __launch_bounds__(256)
+potrf_tile_kernel(int n, double *A, long lda, int *dinfo, int ioff) {
+  extern __shared__ __align__(16) double tile_smem[];
+  TileSmem &W = *reinterpret_cast<TileSmem *>(tile_smem);
+  const int fail = cholt::factor<256, UP>(n, A, lda, nullptr, 0, 0, W.pool, nullptr, W.S);
+  if (fail && threadIdx.x == 0) atomicMin(dinfo, ioff + fail);
+}
+
+void potrf_leaf(int n, double *Ad, long lda, int upper, int *dinfo, int ioff, cudaStream_t st) {
+  static bool configured = false;
+  if (!configured) {
+    ATLB_CUDA_CHECK(cudaFuncSetAttribute(potrf_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(TileSmem)));
+    ATLB_CUDA_CHECK(cudaFuncSetAttribute(potrf_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(TileSmem)));
+    configured = true;
+  }
+  const int nb = cdiv(n, cholt::TB);
+  const size_t smem = sizeof(cholt::Shared<cholt::MAXNB>) +
+                      sizeof(double) * cholt::TILE * (size_t)cholt::pool_tiles(nb, false);
+  if (upper) potrf_tile_kernel<true><<<1, 256, smem, st>>>(n, Ad, lda, dinfo, ioff);
+  else potrf_tile_kernel<false><<<1, 256, smem, st>>>(n, Ad, lda, dinfo, ioff);
   ATLB_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -96,8 +129,9 @@ void potrf_rec(int upper, int off, int N, T *A, long lda, int *dinfo, cudaStream
                SgemmFn gemm) {
   if (N <= 0) return;
   T *Ad = A + off + (long)off * lda;
-  if (N <= CLEAF) {
-    potrf_leaf<T>(N, Ad, lda, upper, dinfo, off, st);
+  // FP64: an order <= 256 is one launch; splitting it would add a TRSM and a SYRK
+  if (N <= (sizeof(T) == 8 ? 2 * CLEAF : CLEAF)) {
+    potrf_leaf(N, Ad, lda, upper, dinfo, off, st);
     return;
   }
   const int Nl = std::max(CLEAF, (N / 2) / CLEAF * CLEAF), Nr = N - Nl;
@@ -122,7 +156,8 @@ void potrf_rec(int upper, int off, int N, T *A, long lda, int *dinfo, cudaStream
 
 template <typename T>
 void potrf_dev(int uplo, int N, T *A, long lda, int *dinfo, cudaStream_t st, SgemmFn gemm) {
-  const int NBO = tune(kTunePotrfNB);  // multiple of 64
+  // multiple of 64; an FP64 order one launch covers is not split
+  const int NBO = sizeof(T) == 8 && N <= 2 * CLEAF ? 2 * CLEAF : tune(kTunePotrfNB);
   const std::vector<unsigned long long> key = {21ull + sizeof(T), (unsigned long long)tune_generation(),
       (unsigned long long)uplo,
       (unsigned long long)N, (unsigned long long)lda, (unsigned long long)(uintptr_t)A,

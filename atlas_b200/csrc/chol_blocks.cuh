@@ -1,6 +1,6 @@
-// Blocked Cholesky building blocks in shared memory, for one CTA of 256
-// threads: the batched solver (batched.cu) factors whole small matrices with
-// them, the blocked potrf (chol.cu) its diagonal blocks.
+// Blocked Cholesky in shared memory, for one CTA of 256 threads: the FP32
+// potrf (chol.cu) factors its diagonal blocks with it (FP64: chol_tiles.cuh).
+// Also the FP64 MMA and the leading dimension shared by the batched LU.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -48,8 +48,8 @@ __device__ __forceinline__ void syrk_lower_update(int mt, int nc, int jb, const 
 }
 
 // Leading dimension for an order-n matrix in shared memory: the smallest
-// value >= n that is 8 (mod 16) doubles, so that the 8 x 4 operand fragments
-// of the FP64 MMA below (lanes: 8 rows x 4 columns) fall in distinct banks.
+// value >= n that is 8 (mod 16), so that the 8 x 4 operand fragments of the
+// FP64 MMA below (lanes: 8 rows x 4 columns) fall in distinct banks.
 __host__ __device__ constexpr int ld_for(int n) { return (n + 7) / 16 * 16 + 8; }
 
 // d += a b on one m8n8k4 FP64 tensor-core tile (PTX mma.m8n8k4 .f64
@@ -59,74 +59,6 @@ __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                : "+d"(d[0]), "+d"(d[1])
                : "d"(a), "d"(b));
-}
-
-// FP64 form of syrk_lower_update on the tensor cores: each warp of the 256
-// owns a 16 x 32 part of every 64 x 64 block (2 x 4 tiles of 8 x 8), skips
-// the tiles strictly above the diagonal, starts its accumulators from C and
-// adds (-P) P^T in k-steps of 4 (P read as zero beyond jb); KJ > 0 fixes jb
-// at compile time.
-template <int KJ, typename CT>
-__device__ __forceinline__ void syrk_lower_update_dmma(int mt, int nc, int jb_, const double *P, int lds, CT *C,
-                                                       long ldc) {
-  const int jb = KJ ? KJ : jb_;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const int wr = (warp >> 1) * 16, wc = (warp & 1) * 32;
-  for (int ib = 0; ib < mt; ib += 64)
-    for (int kb = 0; kb <= ib && kb < nc; kb += 64) {
-      const int r0 = ib + wr, c0 = kb + wc;
-      if (r0 >= mt || c0 >= nc || c0 > r0 + 15) continue;  // warp-uniform: nothing of this warp's part is stored
-      double acc[2][4][2];
-#pragma unroll
-      for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++)
-#pragma unroll
-          for (int e = 0; e < 2; e++) {
-            const int i = r0 + 8 * a + g, k = c0 + 8 * b + 2 * t + e;
-            acc[a][b][e] = (i < mt && k < nc && k <= i) ? double(C[i + (long)k * ldc]) : 0.0;
-          }
-#pragma unroll 4
-      for (int q = 0; q < jb; q += 4) {
-        const int qq = q + t;
-        double av[2], bv[4];
-#pragma unroll
-        for (int a = 0; a < 2; a++) {
-          const int i = r0 + 8 * a + g;
-          av[a] = (i < mt && qq < jb) ? -P[i + qq * lds] : 0.0;
-        }
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-          const int k = c0 + 8 * b + g;
-          bv[b] = (k < nc && qq < jb) ? P[k + qq * lds] : 0.0;
-        }
-#pragma unroll
-        for (int a = 0; a < 2; a++)
-#pragma unroll
-          for (int b = 0; b < 4; b++)
-            if (c0 + 8 * b <= r0 + 8 * a + 7) dmma_8x8x4(acc[a][b], av[a], bv[b]);
-      }
-#pragma unroll
-      for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++)
-#pragma unroll
-          for (int e = 0; e < 2; e++) {
-            const int i = r0 + 8 * a + g, k = c0 + 8 * b + 2 * t + e;
-            if (i < mt && k < nc && k <= i) C[i + (long)k * ldc] = acc[a][b][e];
-          }
-    }
-}
-
-// the trailing update of a 16-column panel: FP64 on the tensor cores, FP32 on the FMA pipes
-template <typename T, typename CT>
-__device__ __forceinline__ void syrk_panel(int mt, int nc, int jb, const T *P, int lds, CT *C, long ldc) {
-  if constexpr (sizeof(T) == 8) {
-    if (jb == 16) syrk_lower_update_dmma<16>(mt, nc, jb, P, lds, C, ldc);
-    else syrk_lower_update_dmma<0>(mt, nc, jb, P, lds, C, ldc);
-  } else {
-    syrk_lower_update(mt, nc, jb, P, lds, C, ldc);
-  }
 }
 
 // Cholesky of the jb <= 16 columns of the m x jb panel at s (ld lds, rows
@@ -221,7 +153,7 @@ __device__ int chol_panel(T *s, int lds, int m, int jb) {
     const int f = chol_panel16(P, lds, m - j, w);
     if (f) return j + f;
     if (rest > 0) {
-      syrk_panel(m - j - w, rest, w, P + w, lds, P + w + w * lds, lds);
+      syrk_lower_update(m - j - w, rest, w, P + w, lds, P + w + w * lds, lds);
       __syncthreads();
     }
   }

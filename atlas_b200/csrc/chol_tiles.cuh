@@ -86,66 +86,102 @@ struct Shared {
   double D[TILE];       // the current diagonal tile of L, D[c * 16 + k] = L(k, c)
   double rinv[TB * NB]; // 1 / L(c, c)
   double t[RHS * TB];
-  int fail;
+  unsigned char slot[NB][MAXNB];  // kSlots of this order
+  int fail, stored;
 };
 
-// acc(16 x 8 half hh of the tile) += (-L_i) L_j^T over one 16-column tile pair
-__device__ __forceinline__ void mma_half(double (&acc)[2][2], const double *Li, const double *Lj, int hh) {
+// The operand fragments of one 16-column tile pair: a = rows of -L_i, b = rows of L_j.
+struct Frags {
+  double a[4][2], b[4][2];
+};
+__device__ __forceinline__ void load_frags(Frags &f, const double *Li, const double *Lj) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  double a[4][2], b[4];
 #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    a[q][0] = Li[at(g, 4 * q + t)];
-    a[q][1] = Li[at(g + 8, 4 * q + t)];
-    b[q] = Lj[at(8 * hh + g, 4 * q + t)];
-  }
+  for (int q = 0; q < 4; q++)
 #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    cholb::dmma_8x8x4(acc[0], -a[q][0], b[q]);
-    cholb::dmma_8x8x4(acc[1], -a[q][1], b[q]);
-  }
+    for (int h = 0; h < 2; h++) {
+      f.a[q][h] = Li[at(g + 8 * h, 4 * q + t)];
+      f.b[q][h] = Lj[at(g + 8 * h, 4 * q + t)];
+    }
 }
-__device__ __forceinline__ void mma_rhs_half(double (&acc)[2], const double *Lr, const double *Lj, int hh) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+__device__ __forceinline__ void mma_tile(double (&acc)[2][2][2], const Frags &f) {
 #pragma unroll
-  for (int q = 0; q < 4; q++) cholb::dmma_8x8x4(acc, -Lr[rat(g, 4 * q + t)], Lj[at(8 * hh + g, 4 * q + t)]);
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int a = 0; a < 2; a++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) cholb::dmma_8x8x4(acc[a][h], -f.a[q][a], f.b[q][h]);
 }
 
-// tile(i, c) half hh -= sum over k in [k0, k1) of L(i, k) L(c, k)^T
-__device__ __forceinline__ void update_half(double *pool, const unsigned char (*sl)[MAXNB], int i, int c, int hh,
-                                            int k0, int k1) {
+// tile(i, c) -= sum over k in [k0, k1) of L(i, k) L(c, k)^T by one warp; four
+// accumulators, because a dependent FP64 MMA waits 26 cycles for the one
+// before, and the next tile pair's fragments are loaded under the products
+__device__ __forceinline__ void update_tile(double *pool, const unsigned char (*sl)[MAXNB], int i, int c, int k0,
+                                            int k1) {
   if (k0 >= k1) return;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   double *C = pool + (int)sl[i][c] * TILE;
-  double acc[2][2];
+  double acc[2][2][2];
+  Frags f;
+  load_frags(f, pool + (int)sl[i][k0] * TILE, pool + (int)sl[c][k0] * TILE);
 #pragma unroll
   for (int a = 0; a < 2; a++)
 #pragma unroll
-    for (int e = 0; e < 2; e++) acc[a][e] = C[at(g + 8 * a, 8 * hh + 2 * t + e)];
-  for (int k = k0; k < k1; k++)
-    mma_half(acc, pool + (int)sl[i][k] * TILE, pool + (int)sl[c][k] * TILE, hh);
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) acc[a][h][e] = C[at(g + 8 * a, 8 * h + 2 * t + e)];
+#pragma unroll 1
+  for (int k = k0 + 1; k < k1; k++) {
+    Frags nx;
+    load_frags(nx, pool + (int)sl[i][k] * TILE, pool + (int)sl[c][k] * TILE);
+    mma_tile(acc, f);
+    f = nx;
+  }
+  mma_tile(acc, f);
 #pragma unroll
   for (int a = 0; a < 2; a++)
 #pragma unroll
-    for (int e = 0; e < 2; e++) C[at(g + 8 * a, 8 * hh + 2 * t + e)] = acc[a][e];
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) C[at(g + 8 * a, 8 * h + 2 * t + e)] = acc[a][h][e];
 }
-__device__ __forceinline__ void update_rhs_half(double *pool, const unsigned char (*sl)[MAXNB], double *rhs, int c,
-                                                int hh, int k0, int k1) {
+// the same for the right-hand sides' rows
+__device__ __forceinline__ void update_rhs(double *pool, const unsigned char (*sl)[MAXNB], double *rhs, int c, int k0,
+                                           int k1) {
   if (k0 >= k1) return;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   double *C = rhs + c * RTILE;
-  double acc[2];
+  double acc[2][2];
 #pragma unroll
-  for (int e = 0; e < 2; e++) acc[e] = C[rat(g, 8 * hh + 2 * t + e)];
-  for (int k = k0; k < k1; k++) mma_rhs_half(acc, rhs + k * RTILE, pool + (int)sl[c][k] * TILE, hh);
+  for (int h = 0; h < 2; h++)
 #pragma unroll
-  for (int e = 0; e < 2; e++) C[rat(g, 8 * hh + 2 * t + e)] = acc[e];
+    for (int e = 0; e < 2; e++) acc[h][e] = C[rat(g, 8 * h + 2 * t + e)];
+#pragma unroll 1
+  for (int k = k0; k < k1; k++) {
+    const double *Lr = rhs + k * RTILE, *Lj = pool + (int)sl[c][k] * TILE;
+    double a[4], b[4][2];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      a[q] = Lr[rat(g, 4 * q + t)];
+      b[q][0] = Lj[at(g, 4 * q + t)];
+      b[q][1] = Lj[at(g + 8, 4 * q + t)];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) cholb::dmma_8x8x4(acc[h], -a[q], b[q][h]);
+  }
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) C[rat(g, 8 * h + 2 * t + e)] = acc[h][e];
 }
 
 // Factor the jb <= 16 columns of diagonal tile T (one warp; lane i and lane
 // i + 16 hold row i).  Every lane carries its own diagonal entry, so the
 // chain from column to column is: the diagonal by shuffle, 1/sqrt, this
-// lane's multiplier, its next diagonal entry.  L(k, c) goes to D[c * 16 + k],
+// lane's multiplier, its next diagonal entry; the other lanes' multipliers
+// come back from D two at a time (shuffling them doubled the instructions).  L(k, c) goes to D[c * 16 + k],
 // 1/L(c, c) to rinv; columns from the first non-positive pivot on are not
 // stored.  Returns 0 or that pivot's 1-based column.
 __device__ __forceinline__ int factor_diag(const double *T, int jb, double *D, double *rinv) {
@@ -153,20 +189,23 @@ __device__ __forceinline__ int factor_diag(const double *T, int jb, double *D, d
   double r[TB];
 #pragma unroll
   for (int k = 0; k < TB; k++) r[k] = T[at(i, k)];
-  double dg = T[at(i, i)];
+  double dg = i < jb ? T[at(i, i)] : 1.0;
   int fail = 0;
+  double d = __shfl_sync(0xffffffffu, dg, 0);
 #pragma unroll
   for (int c = 0; c < TB; c++) {
-    if (c < jb) {
-      const double d = __shfl_sync(0xffffffffu, dg, c);
-      if (!(d > 0.0) && !fail) fail = c + 1;
-      const double ri = rsqrt(d);
-      const double l = (i == c ? d : r[c]) * ri;
-      dg = fma(-l, l, dg);
-      if (!fail && lane < TB && i >= c) D[c * TB + i] = l;
-      if (lane == 0) rinv[c] = ri;
+    if (!(d > 0.0) && !fail) fail = c + 1;  // later columns run on, unused
+    const double ri = rsqrt(d), l = (i == c ? d : r[c]) * ri;
+    dg = fma(-l, l, dg);
+    if (c + 1 < TB) d = __shfl_sync(0xffffffffu, dg, c + 1);
+    if (lane < TB) D[c * TB + i] = l;  // above the diagonal: not a value anyone reads
+    if (lane == 0) rinv[c] = ri;
+    __syncwarp();
 #pragma unroll
-      for (int k = c + 1; k < TB; k++) r[k] = fma(-l, __shfl_sync(0xffffffffu, l, k), r[k]);
+    for (int k = (c + 1) & ~1; k < TB; k += 2) {
+      const double2 m = *reinterpret_cast<const double2 *>(D + c * TB + k);
+      if (k > c) r[k] = fma(-l, m.x, r[k]);
+      r[k + 1] = fma(-l, m.y, r[k + 1]);
     }
   }
   return fail;
@@ -186,10 +225,13 @@ __device__ int factor(int n, double *A, long lda, const double *B, long ldb, int
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr int NW = NT / 32, NC = NT - 32;  // warps 1.. copy panels in
   const int nb = (n + TB - 1) / TB;
-  const unsigned char(*sl)[MAXNB] = kSlots.slot[nb];
+  const unsigned char(*sl)[MAXNB] = S.slot;
+  for (int idx = tid; idx < nb * MAXNB; idx += NT) S.slot[0][idx] = kSlots.slot[nb][0][idx];
+  __syncthreads();
   // panel c of A (and of B^T) into its tiles, zero beyond the matrix
   auto load_panel = [&](int c, int id, int step) {
     const int tot = (nb - c) * TILE;
+#pragma unroll 2
     for (int idx = id; idx < tot; idx += step) {
       const int i = c + (idx >> 8);
       const int r = UP ? (idx >> 4) & 15 : idx & 15, q = UP ? idx & 15 : (idx >> 4) & 15;
@@ -206,52 +248,52 @@ __device__ int factor(int n, double *A, long lda, const double *B, long ldb, int
       }
   };
   if (tid == 0) S.fail = 0;
-  load_panel(0, tid, NT);
-  if (nb > 1) load_panel(1, tid, NT);
+#pragma unroll 1
+  for (int c = 0; c < min(nb, 2); c++) load_panel(c, tid, NT);
   cp_async_commit();
   cp_async_wait<0>();
   __syncthreads();
+#pragma unroll 1
   for (int j = 0; j < nb; j++) {
     const int jb = min(TB, n - j * TB);
     // phase 1
     if (warp == 0) {
-      update_half(pool, sl, j, j, 0, max(0, j - 1), j);
-      update_half(pool, sl, j, j, 1, max(0, j - 1), j);
+      update_tile(pool, sl, j, j, max(0, j - 1), j);
       __syncwarp();
       const int f = factor_diag(pool + (int)sl[j][j] * TILE, jb, S.D, S.rinv + j * TB);
-      if (lane == 0 && f) S.fail = j * TB + f;
-      __syncwarp();
-      const int stored = f ? f - 1 : jb;
-      for (int idx = lane; idx < stored * TB; idx += 32) {
-        const int c = idx >> 4, i = idx & 15;
-        if (i >= c && i < jb) {
-          if (UP) A[j * TB + c + (long)(j * TB + i) * lda] = S.D[idx];
-          else A[j * TB + i + (long)(j * TB + c) * lda] = S.D[idx];
-        }
+      if (lane == 0) {
+        S.stored = f ? f - 1 : jb;
+        if (f) S.fail = j * TB + f;
       }
-      for (int idx = lane; idx < TILE; idx += 32)  // columns the matrix does not have solve to zero
-        if ((idx >> 4) >= jb) {
+      if (jb < TB)  // columns the matrix does not have solve to zero
+        for (int idx = jb * TB + lane; idx < TILE; idx += 32) {
           S.D[idx] = 0.0;
           S.rinv[j * TB + (idx >> 4)] = 0.0;
         }
     } else {
       if (j + 2 < nb) load_panel(j + 2, tid - 32, NC);
-      const int rows = nb - 1 - j, tasks = 2 * rows + (nr > 0 ? 2 : 0);
-      for (int s = warp - 1; s < tasks; s += NW - 1) {
-        const int i = j + 1 + (s >> 1), hh = s & 1;
-        if (i < nb) {
-          update_half(pool, sl, i, j, hh, max(0, j - 1), j);
-          update_half(pool, sl, i, j + 1, hh, 0, j);
-        } else {
-          update_rhs_half(pool, sl, rhs, j, hh, max(0, j - 1), j);
-          if (j + 1 < nb) update_rhs_half(pool, sl, rhs, j + 1, hh, 0, j);
+#pragma unroll 1
+      for (int i = j + warp; i <= nb; i += NW - 1)
+#pragma unroll 1
+        for (int c = j; c <= min(j + 1, nb - 1); c++) {
+          const int k0 = c == j ? max(0, j - 1) : 0;
+          if (i < nb) update_tile(pool, sl, i, c, k0, j);
+          else if (nr > 0) update_rhs(pool, sl, rhs, c, k0, j);
         }
-      }
     }
     __syncthreads();
+#pragma unroll 1
+    for (int idx = tid; idx < TILE; idx += NT) {  // the diagonal tile goes out
+      const int c = idx >> 4, i = idx & 15;
+      if (i >= c && i < jb && c < S.stored) {
+        if (UP) A[j * TB + c + (long)(j * TB + i) * lda] = S.D[idx];
+        else A[j * TB + i + (long)(j * TB + c) * lda] = S.D[idx];
+      }
+    }
     if (S.fail) break;
     // phase 2: rows below the diagonal tile, and the right-hand sides
     const int nrow = (nb - 1 - j) * TB;
+#pragma unroll 1
     for (int row = tid; row < nrow + nr; row += NT) {
       const bool isr = row >= nrow;
       const int i = j + 1 + (row >> 4), rr = isr ? row - nrow : row & 15;
@@ -263,7 +305,11 @@ __device__ int factor(int n, double *A, long lda, const double *B, long ldb, int
       for (int c = 0; c < TB; c++) {
         x[c] *= S.rinv[j * TB + c];
 #pragma unroll
-        for (int k = c + 1; k < TB; k++) x[k] = fma(-x[c], S.D[c * TB + k], x[k]);
+        for (int k = (c + 1) & ~1; k < TB; k += 2) {
+          const double2 d = *reinterpret_cast<const double2 *>(S.D + c * TB + k);
+          if (k > c) x[k] = fma(-x[c], d.x, x[k]);
+          x[k + 1] = fma(-x[c], d.y, x[k + 1]);
+        }
       }
 #pragma unroll
       for (int c = 0; c < TB; c++) T[isr ? rat(rr, c) : at(rr, c)] = x[c];
@@ -305,6 +351,7 @@ __device__ void stream_solve(int n, const double *A, long lda, int nr, double *x
       const int j = backward ? nb - 1 - s : s;
       double *P = ring + (s & 1) * nb * TILE;
       const int tot = (nb - j) * TILE;
+#pragma unroll 2
       for (int idx = tid; idx < tot; idx += NT) {
         const int i = j + (idx >> 8), r = idx & 15, q = (idx >> 4) & 15;
         const int gi = i * TB + r, gk = j * TB + q;
@@ -315,6 +362,7 @@ __device__ void stream_solve(int n, const double *A, long lda, int nr, double *x
     cp_async_commit();
   };
   fetch(0);
+#pragma unroll 1
   for (int s = 0; s < nb; s++) {
     const int j = backward ? nb - 1 - s : s;
     fetch(s + 1);
@@ -323,10 +371,12 @@ __device__ void stream_solve(int n, const double *A, long lda, int nr, double *x
     const double *P = ring + (s & 1) * nb * TILE;
     if (backward) {  // t(c) = sum over the rows below of L(i, c) x(i): half a warp per column
       const int rr = tid & 15;
+#pragma unroll 1
       for (int c = tid >> 4; c < TB; c += NT / 16) {
         double acc[RHS];
 #pragma unroll
         for (int r = 0; r < RHS; r++) acc[r] = 0.0;
+#pragma unroll 2
         for (int i = 1; i < nb - j; i++) {
           const double l = P[i * TILE + c * TB + (rr ^ c)];
           const double *x = xs + (j + i) * TB + rr;
@@ -344,6 +394,7 @@ __device__ void stream_solve(int n, const double *A, long lda, int nr, double *x
       }
       __syncthreads();
     }
+#pragma unroll 1
     for (int r = warp; r < nr; r += NW) {  // the diagonal tile: one warp per right-hand side
       const int c = lane & 15;
       double v = xs[r * np + j * TB + c];
@@ -368,6 +419,7 @@ __device__ void stream_solve(int n, const double *A, long lda, int nr, double *x
     }
     __syncthreads();
     if (!backward) {
+#pragma unroll 1
       for (int row = tid; row < (nb - 1 - j) * TB; row += NT) {
         const int i = 1 + (row >> 4), rr = row & 15;
         double l[TB];
@@ -397,9 +449,11 @@ __device__ void solve(int n, const double *A, long lda, double *B, long ldb, int
                       const double *rhs, Shared<NB> &S) {
   const int tid = threadIdx.x, nb = (n + TB - 1) / TB, np = nb * TB;
   double *xs = pool, *ring = pool + (nb + 1) / 2 * TILE;  // 8 x 16 nb values take nb / 2 tiles
+#pragma unroll 1
   for (int r0 = 0; r0 < nrhs; r0 += RHS) {
     const int nr = min(RHS, nrhs - r0);
     double *Bc = B + (long)r0 * ldb;
+#pragma unroll 1
     for (int idx = tid; idx < nr * np; idx += NT) {
       const int r = idx / np, i = idx - r * np;
       xs[idx] = r0 == 0 ? rhs[(i >> 4) * RTILE + rat(r, i & 15)] : (i < n ? Bc[i + (long)r * ldb] : 0.0);
@@ -407,6 +461,7 @@ __device__ void solve(int n, const double *A, long lda, double *B, long ldb, int
     __syncthreads();
     if (r0 > 0) stream_solve<NT, false>(n, A, lda, nr, xs, ring, S);
     stream_solve<NT, true>(n, A, lda, nr, xs, ring, S);
+#pragma unroll 1
     for (int idx = tid; idx < nr * np; idx += NT) {
       const int r = idx / np, i = idx - r * np;
       if (i < n) Bc[i + (long)r * ldb] = xs[idx];

@@ -123,6 +123,32 @@ def test_potrf_vs_oracle(gpu, orc, uplo, n):
     assert np.array_equal(a[:n][other], a0[other])
 
 
+@pytest.mark.parametrize("uplo", [121, 122])
+@pytest.mark.parametrize("n,bad", [(1, 0), (15, 0), (16, 0), (17, 17), (129, 0), (240, 200), (255, 0), (256, 0),
+                                   (256, 241), (256, 256), (257, 0)])
+def test_potrf_one_launch_orders(gpu, uplo, n, bad):
+    """Orders around the tiles of the one-launch factorization, and a negative
+    minor in the first, middle and last tile.  |A - L L^T| <= (n + 1) u |L||L^T|
+    componentwise (Higham, theorem 10.3), doubled for the reciprocal diagonal;
+    the other triangle and the rows below the matrix are not written."""
+    rng = np.random.default_rng(n + bad)
+    lda = n + 2
+    g = rng.standard_normal((n, n))
+    sym = g @ g.T + n * np.eye(n)
+    if bad:
+        sym[bad - 1, bad - 1] = -1.0
+    a = np.full((lda, n), 5.0, order="F")
+    a[:n] = sym
+    a0 = a.copy(order="F")
+    assert AB.clapack_dpotrf(CM, uplo, n, a, lda) == bad
+    assert np.array_equal(a[n:], a0[n:])
+    other = np.triu(np.ones((n, n), bool), 1) if uplo == 122 else np.tril(np.ones((n, n), bool), -1)
+    assert np.array_equal(a[:n][other], a0[:n][other])
+    if not bad:
+        low = np.tril(a[:n]) if uplo == 122 else np.triu(a[:n]).T
+        assert np.all(np.abs(low @ low.T - sym) <= 2 * (n + 2) * 2.0 ** -53 * (np.abs(low) @ np.abs(low.T)))
+
+
 @pytest.mark.parametrize("bad", [0, 37, 64, 150])
 def test_potrf_not_spd_info(gpu, orc, bad):
     n = 200
