@@ -36,16 +36,16 @@ template <int BO> struct Lay<true, BO> {
 };
 
 // Issue the cp.async copies of one BO x BK tile (o0.., k0..) of an operand.
-template <bool KC, int VEC, int BO>
+template <bool KC, int VEC, int BO, int NTHR = THREADS>
 __device__ __forceinline__ void load_tile(double *s, const double *X, long ld, int o0, int k0,
                                           int O, int K, int tid) {
   using L = Lay<KC, BO>;
-  constexpr int N16 = BO * BK / 2 / THREADS, N8 = BO * BK / THREADS;  // copies per thread
+  constexpr int N16 = BO * BK / 2 / NTHR, N8 = BO * BK / NTHR;  // copies per thread
   if (!KC) {
     if (VEC == 2) {
 #pragma unroll
       for (int i = 0; i < N16; i++) {
-        int c = tid + THREADS * i, k = c / (BO / 2), o = (c % (BO / 2)) * 2;
+        int c = tid + NTHR * i, k = c / (BO / 2), o = (c % (BO / 2)) * 2;
         int go = o0 + o, gk = k0 + k;
         double *d = s + L::at(o, k);
         const double *g = X + go + (long)gk * ld;
@@ -59,7 +59,7 @@ __device__ __forceinline__ void load_tile(double *s, const double *X, long ld, i
     } else {
 #pragma unroll
       for (int i = 0; i < N8; i++) {
-        int c = tid + THREADS * i, k = c / BO, o = c % BO;
+        int c = tid + NTHR * i, k = c / BO, o = c % BO;
         int go = o0 + o, gk = k0 + k;
         bool p = gk < K && go < O;
         cp_async8(s + L::at(o, k), p ? X + go + (long)gk * ld : X, p);
@@ -69,7 +69,7 @@ __device__ __forceinline__ void load_tile(double *s, const double *X, long ld, i
     if (VEC == 2) {
 #pragma unroll
       for (int i = 0; i < N16; i++) {
-        int c = tid + THREADS * i, o = c >> 3, k = (c & 7) * 2;
+        int c = tid + NTHR * i, o = c >> 3, k = (c & 7) * 2;
         int go = o0 + o, gk = k0 + k;
         double *d = s + L::at(o, k);
         const double *g = X + gk + (long)go * ld;
@@ -83,7 +83,7 @@ __device__ __forceinline__ void load_tile(double *s, const double *X, long ld, i
     } else {
 #pragma unroll
       for (int i = 0; i < N8; i++) {
-        int c = tid + THREADS * i, o = c >> 4, k = c & 15;
+        int c = tid + NTHR * i, o = c >> 4, k = c & 15;
         int go = o0 + o, gk = k0 + k;
         bool p = go < O && gk < K;
         cp_async8(s + L::at(o, k), p ? X + gk + (long)go * ld : X, p);
@@ -107,6 +107,7 @@ template <int BNT> struct TileCfg {
   static constexpr int smem_doubles() { return STG * (Lay<TA, BM>::SIZE + Lay<!TB, BNT>::SIZE); }
 };
 constexpr int SMALL_K = 256;  // K up to this uses the 128 x 64 tiles
+constexpr int SMALL_TILE_K = 512;  // K up to this, with few tiles, uses 64 x 64 or 32 x 32 tiles
 // the grouped (batched) GEMM's tile width: its problems are small (K <= 512,
 // M, N from 16), where the narrower tile wastes less on padding and two CTAs
 // per SM overlap their epilogues
@@ -143,7 +144,7 @@ __device__ __forceinline__ void dgemm_tile(int M, int N, int K, double alpha, co
 
   const int KT = (K + BK - 1) / BK;
 #pragma unroll
-  for (int s = 0; s < STG - 1; s++) {
+  for (int s = 0; s < STG; s++) {
     if (s < KT) {
       load_tile<TA, VEC, BM>(sA + s * LA::SIZE, A, lda, m0, s * BK, M, K, tid);
       load_tile<!TB, VEC, BNT>(sB + s * LB::SIZE, B, ldb, n0, s * BK, N, K, tid);
@@ -151,33 +152,55 @@ __device__ __forceinline__ void dgemm_tile(int M, int N, int K, double alpha, co
     cp_async_commit();
   }
 
-  const int fr = lane >> 2, fk = lane & 3;
-  for (int kt = 0; kt < KT; kt++) {
-    cp_async_wait<STG - 2>();
-    __syncthreads();
-    {
-      int nk = kt + STG - 1;
-      if (nk < KT) {
-        int st = nk % STG;
-        load_tile<TA, VEC, BM>(sA + st * LA::SIZE, A, lda, m0, nk * BK, M, K, tid);
-        load_tile<!TB, VEC, BNT>(sB + st * LB::SIZE, B, ldb, n0, nk * BK, N, K, tid);
-      }
-      cp_async_commit();
+  if (beta != 0.0) {  // the old C tile on its way to L2 while the products run
+    for (int idx = tid; idx < BNT * (BM / 16); idx += THREADS) {
+      const int r = m0 + idx % (BM / 16) * 16, c = n0 + idx / (BM / 16);
+      if (r < M && c < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + r + (long)c * ldc));
     }
-    const double *a_s = sA + (kt % STG) * LA::SIZE;
-    const double *b_s = sB + (kt % STG) * LB::SIZE;
+  }
+
+  // The FP64 MMA unit is one per SM and a few warps keep it full, so what
+  // costs is every warp being away from it at once: at a barrier, issuing
+  // copies, waiting for the first fragments behind the barrier.  Fragments
+  // are therefore loaded one k-step ahead, the barrier that opens the next k
+  // tile stands before the last k-step's products (whose fragments are in
+  // registers already), and the copies that refill the stage just finished
+  // are issued behind those products.  8192^3: 31.5 -> 34.3 TFLOP/s (cuBLAS
+  // 35.5); 8192^2 x K with C read back: K = 128 23.4 -> 25.8, 256 27.6 -> 28.7.
+  const int fr = lane >> 2, fk = lane & 3;
+  double a[2][MI], b[2][4];
+  auto fragments = [&](int buf, const double *a_s, const double *b_s, int kk) {
 #pragma unroll
-    for (int kk = 0; kk < BK; kk += 4) {
-      double a[MI], b[4];
+    for (int i = 0; i < MI; i++) a[buf][i] = a_s[LA::at(wm + i * 8 + fr, kk + fk)];
 #pragma unroll
-      for (int i = 0; i < MI; i++) a[i] = a_s[LA::at(wm + i * 8 + fr, kk + fk)];
+    for (int j = 0; j < 4; j++) b[buf][j] = b_s[LB::at(wn + j * 8 + fr, kk + fk)];
+  };
+  cp_async_wait<STG - 1>();
+  __syncthreads();
+  fragments(0, sA, sB, 0);
+  int stage = 0;
+  for (int kt = 0; kt < KT; kt++) {
+    double *a_s = sA + stage * LA::SIZE, *b_s = sB + stage * LB::SIZE;
+    stage = stage + 1 == STG ? 0 : stage + 1;
 #pragma unroll
-      for (int j = 0; j < 4; j++) b[j] = b_s[LB::at(wn + j * 8 + fr, kk + fk)];
+    for (int s = 0; s < BK / 4; s++) {
+      if (s < BK / 4 - 1) {
+        fragments((s + 1) & 1, a_s, b_s, 4 * (s + 1));
+      } else {
+        cp_async_wait<STG - 2>();
+        __syncthreads();  // tile kt + 1 has landed, and nobody reads tile kt's stage any more
+        if (kt + 1 < KT) fragments((s + 1) & 1, sA + stage * LA::SIZE, sB + stage * LB::SIZE, 0);
+      }
 #pragma unroll
       for (int i = 0; i < MI; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) dmma(acc[i][j], a[i], b[j]);
+        for (int j = 0; j < 4; j++) dmma(acc[i][j], a[s & 1][i], b[s & 1][j]);
     }
+    if (kt + STG < KT) {
+      load_tile<TA, VEC, BM>(a_s, A, lda, m0, (kt + STG) * BK, M, K, tid);
+      load_tile<!TB, VEC, BNT>(b_s, B, ldb, n0, (kt + STG) * BK, N, K, tid);
+    }
+    cp_async_commit();
   }
   cp_async_wait<0>();
 
@@ -193,9 +216,22 @@ __device__ __forceinline__ void dgemm_tile(int M, int N, int K, double alpha, co
   double *sC = smem;
   if (beta != 0.0) {
     __syncthreads();  // every warp is done with the pipeline buffers
-    for (int idx = tid; idx < BM * BNT; idx += THREADS) {
-      const int rr = idx % BM, cc = idx / BM, r = m0 + rr, c = n0 + cc;
-      if (ok(r, c)) cp_async8(sC + rr + cc * CLD, C + r + (long)c * ldc, true);
+    if (VEC == 2 && (uintptr_t)C % 16 == 0 && ldc % 2 == 0) {
+#pragma unroll 4
+      for (int idx = tid; idx < BM * BNT / 2; idx += THREADS) {
+        const int rr = idx % (BM / 2) * 2, cc = idx / (BM / 2), r = m0 + rr, c = n0 + cc;
+        const bool ok0 = ok(r, c), ok1 = ok(r + 1, c);
+        const double *g = C + r + (long)c * ldc;
+        double *d = sC + rr + cc * CLD;
+        if (ok0 && ok1) cp_async16(d, g, true);
+        else if (ok0) cp_async8(d, g, true);
+        else if (ok1) cp_async8(d + 1, g + 1, true);
+      }
+    } else {
+      for (int idx = tid; idx < BM * BNT; idx += THREADS) {
+        const int rr = idx % BM, cc = idx / BM, r = m0 + rr, c = n0 + cc;
+        if (ok(r, c)) cp_async8(sC + rr + cc * CLD, C + r + (long)c * ldc, true);
+      }
     }
     cp_async_commit();
     cp_async_wait<0>();
@@ -233,6 +269,94 @@ dgemm_dmma_kernel(int M, int N, int K, double alpha, const double *__restrict__ 
   if (tri == 1 && m0 + BM - 1 < n0) return;
   if (tri == 2 && m0 > n0 + BNT - 1) return;
   dgemm_tile<TA, TB, VEC, BNT>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, tri, m0, n0, smem);
+}
+
+// GEMMs whose output has too few 128 x 128 tiles for the SMs and whose K is
+// short (the small updates inside the factorizations, a user's small
+// products): BT x BT tiles (64, or 32 when even those are fewer than the SMs),
+// four warps, old C fetched into registers before the main loop.  Split K
+// needs a second launch and a round trip of the partials through memory,
+// which is most of the time of such a product.  Against split K (device time,
+// launches included): 128^3 14.4 -> 7.5 us, 96 x 80 x 112 16.2 -> 8.9,
+// 1000 x 128 x 128 14.5 -> 8.7, 8000 x 128 x 128 28.2 -> 18.4,
+// 1000 x 1000 x 500 63.6 -> 49.9.
+constexpr int SM_THREADS = 128, SM_STAGES = 3;
+template <bool TA, bool TB, int BT>
+constexpr int small_smem() { return SM_STAGES * (Lay<TA, BT>::SIZE + Lay<!TB, BT>::SIZE) * (int)sizeof(double); }
+
+template <bool TA, bool TB, int VEC, int BT>
+__global__ void __launch_bounds__(SM_THREADS)
+dgemm_small_kernel(int M, int N, int K, double alpha, const double *__restrict__ A, long lda,
+                   const double *__restrict__ B, long ldb, double beta, double *__restrict__ C,
+                   long ldc, int tri) {
+  extern __shared__ __align__(16) double smem[];
+  using LA = Lay<TA, BT>;
+  using LB = Lay<!TB, BT>;
+  constexpr int WT = BT / 2, MI = WT / 8;  // a warp's part: WT x WT
+  double *sA = smem, *sB = smem + SM_STAGES * LA::SIZE;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tiles_m = (M + BT - 1) / BT;
+  const int m0 = (blockIdx.x % tiles_m) * BT, n0 = (blockIdx.x / tiles_m) * BT;
+  if (tri == 1 && m0 + BT - 1 < n0) return;
+  if (tri == 2 && m0 > n0 + BT - 1) return;
+  const int fr = lane >> 2, fk = lane & 3, wm = (warp & 1) * WT, wn = (warp >> 1) * WT;
+  const int KT = (K + BK - 1) / BK;
+  auto load = [&](int kt) {
+    if (kt < KT) {
+      load_tile<TA, VEC, BT, SM_THREADS>(sA + kt % SM_STAGES * LA::SIZE, A, lda, m0, kt * BK, M, K, tid);
+      load_tile<!TB, VEC, BT, SM_THREADS>(sB + kt % SM_STAGES * LB::SIZE, B, ldb, n0, kt * BK, N, K, tid);
+    }
+    cp_async_commit();
+  };
+#pragma unroll 1
+  for (int s = 0; s < SM_STAGES - 1; s++) load(s);
+  auto ok = [&](int r, int c) {
+    return r < M && c < N && !(tri == 1 && r < c) && !(tri == 2 && r > c);
+  };
+  double acc[MI][MI][2], old[MI][MI][2];
+#pragma unroll
+  for (int i = 0; i < MI; i++)
+#pragma unroll
+    for (int j = 0; j < MI; j++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int r = m0 + wm + i * 8 + fr, c = n0 + wn + j * 8 + fk * 2 + h;
+        acc[i][j][h] = 0.0;
+        old[i][j][h] = beta != 0.0 && ok(r, c) ? C[r + (long)c * ldc] : 0.0;
+      }
+#pragma unroll 1
+  for (int kt = 0; kt < KT; kt++) {
+    cp_async_wait<SM_STAGES - 2>();
+    __syncthreads();
+    load(kt + SM_STAGES - 1);
+    const double *a_s = sA + kt % SM_STAGES * LA::SIZE, *b_s = sB + kt % SM_STAGES * LB::SIZE;
+#pragma unroll
+    for (int kk = 0; kk < BK; kk += 4) {
+      double a[MI], b[MI];
+#pragma unroll
+      for (int i = 0; i < MI; i++) {
+        a[i] = a_s[LA::at(wm + i * 8 + fr, kk + fk)];
+        b[i] = b_s[LB::at(wn + i * 8 + fr, kk + fk)];
+      }
+#pragma unroll
+      for (int i = 0; i < MI; i++)
+#pragma unroll
+        for (int j = 0; j < MI; j++) dmma(acc[i][j], a[i], b[j]);
+    }
+  }
+  cp_async_wait<0>();
+#pragma unroll
+  for (int i = 0; i < MI; i++)
+#pragma unroll
+    for (int j = 0; j < MI; j++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int r = m0 + wm + i * 8 + fr, c = n0 + wn + j * 8 + fk * 2 + h;
+        if (!ok(r, c)) continue;
+        double v = alpha * acc[i][j][h];
+        if (beta != 0.0) v = fma(beta, old[i][j][h], v);
+        C[r + (long)c * ldc] = v;
+      }
 }
 
 // The same GEMM on a capped number of CTAs, each walking tiles t, t + grid,
@@ -367,8 +491,26 @@ void launch(int M, int N, int K, double alpha, const double *A, long lda, const 
     configured = true;
   }
   int tiles = cdiv(M, BM) * cdiv(N, BN);
-  // too few tiles for the 148 SMs and a long K: split K (partials + reduction)
   const int nsm = num_sms();
+  // too few tiles for the 148 SMs: smaller tiles while K is short, else split
+  // K (partials + reduction).  At K = 500 the two are level on few tiles
+  // (300 x 300: 16.5 us both ways) and the smaller tiles ahead on many; beyond,
+  // the serial K loop of one tile is the longer.
+  if (tiles * 2 <= nsm && K <= SMALL_TILE_K) {
+    auto go = [&](auto kern, int bt, int bytes, bool &set) {
+      if (!set) {
+        ATLB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        ATLB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+        set = true;
+      }
+      kern<<<cdiv(M, bt) * cdiv(N, bt), SM_THREADS, bytes, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, tri);
+      ATLB_CUDA_CHECK(cudaGetLastError());
+    };
+    static bool set64 = false, set32 = false;
+    if (cdiv(M, 64) * cdiv(N, 64) >= nsm) go(dgemm_small_kernel<TA, TB, VEC, 64>, 64, small_smem<TA, TB, 64>(), set64);
+    else go(dgemm_small_kernel<TA, TB, VEC, 32>, 32, small_smem<TA, TB, 32>(), set32);
+    return;
+  }
   int S = 1;
   if (tune(kTuneSplitK) && tiles * 2 <= nsm && K >= 4 * BK && !no_alloc_active()) S = splitk_count(tiles, K, nsm);
   if (S > 1) {

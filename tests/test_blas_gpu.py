@@ -187,3 +187,41 @@ def test_syrk_golden_cases(gpu, orc, gold):
         mask = np.tril(np.ones((n, n), bool), -1) if uplo == 121 else np.triu(np.ones((n, n), bool), 1)
         assert np.array_equal(c[:n, :n][mask], c0[:n, :n][mask])
         assert orc.gechkgap(c, n, n) == 0
+
+
+@pytest.mark.parametrize("ta,tb", [(111, 111), (111, 112), (112, 111), (112, 112)])
+@pytest.mark.parametrize("m,n,k,pad", [(1, 1, 1, 0), (31, 33, 7, 1), (32, 32, 16, 0), (33, 31, 17, 0), (64, 96, 48, 1),
+                                       (96, 80, 112, 0), (700, 640, 512, 0), (700, 640, 513, 1), (513, 65, 300, 1)])
+def test_dgemm_few_tiles(gpu, ta, tb, m, n, k, pad):
+    """Products with few output tiles (32 x 32 and 64 x 64 tiles up to K = 512,
+    split K above): sizes around the tiles and the K steps, aligned and
+    unaligned leading dimensions; |C - C_ref| <= (k + 3) u (|alpha||A||B| + |beta||C|)
+    componentwise, doubled for the reference's own rounding."""
+    rng = np.random.default_rng(m + n + k)
+    mat = lambda r, c: np.asfortranarray(rng.uniform(-1, 1, (r + pad, c)))
+    a, b = mat(*((m, k) if ta == 111 else (k, m))), mat(*((k, n) if tb == 111 else (n, k)))
+    c0 = mat(m, n)
+    opa = (a[:m] if ta == 111 else a[:k].T)
+    opb = (b[:k] if tb == 111 else b[:n].T)
+    for beta in (0.0, -0.5):
+        c = c0.copy(order="F")
+        AB.cblas_dgemm(102, ta, tb, m, n, k, 1.5, a, a.shape[0], b, b.shape[0], beta, c, c.shape[0])
+        ref = 1.5 * (opa @ opb) + beta * c0[:m]
+        mag = 1.5 * (np.abs(opa) @ np.abs(opb)) + abs(beta) * np.abs(c0[:m])
+        assert np.all(np.abs(c[:m] - ref) <= 2 * (k + 3) * 2.0 ** -53 * mag)
+        assert np.array_equal(c[m:], c0[m:])
+
+
+@pytest.mark.parametrize("uplo", [121, 122])
+@pytest.mark.parametrize("n,k", [(1, 1), (33, 20), (64, 130), (200, 64), (640, 300)])
+def test_dsyrk_few_tiles(gpu, uplo, n, k):
+    """The triangle mask of the small tiles: the other triangle is not written."""
+    rng = np.random.default_rng(n + k)
+    a = np.asfortranarray(rng.uniform(-1, 1, (n, k)))
+    c0 = np.asfortranarray(rng.uniform(-1, 1, (n, n)))
+    c = c0.copy(order="F")
+    AB.cblas_dsyrk(102, uplo, 111, n, k, -1.0, a, n, 1.0, c, n)
+    part = np.triu(np.ones((n, n), bool)) if uplo == 121 else np.tril(np.ones((n, n), bool))
+    mag = np.abs(a) @ np.abs(a.T) + np.abs(c0)
+    assert np.all((np.abs(c - (c0 - a @ a.T)) <= 2 * (k + 3) * 2.0 ** -53 * mag)[part])
+    assert np.array_equal(c[~part], c0[~part])
