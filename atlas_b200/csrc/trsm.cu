@@ -11,6 +11,7 @@
 #include <algorithm>
 #include "common.cuh"
 #include "kernels.h"
+#include "chol_blocks.cuh"
 
 namespace atlb {
 
@@ -741,94 +742,148 @@ template void trsm_dev<float>(int, int, int, int, int, int, float, const float *
 namespace {
 // X = L^-1 B in place, L unit lower triangular of order m <= 256, B m x n:
 // the U12 = L11^-1 A12 step of the blocked LU in ONE launch (the recursive
-// trsm_dev issues a TRSM/GEMM cascade of ~8 kernels for it).  CTA q solves
-// columns 32q .. 32q+31, the whole column tile in shared memory: for each
-// 32-row block, the product of L's 32 x (32 ib) panel with the rows already
-// solved (L read in 32 x 32 tiles, the next tile fetched into registers while
-// the current one is used), then forward substitution with the unit lower
-// 32 x 32 diagonal tile (lane = row, x_k by shuffle, four columns per warp).
-constexpr int LLU_COLS = 32, LLU_MAX = 256;
+// trsm_dev issues a TRSM/GEMM cascade of ~8 kernels for it).
+//
+// FP64, on the tensor cores.  It stands on the factorization's critical chain
+// (the look-ahead block's U12), so what counts is the latency of one CTA: all
+// diagonal 32 x 32 tiles are inverted at once, a warp each (one lane per
+// column, the column shifted through registers), and block row ib is then
+//   X_ib = inv(L_ib,ib) (B_ib - sum_{kt < ib} L_ib,kt X_kt),
+// two runs of MMAs with the next block row of L on its way to shared memory
+// (for m <= 192, where two fit).  CTAs of 32 columns, or of 8 with the k range
+// split between two halves of the warps when the columns are few.  The forward
+// substitution by shuffles that this replaces took 47 us at m = 192; this takes
+// 20 us (192 columns) and 33 us (up to 8000).
+constexpr int LLU_MAX = 256, LLU_LD = 36;  // 4 (mod 16): the MMA's fragments fall in distinct banks
+constexpr int LLU_TILE = 32 * LLU_LD;      // a 32 x 32 tile, (r, k) at k * LLU_LD + r
 
-template <typename T>
+constexpr int llu_smem(int m, int ncol) {
+  const int nblk = (m + 31) / 32, nbuf = m <= 192 ? 2 : 1;
+  return 8 * (ncol * (32 * nblk + 4) + nblk * LLU_TILE + 64 + nbuf * (nblk - 1) * LLU_TILE + 256);
+}
+
+template <int NCOL>
 __global__ void __launch_bounds__(256, 1)
-trsm_llu_small_kernel(int m, int n, const T *__restrict__ L, long lda, T *B, long ldb) {
-  extern __shared__ __align__(16) unsigned char llu_smem[];
-  T(*sX)[LLU_COLS + 1] = reinterpret_cast<T(*)[LLU_COLS + 1]>(llu_smem);  // [LLU_MAX]: B, then X
-  T(*sL)[33] = reinterpret_cast<T(*)[33]>(sX + LLU_MAX);                  // [32]: one tile of L
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int c0 = blockIdx.x * LLU_COLS, nc = min(LLU_COLS, n - c0);
-  for (int base = 0; base < LLU_MAX * LLU_COLS; base += 256 * 8) {  // eight loads in flight per thread
-    T v[8];
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int idx = base + u * 256 + tid, r = idx % LLU_MAX, c = idx / LLU_MAX;
-      v[u] = (r < m && c < nc) ? B[r + (long)(c0 + c) * ldb] : T(0);
+trsm_llu_mma_kernel(int m, int n, const double *__restrict__ L, long lda, double *B, long ldb) {
+  extern __shared__ __align__(16) unsigned char llu_smem_raw[];
+  const int nblk = (m + 31) / 32, LDX = 32 * nblk + 4, nbuf = m <= 192 ? 2 : 1;
+  double *sX = reinterpret_cast<double *>(llu_smem_raw);  // [NCOL][LDX]: B, then X
+  double *sD = sX + NCOL * LDX;                           // the diagonal tiles, then their inverses
+  double *sL = sD + nblk * LLU_TILE + 64;                 // block rows of L, k-major
+  double *sP = sL + nbuf * (nblk - 1) * LLU_TILE;         // the second half's sums (NCOL = 8)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int c0 = blockIdx.x * NCOL, nc = min(NCOL, n - c0);
+  auto fetch_row = [&](int ib) {  // L's block row ib, columns before its diagonal tile
+    if (ib < nblk) {
+      double *dst = sL + (ib % nbuf) * (nblk - 1) * LLU_TILE;
+      for (int e = tid; e < 32 * 32 * ib; e += 256) {
+        const int i = e & 31, k = e >> 5, r = 32 * ib + i;
+        cp_async8(dst + k * LLU_LD + i, r < m ? L + r + (long)k * lda : L, r < m);
+      }
     }
+    cp_async_commit();
+  };
+  for (int e = tid; e < nblk * 1024; e += 256) {  // strictly lower, zero elsewhere: U's entries are not read
+    const int b = e >> 10, k = (e >> 5) & 31, i = e & 31, r = 32 * b + i, c = 32 * b + k;
+    const bool ok = r < m && i > k;
+    cp_async8(sD + b * LLU_TILE + k * LLU_LD + i, ok ? L + r + (long)c * lda : L, ok);
+  }
+  for (int e = tid; e < NCOL * 32 * nblk; e += 256) {
+    const int r = e % (32 * nblk), c = e / (32 * nblk);
+    const bool ok = r < m && c < nc;
+    cp_async8(sX + c * LDX + r, ok ? B + r + (long)(c0 + c) * ldb : B, ok);
+  }
+  cp_async_commit();
+  fetch_row(1);
+  cp_async_wait<1>();
+  __syncthreads();
+  if (warp < nblk) {  // lane j: column j of the inverse, by forward substitution
+    double *D = sD + warp * LLU_TILE;
+    double x[32];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int idx = base + u * 256 + tid;
-      sX[idx % LLU_MAX][idx / LLU_MAX] = v[u];
+    for (int r = 0; r < 32; r++) x[r] = r == lane ? 1.0 : 0.0;
+#pragma unroll 1
+    for (int q = 0; q < 32; q++) {
+      const double v = x[0], *l = D + q * LLU_LD + q;  // column q of L is not needed after this step
+#pragma unroll
+      for (int r = 1; r < 32; r++) x[r - 1] = fma(-l[r], v, x[r]);  // past the tile: values nobody uses
+      __syncwarp();
+      if (lane <= q) D[lane * LLU_LD + q] = v;
+      __syncwarp();
     }
   }
-  const int nblk = (m + 31) / 32;
-  const int rr = tid % 32, cq = tid / 32;  // update: row rr of the block, columns 4 cq .. 4 cq + 3
-  // a thread's four elements of an L tile (rows r0 + i, columns k0 + k)
-  auto fetch = [&](int r0, int k0, T (&v)[4]) {
+  constexpr int NH = NCOL == 8 ? 1 : NCOL / 16;  // 8-column groups of a warp
+  const int rt = 8 * (warp & 3), half = warp >> 2, n0 = NCOL == 8 ? 0 : half * 8 * NH;
+  auto mma = [&](const double *T, const double *X, int k0, int k1, double (&acc)[NH][2]) {
+    const double *a = T + t * LLU_LD + rt + g, *x = X + (n0 + g) * LDX + t;
+#pragma unroll 4
+    for (int k = k0; k < k1; k += 4) {
+      const double av = a[k * LLU_LD];
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-      const int idx = tid + 256 * e, i = idx % 32, k = idx / 32;
-      v[e] = (r0 + i < m && k0 + k < m) ? L[r0 + i + (long)(k0 + k) * lda] : T(0);
-    }
-  };
-  auto store = [&](const T (&v)[4]) {
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-      const int idx = tid + 256 * e;
-      sL[idx % 32][idx / 32] = v[e];
+      for (int h = 0; h < NH; h++) cholb::dmma_8x8x4(acc[h], av, x[8 * h * LDX + k]);
     }
   };
   for (int ib = 0; ib < nblk; ib++) {
-    const int r0 = ib * 32;
-    T acc[4] = {T(0), T(0), T(0), T(0)};
-    T nxt[4];
-    fetch(r0, 0, nxt);  // tile (ib, 0), or the diagonal tile when ib == 0
-    for (int kt = 0; kt < ib; kt++) {
-      __syncthreads();  // the previous tile has been used
-      store(nxt);
+    double acc[NH][2];
+    double *Xr = sX + 32 * ib + rt + g;  // this warp's rows of the block
+    if (ib > 0) {
+      cp_async_wait<0>();
       __syncthreads();
-      fetch(r0, (kt + 1) * 32, nxt);  // the next tile (the diagonal one after the last)
-#pragma unroll 8
-      for (int k = 0; k < 32; k++) {
-        const T lv = sL[rr][k];
+      if (nbuf == 2) fetch_row(ib + 1);
 #pragma unroll
-        for (int e = 0; e < 4; e++) acc[e] = fma(lv, sX[kt * 32 + k][4 * cq + e], acc[e]);
+      for (int h = 0; h < NH; h++) acc[h][0] = acc[h][1] = 0.0;
+      const double *T = sL + (ib % nbuf) * (nblk - 1) * LLU_TILE;
+      if constexpr (NCOL == 8) {
+        mma(T, sX, half * 16 * ib, (half + 1) * 16 * ib, acc);
+        if (half) {
+          sP[(2 * t) * 32 + rt + g] = acc[0][0];
+          sP[(2 * t + 1) * 32 + rt + g] = acc[0][1];
+        }
+        __syncthreads();
+        if (!half)
+#pragma unroll
+          for (int e = 0; e < 2; e++) Xr[(2 * t + e) * LDX] -= acc[0][e] + sP[(2 * t + e) * 32 + rt + g];
+      } else {
+        mma(T, sX, 0, 32 * ib, acc);
+#pragma unroll
+        for (int h = 0; h < NH; h++)
+#pragma unroll
+          for (int e = 0; e < 2; e++) Xr[(n0 + 8 * h + 2 * t + e) * LDX] -= acc[h][e];
+      }
+      if (nbuf == 1) {
+        __syncthreads();
+        fetch_row(ib + 1);
       }
     }
-    __syncthreads();  // every thread is done with sL and the rows it read
-#pragma unroll
-    for (int e = 0; e < 4; e++) sX[r0 + rr][4 * cq + e] -= acc[e];
-    store(nxt);       // the diagonal tile
     __syncthreads();
-    T x[4];
 #pragma unroll
-    for (int e = 0; e < 4; e++) x[e] = sX[r0 + lane][4 * warp + e];
-#pragma unroll
-    for (int k = 0; k < 31; k++) {
-      const T lk = sL[lane][k];
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const T xk = __shfl_sync(0xffffffffu, x[e], k);
-        if (lane > k) x[e] = fma(-lk, xk, x[e]);
-      }
-    }
-#pragma unroll
-    for (int e = 0; e < 4; e++) sX[r0 + lane][4 * warp + e] = x[e];
+    for (int h = 0; h < NH; h++) acc[h][0] = acc[h][1] = 0.0;
+    mma(sD + ib * LLU_TILE, sX + 32 * ib, 0, rt + 8, acc);  // the inverse is lower triangular
     __syncthreads();
+    if (NCOL > 8 || !half)
+#pragma unroll
+      for (int h = 0; h < NH; h++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) Xr[(n0 + 8 * h + 2 * t + e) * LDX] = acc[h][e];
   }
-  for (int idx = tid; idx < LLU_MAX * LLU_COLS; idx += 256) {
-    const int r = idx % LLU_MAX, c = idx / LLU_MAX;
-    if (r < m && c < nc) B[r + (long)(c0 + c) * ldb] = sX[r][c];
+  __syncthreads();
+  for (int e = tid; e < NCOL * 32 * nblk; e += 256) {
+    const int r = e % (32 * nblk), c = e / (32 * nblk);
+    if (r < m && c < nc) B[r + (long)(c0 + c) * ldb] = sX[c * LDX + r];
   }
+}
+
+template <int NCOL>
+void trsm_llu_mma_launch(int m, int n, const double *L, long lda, double *B, long ldb, cudaStream_t st) {
+  static bool configured = false;
+  if (!configured) {
+    constexpr int most = llu_smem(192, NCOL) > llu_smem(LLU_MAX, NCOL) ? llu_smem(192, NCOL) : llu_smem(LLU_MAX, NCOL);
+    static_assert(most <= 227 * 1024, "a column tile does not fit");
+    ATLB_CUDA_CHECK(cudaFuncSetAttribute(trsm_llu_mma_kernel<NCOL>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    configured = true;
+  }
+  trsm_llu_mma_kernel<NCOL><<<cdiv(n, NCOL), 256, llu_smem(m, NCOL), st>>>(m, n, L, lda, B, ldb);
+  ATLB_CUDA_CHECK(cudaGetLastError());
 }
 
 // The same solve in FP32 (the factorization inside the mixed solvers), with
@@ -999,14 +1054,9 @@ void trsm_llu_small_dev(int m, int n, const T *L, long lda, T *B, long ldb, cuda
     else trsm_llu_inv_launch<4, 1>(m, n, (const float *)L, lda, (float *)B, ldb, st);
     return;
   }
-  constexpr int smem = (LLU_MAX * (LLU_COLS + 1) + 32 * 33) * (int)sizeof(T);
-  static bool configured = false;
-  if (!configured) {
-    ATLB_CUDA_CHECK(cudaFuncSetAttribute(trsm_llu_small_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    configured = true;
-  }
-  trsm_llu_small_kernel<T><<<cdiv(n, LLU_COLS), 256, smem, st>>>(m, n, L, lda, B, ldb);
-  ATLB_CUDA_CHECK(cudaGetLastError());
+  // FP64: 8 columns a CTA while that still leaves SMs free, else 32
+  if (n <= 4 * num_sms()) trsm_llu_mma_launch<8>(m, n, (const double *)L, lda, (double *)B, ldb, st);
+  else trsm_llu_mma_launch<32>(m, n, (const double *)L, lda, (double *)B, ldb, st);
 }
 template void trsm_llu_small_dev<double>(int, int, const double *, long, double *, long, cudaStream_t);
 template void trsm_llu_small_dev<float>(int, int, const float *, long, float *, long, cudaStream_t);
