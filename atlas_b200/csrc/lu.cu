@@ -24,6 +24,8 @@
 #include <cooperative_groups.h>
 #include "common.cuh"
 #include "kernels.h"
+#include "pivot.cuh"
+#include "cluster.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -211,8 +213,6 @@ getf2_cluster_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restr
 // first maximum, like cblas_idamax); a NaN entry ranks below every number.
 // One CTA's candidate for one column as it lands in every CTA's shared
 // memory: a whole number of 16-byte units, each sent by one st.async.
-template <typename T>
-using PivKey = typename std::conditional<sizeof(T) == 8, unsigned long long, unsigned>::type;
 template <typename T, int NB>
 struct __align__(16) PanelSlot {
   T row[NB];
@@ -221,70 +221,6 @@ struct __align__(16) PanelSlot {
   T rcp;          // 1 / (candidate value), computed by the sender off the critical path
   T lm;           // the sender's pending multiplier: the row is row - lm * u (see below)
 };
-
-// Candidates are compared through one integer key: |value|'s bit pattern + 1
-// (non-negative IEEE values order like their bit patterns), 0 for a NaN or
-// for "no candidate"; ties go to the lowest row position.  A warp's arg-max
-// is then three redux instructions instead of a shuffle tree.
-template <typename T>
-__device__ __forceinline__ unsigned long long pivot_key(T v) {
-  const T t = fabs(v);
-  if (!(t >= T(0))) return 0ull;
-  if (sizeof(T) == 8) return (unsigned long long)__double_as_longlong((double)t) + 1ull;
-  return (unsigned long long)__float_as_uint((float)t) + 1ull;
-}
-__device__ __forceinline__ void warp_argmax_key(unsigned &key, unsigned &pos) {  // FP32 keys fit 32 bits
-  const unsigned m = __reduce_max_sync(0xffffffffu, key);
-  pos = __reduce_min_sync(0xffffffffu, key == m ? pos : 0xffffffffu);
-  key = m;
-}
-__device__ __forceinline__ void warp_argmax_key(unsigned long long &key, unsigned &pos) {
-  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-  const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
-  const bool eq = hi == mhi && lo == mlo;
-  pos = __reduce_min_sync(0xffffffffu, eq ? pos : 0xffffffffu);
-  key = ((unsigned long long)mhi << 32) | mlo;
-}
-
-// Lane of the warp's largest key (lowest pos among equal keys).  Usually
-// the high 32 bits of the largest key occur in one lane only: one redux and
-// one ballot then settle it.
-template <typename K>
-__device__ __forceinline__ int warp_argmax_lane(K key, unsigned pos) {
-  const unsigned hi = sizeof(K) == 8 ? (unsigned)((unsigned long long)key >> 32) : (unsigned)key;
-  const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned m = __ballot_sync(0xffffffffu, hi == mhi);
-  if ((m & (m - 1)) == 0) return __ffs(m) - 1;
-  K k = key;
-  unsigned p = pos;
-  warp_argmax_key(k, p);
-  return __ffs(__ballot_sync(0xffffffffu, key == k && pos == p)) - 1;
-}
-
-__device__ __forceinline__ void cluster_arrive() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() {
-  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ uint32_t mapa_u32(uint32_t a, int rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  return r;
-}
-// one-way 16-byte store into another CTA's shared memory that completes a
-// transaction on that CTA's mbarrier (no fence, no round trip)
-__device__ __forceinline__ void st_async16(uint32_t addr, uint4 v, uint32_t mbar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
-               ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(mbar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t a, uint32_t parity) {
-  uint32_t ok;
-  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-               " selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(a), "r"(parity) : "memory");
-  return ok != 0;
-}
 
 // U12 = L11^-1 A12 for the panel kernels: L11 = the unit lower MN x MN top
 // of the factored panel, A12 the top MN rows of the right columns.  Warp gw

@@ -22,6 +22,8 @@
 #include <cooperative_groups.h>
 #include "common.cuh"
 #include "kernels.h"
+#include "chol_blocks.cuh"
+#include "cluster.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -30,12 +32,6 @@ namespace {
 
 constexpr int QT = 512;
 constexpr int NBQ_MAX = 128;  // widest panel factored in one piece (wider panels: two halves)
-
-template <int NB>
-struct QPub {
-  double s[NB];    // this CTA's partial dot products
-  double row[NB];  // row j (published by its owner, CTA 0)
-};
 
 // lane l returns sum over the warp of v[l % NB]; v is destroyed
 template <int NB>
@@ -56,19 +52,38 @@ __device__ __forceinline__ double warp_reduce_scatter(double (&v)[NB], int lane)
   return r;
 }
 
+// Rows are held shifted -- a[.][0] is the current column -- so the column loop
+// is one small body.  Per column every CTA sends its partial dot products
+// straight into every CTA's shared memory (st.async, counted by the receiver's
+// mbarrier): a cluster barrier there also waits for the multipliers' global
+// stores, and remote reads after it cost another round trip.  One warp then
+// forms beta, tau and the update row w, and every thread applies it.  Waits
+// are bounded (1 s, g_qr_timeout).  16 columns of 16384 rows: 72 us with the
+// barrier, the remote reads and the columns unrolled; 34 us now.
+__device__ int g_qr_timeout = 0;
 template <int NB, int RPT>
 __global__ void __launch_bounds__(QT, 1)
 geqr2_cluster_kernel(int M, int ncols, double *__restrict__ A, long lda, double *__restrict__ tau) {
+  static_assert(NB <= 32 && 16 * NB <= QT, "one lane per column, one thread per (CTA, column)");
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks(), crank = (int)cl.block_rank();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int TOT = C * QT;
   const int K = min(M, ncols);
 
-  __shared__ QPub<NB> pub[2];
+  __shared__ double part[2][16][NB];           // every CTA's partial dot products, by column parity
+  __shared__ double prow[2][NB];               // row j
+  __shared__ double own_row[2][NB];            // CTA 0: row j before it is sent
   __shared__ double red[QT / 32][NB];
-  __shared__ double ssum[NB];
-  __shared__ double srow[NB];
+  __shared__ __align__(16) double sw[NB];      // the update row: w = v^T A
+  __shared__ double s_tau, s_scale, s_beta;
+  __shared__ __align__(8) unsigned long long mbar[2];
+  const uint32_t mb[2] = {smem_u32(&mbar[0]), smem_u32(&mbar[1])};
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb[0]));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb[1]));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
 
   double a[RPT][NB];
   int rows[RPT];
@@ -79,80 +94,123 @@ geqr2_cluster_kernel(int M, int ncols, double *__restrict__ A, long lda, double 
 #pragma unroll
     for (int k = 0; k < NB; k++) a[q][k] = (r < M && k < ncols) ? A[r + (long)k * lda] : 0.0;
   }
+  cl.sync();  // every CTA's barriers exist before anyone sends
 
-#pragma unroll
-  for (int j = 0; j < NB; j++) {
-    if (j >= K) break;
+#pragma unroll 1
+  for (int j = 0; j < K; j++) {
     const int b = j & 1;
+    const uint32_t mbj = b ? mb[1] : mb[0];
+    if (tid == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbj), "r"((C + 1) * NB * 8) : "memory");
     // partial dot products of column j with columns j.. over my rows below j
-    double p[NB];
+    constexpr int H = NB < 16 ? NB : 16;  // columns summed at a time (registers)
 #pragma unroll
-    for (int k = 0; k < NB; k++) p[k] = 0.0;
+    for (int k0 = 0; k0 < NB; k0 += H) {
+      double p[H];
 #pragma unroll
-    for (int q = 0; q < RPT; q++) {
-      if (rows[q] > j && rows[q] < M) {
-#pragma unroll
-        for (int k = j; k < NB; k++) p[k] = fma(a[q][j], a[q][k], p[k]);
-      }
-      if (rows[q] == j) {
-#pragma unroll
-        for (int k = 0; k < NB; k++) pub[b].row[k] = a[q][k];
-      }
-    }
-    double ws = warp_reduce_scatter<NB>(p, lane);
-    if (lane < NB) red[warp][lane] = ws;
-    __syncthreads();
-    if (tid < NB) {
-      double t = 0.0;
-#pragma unroll
-      for (int w = 0; w < QT / 32; w++) t += red[w][tid];
-      pub[b].s[tid] = t;
-    }
-    cl.sync();
-    // gather every CTA's partial sums and row j
-    if (tid < NB) {
-      double t = 0.0;
-      for (int r = 0; r < C; r++) t += cl.map_shared_rank(&pub[b], r)->s[tid];
-      ssum[tid] = t;
-      srow[tid] = cl.map_shared_rank(&pub[b], 0)->row[tid];
-    }
-    __syncthreads();
-    const double alpha = srow[j], xn2 = ssum[j];
-    double t_ = 0.0, beta = alpha, scale = 0.0;
-    if (xn2 != 0.0) {
-      const double bp = sqrt(fma(alpha, alpha, xn2));
-      beta = alpha >= 0.0 ? -bp : bp;
-      t_ = (beta - alpha) / beta;
-      scale = 1.0 / (alpha - beta);
-    }
-    if (crank == 0 && tid == 0) tau[j] = t_;
-    if (t_ != 0.0) {
+      for (int k = 0; k < H; k++) p[k] = 0.0;
 #pragma unroll
       for (int q = 0; q < RPT; q++) {
-        if (rows[q] > j && rows[q] < M) {
-          const double v = a[q][j] * scale;
-          a[q][j] = v;
-          const double tv = t_ * v;
+        const double f = rows[q] > j ? a[q][0] : 0.0;  // rows past M hold zeros
 #pragma unroll
-          for (int k = j + 1; k < NB; k++) a[q][k] = fma(-tv, fma(scale, ssum[k], srow[k]), a[q][k]);
-        } else if (rows[q] == j) {
-          a[q][j] = beta;
+        for (int k = 0; k < H; k++) p[k] = fma(f, a[q][k0 + k], p[k]);
+      }
+      const double ws = warp_reduce_scatter<H>(p, lane);
+      if (lane < H) red[warp][k0 + lane] = ws;
+    }
+    if (rows[0] == j) {  // rows below NB are CTA 0's first ones
 #pragma unroll
-          for (int k = j + 1; k < NB; k++) a[q][k] = fma(-t_, fma(scale, ssum[k], srow[k]), a[q][k]);
+      for (int k = 0; k < NB; k++) own_row[b][k] = a[0][k];
+    }
+    __syncthreads();
+    if (tid < C * NB) {  // thread (CTA, column): this CTA's sum to that CTA
+      const int dst = tid / NB, k = tid % NB;
+      double t[QT / 32];
+#pragma unroll
+      for (int w = 0; w < QT / 32; w++) t[w] = red[w][k];
+#pragma unroll
+      for (int h = QT / 64; h >= 1; h >>= 1)
+#pragma unroll
+        for (int w = 0; w < h; w++) t[w] += t[w + h];
+      const uint32_t to = mapa_u32(mbj, dst);
+      st_async8(mapa_u32(smem_u32(&part[b][crank][k]), dst), t[0], to);
+      if (crank == 0) st_async8(mapa_u32(smem_u32(&prow[b][k]), dst), own_row[b][k], to);
+    }
+    if (warp == 0) {
+      const uint32_t parity = (j >> 1) & 1;
+      if (!mbar_try_wait(mbj, parity)) {
+        uint64_t t0, t1;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+        while (!mbar_try_wait(mbj, parity)) {
+          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+          if (t1 - t0 > 1000000000ull) { atomicExch(&g_qr_timeout, 1); break; }
         }
       }
-    }
-    // ssum/srow/red are rewritten next column only after two more barriers
-  }
+      __syncwarp();
+      const int k = lane % NB;
+      double t[16];
 #pragma unroll
-  for (int q = 0; q < RPT; q++) {
-    if (rows[q] < M) {
+      for (int r = 0; r < 16; r++) t[r] = r < C ? part[b][r][k] : 0.0;
 #pragma unroll
-      for (int k = 0; k < NB; k++)
-        if (k < ncols) A[rows[q] + (long)k * lda] = a[q][k];
+      for (int h = 8; h >= 1; h >>= 1)
+#pragma unroll
+        for (int r = 0; r < h; r++) t[r] += t[r + h];
+      const double row = prow[b][k], sum = t[0];
+      const double alpha = __shfl_sync(0xffffffffu, row, 0), xn2 = __shfl_sync(0xffffffffu, sum, 0);
+      double t_ = 0.0, beta = alpha, scale = 0.0;
+      if (xn2 != 0.0) {
+        const double bp = sqrt(fma(alpha, alpha, xn2));
+        beta = alpha >= 0.0 ? -bp : bp;
+        t_ = (beta - alpha) / beta;
+        scale = 1.0 / (alpha - beta);
+      }
+      if (lane < NB) sw[lane] = fma(scale, sum, row);
+      if (lane == 0) {
+        s_tau = t_;
+        s_scale = scale;
+        s_beta = beta;
+        if (crank == 0) tau[j] = t_;
+      }
     }
+    __syncthreads();
+    const double t_ = s_tau, scale = s_scale;
+#pragma unroll
+    for (int q = 0; q < RPT; q++) {
+      // row j keeps its place from here on: a[0][k] is R(j, j + k)
+      const bool below = rows[q] > j, diag = rows[q] == j;
+      if (t_ != 0.0) {
+        const double v = a[q][0] * scale, f = diag ? t_ : t_ * v;
+        if (diag) {
+          a[q][0] = s_beta;
+#pragma unroll
+          for (int k = 1; k < NB; k++) a[q][k] = fma(-f, sw[k], a[q][k]);
+        } else if (below) {
+          if (rows[q] < M) A[rows[q] + (long)j * lda] = v;
+#pragma unroll
+          for (int k = 0; k < NB; k += 2) {
+            const double2 w = *reinterpret_cast<const double2 *>(sw + k);
+            if (k > 0) a[q][k - 1] = fma(-f, w.x, a[q][k]);
+            a[q][k] = fma(-f, w.y, a[q][k + 1]);
+          }
+          a[q][NB - 1] = 0.0;
+        }
+      } else if (below) {  // H = I: the column below the diagonal is zero already
+        if (rows[q] < M) A[rows[q] + (long)j * lda] = a[q][0];
+#pragma unroll
+        for (int k = 1; k < NB; k++) a[q][k - 1] = a[q][k];
+        a[q][NB - 1] = 0.0;
+      }
+    }
+    // part and prow of this parity: a peer sends column j + 2 only after it has
+    // column j + 1 of every CTA, which each sends after reading column j;
+    // sw and red are rewritten only after another barrier
   }
-  cl.sync();
+  if (rows[0] < K) {  // R's rows
+#pragma unroll
+    for (int k = 0; k < NB; k++)
+      if (rows[0] + k < ncols) A[rows[0] + (long)(rows[0] + k) * lda] = a[0][k];
+  }
+  cl.sync();  // nobody exits while a peer may still write its shared memory
 }
 
 // Fallback for panels taller than a cluster holds: one CTA in global memory.
@@ -287,26 +345,27 @@ __global__ void extract_v_kernel(int M, int k, const double *P, long ldp, double
 // runs on the 16-column diagonal blocks (one warp each, all at once); the
 // blocks are then merged pairwise, 16 -> 32 -> 64 -> 128, with the identity
 // H1 H2 = I - [V1 V2] [T1, -T1 (V1^T V2) T2; 0, T2] [V1 V2]^T, i.e.
-// T12 = -T1 G12 T2 (two small products in shared memory per level).
+// T12 = -T1 G12 T2 (two products on the FP64 tensor cores per level; as scalar
+// dot products they made up most of the 87 us at k = 128; 27 us now).
 // G's strictly upper part is overwritten in place by T's.
-constexpr int LFT_LD = NBQ_MAX + 1;
+constexpr int LFT_LD = NBQ_MAX + 4;  // 4 (mod 16): the MMA's 8 x 4 fragments fall in distinct banks
 __global__ void __launch_bounds__(256) larft_kernel(int k, const double *G, long ldg, const double *tau, double *T,
                                                     long ldt) {
   extern __shared__ double lft_smem[];
   double *S = lft_smem;                      // k x k, ld LFT_LD: G, then T
-  double *W = lft_smem + NBQ_MAX * LFT_LD;   // products G12 T2 of one level (<= NBQ_MAX^2 / 4 doubles)
+  double *W = lft_smem + NBQ_MAX * LFT_LD;   // products G12 T2 of one level, (r, c) at r + c (h + 4) per pair
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int base = 0; base < k * k; base += 256 * 8) {  // eight loads in flight per thread
-    double v[8];
+  for (int base = 0; base < NBQ_MAX * NBQ_MAX; base += 256 * 16) {  // sixteen loads in flight per thread
+    double v[16];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int idx = base + u * 256 + tid, r = idx % k, c = idx / k;
-      v[u] = (idx < k * k && r < c) ? G[r + (long)c * ldg] : 0.0;
+    for (int u = 0; u < 16; u++) {
+      const int idx = base + u * 256 + tid, r = idx % NBQ_MAX, c = idx / NBQ_MAX;
+      v[u] = r < c && c < k ? G[r + (long)c * ldg] : 0.0;  // zero past k: whole blocks are multiplied below
     }
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
+    for (int u = 0; u < 16; u++) {
       const int idx = base + u * 256 + tid;
-      if (idx < k * k) S[idx % k + (idx / k) * LFT_LD] = v[u];
+      S[idx % NBQ_MAX + (idx / NBQ_MAX) * LFT_LD] = v[u];
     }
   }
   __syncthreads();
@@ -326,31 +385,30 @@ __global__ void __launch_bounds__(256) larft_kernel(int k, const double *G, long
     }
   }
   __syncthreads();
+  const int g = lane >> 2, t = lane & 3;
   for (int h = 16; h < k; h *= 2) {          // merge sibling blocks of order h
-    const int npair = (k + 2 * h - 1) / (2 * h);
-    // W_p = G12 T2 (h x h2): G12 = S[o : o+h, o+h : o+h+h2], T2 upper h2 x h2
-    for (int idx = tid; idx < npair * h * h; idx += 256) {
-      const int p = idx / (h * h), e = idx % (h * h), r = e % h, c = e / h;
-      const int o = 2 * h * p, h2 = min(h, k - o - h);
-      if (h2 <= 0 || c >= h2) continue;
-      const double *G12 = S + o + (o + h) * LFT_LD, *T2 = S + (o + h) + (o + h) * LFT_LD;
-      double v = 0.0;
-      for (int q = 0; q <= c; q++) v = fma(G12[r + q * LFT_LD], T2[q + c * LFT_LD], v);
-      W[p * h * h + r + c * h] = v;
+    const int npair = (k + 2 * h - 1) / (2 * h), nt = h / 8, tiles = npair * nt * nt, ldw = h + 4;
+    // 8 x 8 tiles over the warps, FP64 MMAs: W_p = G12 T2, then T12 = -T1 W_p
+    // (T1, T2 upper triangular: the zero part of the k range left out)
+    for (int pass = 0; pass < 2; pass++) {
+      for (int e = warp; e < tiles; e += 8) {
+        const int p = e / (nt * nt), r = e % nt * 8, c = e / nt % nt * 8, o = 2 * h * p;
+        const double *X = pass ? S + o + o * LFT_LD : S + o + (o + h) * LFT_LD;
+        double *Wp = W + p * h * ldw;
+        const double *Y = pass ? Wp : S + (o + h) + (o + h) * LFT_LD;
+        const int ldy = pass ? ldw : LFT_LD;
+        double acc[2] = {0.0, 0.0};
+#pragma unroll 4
+        for (int q = pass ? r : 0; q < (pass ? h : c + 8); q += 4)
+          cholb::dmma_8x8x4(acc, X[r + g + (q + t) * LFT_LD], Y[q + t + (c + g) * ldy]);
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          if (pass) S[o + r + g + (o + h + c + 2 * t + i) * LFT_LD] = -acc[i];
+          else Wp[r + g + (c + 2 * t + i) * ldw] = acc[i];
+        }
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    // T12 = -T1 W_p, T1 upper h x h
-    for (int idx = tid; idx < npair * h * h; idx += 256) {
-      const int p = idx / (h * h), e = idx % (h * h), r = e % h, c = e / h;
-      const int o = 2 * h * p, h2 = min(h, k - o - h);
-      if (h2 <= 0 || c >= h2) continue;
-      const double *T1 = S + o + o * LFT_LD;
-      const double *Wp = W + p * h * h;
-      double v = 0.0;
-      for (int q = r; q < h; q++) v = fma(T1[r + q * LFT_LD], Wp[q + c * h], v);
-      S[(o + r) + (o + h + c) * LFT_LD] = -v;
-    }
-    __syncthreads();
   }
   for (int idx = tid; idx < k * k; idx += 256) {
     const int r = idx % k, c = idx / k;
@@ -358,7 +416,7 @@ __global__ void __launch_bounds__(256) larft_kernel(int k, const double *G, long
   }
 }
 
-constexpr size_t larft_smem_bytes() { return sizeof(double) * ((size_t)NBQ_MAX * LFT_LD + NBQ_MAX * NBQ_MAX / 4); }
+constexpr size_t larft_smem_bytes() { return sizeof(double) * ((size_t)NBQ_MAX * LFT_LD + NBQ_MAX / 2 * (NBQ_MAX / 2 + 4)); }
 
 // ---- Applying a leaf's reflectors to the rest of its panel.  The leaf is
 // m x kb (kb <= 32) with V its unit lower trapezoid, C the n2 panel columns
@@ -367,8 +425,9 @@ constexpr size_t larft_smem_bytes() { return sizeof(double) * ((size_t)NBQ_MAX *
 // is too small to fill the GPU:
 //   1. qr_leaf_gram_kernel: per-CTA partial sums of V^T [V C] (kb x (kb+n2));
 //   2. qr_leaf_reduce_kernel: the partials summed in a fixed order;
-//   3. qr_leaf_apply_kernel: every CTA forms T from G = V^T V (the column
-//      recurrence) and Y = T^T (V^T C), then C -= V Y for its rows.
+//   3. qr_leaf_apply_kernel: every CTA forms Y = T^T (V^T C) by a forward
+//      substitution with T^-1 = striu(V^T V) + diag(1 / tau), then C -= V Y
+//      for its rows.
 // V is read straight from the factored leaf (unit diagonal and zeros above
 // it applied on the fly).
 constexpr int QL_GRID = 256;         // CTAs of the partial-sum pass (at most)
@@ -381,42 +440,51 @@ __device__ __forceinline__ double leaf_v(const double *L, long lda, int r, int a
 template <int KB>
 __global__ void __launch_bounds__(256) qr_leaf_gram_kernel(int m, int kb, int ncol, const double *L, long lda,
                                                            int rpc, double *part) {
-  __shared__ double X[NBQ_MAX][33];  // 32 rows of [V C], column by column
-  constexpr int SB = 256 / KB, NJ = NBQ_MAX / SB;
-  const int tid = threadIdx.x, a = tid % KB, b0 = tid / KB;
-  double acc[NJ];
+  // 32 rows of [V C], column by column; 4 (mod 16): the MMA's 8 x 4 fragments fall in distinct banks
+  constexpr int LX = 36, MT = KB / 8;
+  __shared__ double X[NBQ_MAX * LX];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  // warp w: columns 16 w .. 16 w + 15 of [V C] against all KB columns of V
+  double acc[MT][2][2];
 #pragma unroll
-  for (int j = 0; j < NJ; j++) acc[j] = 0.0;
+  for (int x = 0; x < MT; x++)
+#pragma unroll
+    for (int y = 0; y < 2; y++) acc[x][y][0] = acc[x][y][1] = 0.0;
   const int rb = blockIdx.x * rpc, re = min(m, rb + rpc);
+#pragma unroll 1
   for (int r0 = rb; r0 < re; r0 += 32) {
     __syncthreads();
     double v[NBQ_MAX / 8];  // all of this thread's loads in flight before the stores
-    const int r = r0 + (tid & 31);
+    const int r = r0 + lane;
+    const double *Lr = L + r + (long)warp * lda;
+#pragma unroll
+    for (int u = 0; u < NBQ_MAX / 8; u++) v[u] = r < re && warp + 8 * u < ncol ? Lr[(long)(8 * u) * lda] : 0.0;
 #pragma unroll
     for (int u = 0; u < NBQ_MAX / 8; u++) {
-      const int c = (tid >> 5) + 8 * u;
-      v[u] = 0.0;
-      if (r < re && c < ncol) v[u] = c < kb ? leaf_v(L, lda, r, c) : L[r + (long)c * lda];
-    }
-#pragma unroll
-    for (int u = 0; u < NBQ_MAX / 8; u++) {
-      const int c = (tid >> 5) + 8 * u;
-      if (c < ncol) X[c][tid & 31] = v[u];
+      const int c = warp + 8 * u;  // V's diagonal is one, the entries above it zero
+      X[c * LX + lane] = c < kb && r <= c ? (r == c && r < re ? 1.0 : 0.0) : v[u];
     }
     __syncthreads();
-    const int nr = min(32, re - r0);
-    for (int rr = 0; rr < nr; rr++) {
-      const double xa = a < kb ? X[a][rr] : 0.0;
+#pragma unroll 2
+    for (int k = 0; k < 32; k += 4) {
+      double av[MT], bv[2];
 #pragma unroll
-      for (int j = 0; j < NJ; j++) {
-        const int b = b0 + SB * j;
-        if (b < ncol) acc[j] = fma(xa, X[b][rr], acc[j]);
-      }
+      for (int x = 0; x < MT; x++) av[x] = 8 * x + g < kb ? X[(8 * x + g) * LX + k + t] : 0.0;
+#pragma unroll
+      for (int y = 0; y < 2; y++) bv[y] = X[(16 * warp + 8 * y + g) * LX + k + t];
+#pragma unroll
+      for (int x = 0; x < MT; x++)
+#pragma unroll
+        for (int y = 0; y < 2; y++) cholb::dmma_8x8x4(acc[x][y], av[x], bv[y]);
     }
   }
   double *P = part + (size_t)blockIdx.x * QL_OUT;
 #pragma unroll
-  for (int j = 0; j < NJ; j++) P[a + (b0 + SB * j) * KB] = acc[j];
+  for (int x = 0; x < MT; x++)
+#pragma unroll
+    for (int y = 0; y < 2; y++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) P[8 * x + g + (16 * warp + 8 * y + 2 * t + e) * KB] = acc[x][y][e];
 }
 
 // P[o] = sum over g < ngrid of part[g][o], o < nout: eight partial sums per
@@ -441,7 +509,7 @@ template <int KB>
 __global__ void __launch_bounds__(256) qr_leaf_apply_kernel(int m, int kb, int n2, double *L, long lda,
                                                             const double *P, const double *tau) {
   constexpr int RPT = KB == 8 ? 4 : 2;  // rows per thread
-  __shared__ double sT[KB][KB + 1];
+  __shared__ double sG[KB * (KB + 1)];    // G = V^T V, row q at q * (KB + 1)
   __shared__ double sW[KB][NBQ_MAX + 1];  // W = V^T C, then Y = T^T W in its place
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   for (int base = 0; base < KB * (kb + n2); base += 256 * 8) {  // eight loads in flight per thread
@@ -456,40 +524,26 @@ __global__ void __launch_bounds__(256) qr_leaf_apply_kernel(int m, int kb, int n
     for (int u = 0; u < 8; u++) {
       const int idx = base + u * 256 + tid, a = idx % KB, b = idx / KB;
       if (idx >= tot) continue;
-      if (b < kb) sT[a][b] = v[u];  // G = V^T V for now
+      if (b < kb) sG[a * (KB + 1) + b] = v[u];
       else sW[a][b - kb] = v[u];
     }
   }
   __syncthreads();
-  if (w == 0) {  // T from G (upper; the recurrence overwrites G's strictly upper part)
-    for (int i = 0; i < kb; i++) {
-      double val = 0.0;
-      if (lane < i) {
-        for (int q = lane; q < i; q++) val = fma(sT[lane][q], sT[q][i], val);
-        val *= -tau[i];
-      }
-      __syncwarp();
-      if (lane < i) sT[lane][i] = val;
-      if (lane == i) sT[i][i] = tau[i];
-      __syncwarp();
+  // Y = T^T W without T: T^-1 has 1/tau on its diagonal and G above it, so
+  // y_q = tau_q (w_q - sum over a < q of G(a, q) y_a), one thread per column
+  // (x shifted: x[0] is the current entry)
+  if (tid < n2) {
+    double x[KB];
+#pragma unroll
+    for (int a = 0; a < KB; a++) x[a] = sW[a][tid];
+#pragma unroll 1
+    for (int q = 0; q < kb; q++) {
+      const double y = tau[q] * x[0], *Gq = sG + q * (KB + 1) + q;
+      sW[q][tid] = y;
+      const int left = KB - q;  // entries of x still to come
+#pragma unroll
+      for (int r = 1; r < KB; r++) x[r - 1] = r < left ? fma(-Gq[r < left ? r : 0], y, x[r]) : 0.0;
     }
-  }
-  __syncthreads();
-  constexpr int NY = KB * NBQ_MAX / 256;  // Y = T^T W: outputs per thread, held until W is read
-  double y[NY];
-#pragma unroll
-  for (int u = 0; u < NY; u++) {
-    const int idx = tid + 256 * u, a = idx % KB, c = idx / KB;
-    double v = 0.0;
-    if (a < kb && c < n2)
-      for (int q = 0; q <= a; q++) v = fma(sT[q][a], sW[q][c], v);
-    y[u] = v;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int u = 0; u < NY; u++) {
-    const int idx = tid + 256 * u;
-    sW[idx % KB][idx / KB] = y[u];
   }
   __syncthreads();
   // C -= V Y: 32 lanes x RPT rows by 8 column groups per CTA tile of 32 * RPT rows
