@@ -8,9 +8,9 @@
 // launch is made of small problems), and each problem is handled entirely by
 // one CTA.  Cholesky: 16 x 16 tiles in shared memory, right-hand sides carried
 // through the factorization, one launch per size bucket.  LU: 16-column
-// pivoted panels in shared memory, the trailing update on the FP64 tensor
-// cores in global memory, then the solves in blocks of 16 rows.  Nothing waits
-// on another CTA, so a launch cannot stall.
+// pivoted panels in registers, the trailing update on the FP64 tensor cores in
+// global memory, right-hand sides carried along too.  Nothing waits on another
+// CTA, so a launch cannot stall.
 #include <algorithm>
 #include <cfloat>
 #include <climits>
@@ -20,13 +20,13 @@
 #include "chol_blocks.cuh"
 #include "chol_tiles.cuh"
 #include "kernels.h"
+#include "pivot.cuh"
 #include "staging.h"
 #include "../../include/atlas_b200.h"
 
 namespace atlb {
 namespace {
 
-constexpr int BT = 256;       // threads per CTA
 constexpr int MAXN = 256;
 
 struct Prob {
@@ -36,69 +36,7 @@ struct Prob {
   int n, lda, ldb, nrhs;
 };
 
-// dst (rows x cols, ld ldd, shared memory) = src (ld lds, global), eight
-// loads in flight per thread before their stores (a plain strided loop would
-// wait for each load in turn)
-__device__ __forceinline__ void stage_tile(double *dst, int ldd, const double *src, long lds, int rows, int cols) {
-  const int tot = rows * cols, tid = threadIdx.x;
-  for (int base = 0; base < tot; base += BT * 8) {
-    double v[8];
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int idx = base + u * BT + tid;
-      v[u] = idx < tot ? src[idx % rows + (long)(idx / rows) * lds] : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int idx = base + u * BT + tid;
-      if (idx < tot) dst[idx % rows + (idx / rows) * ldd] = v[u];
-    }
-  }
-}
-
 // ---------------------------------------------------------------- Cholesky
-
-// Triangular solve of one right-hand side held in shared memory (b, n <=
-// MAXN) with T in shared or global memory (ld ldt): op(T) x = b, op(T)
-// lower (forward) or upper (backward) triangular, T itself read transposed
-// when trans.  Blocks of 16 rows: warp 0 solves a block's 16 x 16 diagonal
-// part (x_c by shuffle), then every thread subtracts the block's
-// contribution from one remaining row -- two barriers per block instead of
-// two per row.
-__device__ void tri_solve_smem(const double *T, long ldt, int n, double *b, bool lower, bool unit, bool trans) {
-  const int tid = threadIdx.x;
-  auto at = [&](int i, int c) { return trans ? T[c + (long)i * ldt] : T[i + (long)c * ldt]; };
-  const int nblk = (n + 15) / 16;
-  for (int t = 0; t < nblk; t++) {
-    const int b0 = lower ? 16 * t : 16 * (nblk - 1 - t), bs = min(16, n - b0);
-    if (tid < 32) {
-      const int i = tid;
-      double x = i < bs ? b[b0 + i] : 0.0;
-      if (lower) {
-        for (int c = 0; c < bs; c++) {
-          if (!unit && i == c) x = x / at(b0 + c, b0 + c);
-          const double xc = __shfl_sync(0xffffffffu, x, c);
-          if (i > c && i < bs) x = fma(-at(b0 + i, b0 + c), xc, x);
-        }
-      } else {
-        for (int c = bs - 1; c >= 0; c--) {
-          if (!unit && i == c) x = x / at(b0 + c, b0 + c);
-          const double xc = __shfl_sync(0xffffffffu, x, c);
-          if (i < c) x = fma(-at(b0 + i, b0 + c), xc, x);
-        }
-      }
-      if (i < bs) b[b0 + i] = x;
-    }
-    __syncthreads();
-    const int r0 = lower ? b0 + bs : 0, r1 = lower ? n : b0;
-    for (int i = r0 + tid; i < r1; i += BT) {
-      double acc = b[i];
-      for (int c = 0; c < bs; c++) acc = fma(-at(i, b0 + c), b[b0 + c], acc);
-      b[i] = acc;
-    }
-    __syncthreads();
-  }
-}
 
 // Batched Cholesky + solve: each CTA takes whole problems off the list, the
 // matrix as 16 x 16 tiles in shared memory (chol_tiles.cuh).  One launch per
@@ -148,287 +86,381 @@ batched_posv_kernel(const Prob *__restrict__ probs, const int *__restrict__ orde
 
 // ---------------------------------------------------------------- LU
 
-// Blocked LU with partial pivoting of one problem by one CTA, the matrix in
-// place in global memory (L2-resident at these orders), ATL_getrfC's
-// right-looking step on panels of LPW columns:
-//   1. the panel (rows j..n-1) is staged in shared memory and factored there
-//      column by column: arg-max with the first maximum on ties
-//      (cblas_idamax / ATL_getf2), the interchange inside the panel, the
-//      scaling (by the reciprocal when the pivot is a normal number), the
-//      rank-1 update of the panel's columns right of it;
-//   2. the panel goes back, ipiv[j + c] = j + its pivot row;
-//   3. the panel's interchanges, composed into one row permutation, move
-//      the rows of every column outside the panel (LAPACK's laswp on the
-//      left and right parts) in one gather / scatter pass;
-//   4. U12 = L11^-1 A12 (one thread per column) into global memory and a
-//      shared copy;
-//   5. A22 -= L21 U12 on the FP64 tensor cores (mma.m8n8k4), L21 and U12
-//      from shared memory, A22 read and written in global memory.
-// Returns the first zero pivot (1-based) or 0; the factorization completes
-// either way (LAPACK getrf semantics).
-constexpr int LPW = 16;              // panel width
-constexpr int LU_LDP = cholb::ld_for(MAXN);  // panel ld (rows of the panel, <= MAXN)
-constexpr int LU_LDU = LPW + 4;      // U12 copy, stored U(q, k) at k * LU_LDU + q
-constexpr int LU_CHUNK = 64;         // columns per gather / scatter pass of the interchanges
+// Blocked LU with partial pivoting of one problem by one CTA, ATL_getrfC's
+// right-looking step on panels of 16 columns, the trailing matrix in place in
+// global memory (L2-resident at these orders):
+//   1. the panel is factored in registers, one row per thread.  A column
+//      costs one barrier: every warp's best row (largest |value|, lowest
+//      current position on ties = cblas_idamax / ATL_getf2) goes to shared
+//      memory before it, every thread picks the winner after it.  Rows do not
+//      move: each carries its current position;
+//   2. one thread per column outside the panel, right-hand sides included,
+//      applies the panel's interchanges (only the top 16 rows and the pivot
+//      rows change: one gather, one scatter) and, right of the panel, solves
+//      U12 = L11^-1 A12 in registers;
+//   3. A22 -= L21 U12 on the FP64 tensor cores, L21 and U12 from shared
+//      memory, the next part of A22 loaded under the products.
+// Up to eight right-hand sides ride along in shared memory, which makes the
+// forward substitution part of the factorization.  What bounds it: the chain
+// of columns (about 16 x 500 cycles a panel) and the L2 round trips of steps
+// 2 and 3, so several CTAs share an SM: buckets of orders <= 64, 128, 256
+// with 64, 128, 256 threads.
+//
+// 10,000 problems of orders 8..256 with one right-hand side, B200: getrf and
+// getrs kernels 14.5 + 3.0 ms before (two barriers and a shared-memory rank-1
+// update per column, interchanges and U12 as separate passes, a solve with
+// loads of the factor on its chain), 11.1 ms now for both.
+constexpr int LPW = 16;         // panel width
+constexpr int LU_RHS = 8;       // right-hand sides carried along
+constexpr int LU_LDU = LPW + 4; // U12 copy, U(q, k) at k * LU_LDU + q
+constexpr int DLD = LPW + 1;
 
+template <int NT>  // threads = largest order
 struct LuSmem {
-  double P[LU_LDP * LPW];
-  double U[MAXN * LU_LDU];
-  double stage[2 * LPW * LU_CHUNK];
-  double wv[BT / 32];
-  int wi[BT / 32];
-  int piv[LPW];
-  int who[MAXN];
-  int src[2 * LPW], dst[2 * LPW];
-  int nmove, fail;
+  static constexpr int LDP = NT + 4;  // 4 (mod 16): the MMA's 8 x 4 fragments fall in distinct banks
+  double P[LPW * LDP];                // the factored panel, rows at their final places
+  double U[NT * LU_LDU];
+  double xs[LU_RHS * NT];             // right-hand sides
+  double cand[2][NT / 32][LPW];       // per-warp candidate rows, by column parity
+  unsigned long long ckey[2][NT / 32];
+  int cpos[2][NT / 32];
+  double D[2][LPW * DLD];             // diagonal blocks of the solves, D(r, q) at q * DLD + r
+  int from[LPW], to[LPW];             // row whose content ends at q; where row q's content ends
+  int moved, fail;
 };
 
-// C (mt x nt, global, ldc) -= P (mt x kb, shared, ld lds) U (kb x nt, shared,
-// U(q, k) at k * ldu + q), kb <= LPW: each warp owns a 16 x 32 part of every
-// 64 x 64 block of C (2 x 4 tiles of 8 x 8), accumulators started from C
-__device__ void lu_update_dmma(int mt, int nt, int kb, const double *P, int lds, const double *U, int ldu,
-                               double *C, long ldc) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const int wr = (warp >> 1) * 16, wc = (warp & 1) * 32;
-  for (int ib = 0; ib < mt; ib += 64)
-    for (int kb0 = 0; kb0 < nt; kb0 += 64) {
-      const int r0 = ib + wr, c0 = kb0 + wc;
-      if (r0 >= mt || c0 >= nt) continue;  // warp-uniform
-      double acc[2][4][2];
-#pragma unroll
-      for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++)
-#pragma unroll
-          for (int e = 0; e < 2; e++) {
-            const int i = r0 + 8 * a + g, k = c0 + 8 * b + 2 * t + e;
-            acc[a][b][e] = (i < mt && k < nt) ? C[i + (long)k * ldc] : 0.0;
-          }
-#pragma unroll
-      for (int q = 0; q < LPW; q += 4) {
-        const int qq = q + t;
-        double av[2], bv[4];
-#pragma unroll
-        for (int a = 0; a < 2; a++) {
-          const int i = r0 + 8 * a + g;
-          av[a] = (i < mt && qq < kb) ? -P[i + qq * lds] : 0.0;
-        }
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-          const int k = c0 + 8 * b + g;
-          bv[b] = (k < nt && qq < kb) ? U[k * ldu + qq] : 0.0;
-        }
-#pragma unroll
-        for (int a = 0; a < 2; a++)
-#pragma unroll
-          for (int b = 0; b < 4; b++) cholb::dmma_8x8x4(acc[a][b], av[a], bv[b]);
-      }
-#pragma unroll
-      for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++)
-#pragma unroll
-          for (int e = 0; e < 2; e++) {
-            const int i = r0 + 8 * a + g, k = c0 + 8 * b + 2 * t + e;
-            if (i < mt && k < nt) C[i + (long)k * ldc] = acc[a][b][e];
-          }
-    }
-}
-
-// step 1: partial-pivoting LU of the m x jb panel in shared memory; S.piv[c]
-// = panel-relative pivot row of column c; returns the first zero pivot
-// (1-based, panel-relative) or 0
-__device__ int lu_panel(LuSmem &S, int m, int jb) {
+// step 1.  a[]: this thread's row of the panel (row tid of m, jb <= 16
+// columns); returns its final position.  The row is shifted as columns are
+// finished -- a[0] is always the current column -- so the loop is one small
+// body (unrolled, the sixteen bodies overflow the instruction cache);
+// multipliers, and the U part of a pivot row, go to S.P at the thread's own
+// row, from where the caller takes the finished row.
+template <int NT>
+__device__ __forceinline__ int lu_panel(LuSmem<NT> &S, double (&a)[LPW], int m, int jb, int j0, int *ipiv) {
+  constexpr int NW = NT / 32, LDP = LuSmem<NT>::LDP;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  double *P = S.P;
-  int fail = 0;
+  bool act = tid < m, chosen = false;
+  int pos = tid;
+#pragma unroll 1
   for (int c = 0; c < jb; c++) {
-    double v = -1.0;
-    int vi = INT_MAX;
-    for (int i = c + tid; i < m; i += BT) {
-      const double a = fabs(P[i + c * LU_LDP]);
-      if (a > v) { v = a; vi = i; }   // NaN never wins
-    }
-    for (int o = 16; o; o >>= 1) {
-      const double ov = __shfl_xor_sync(0xffffffffu, v, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, vi, o);
-      if (ov > v || (ov == v && oi < vi)) { v = ov; vi = oi; }
-    }
-    if (lane == 0) { S.wv[warp] = v; S.wi[warp] = vi; }
-    __syncthreads();
-    double best = -1.0;
-    int p = INT_MAX;
-    for (int w = 0; w < BT / 32; w++)
-      if (S.wv[w] > best || (S.wv[w] == best && S.wi[w] < p)) { best = S.wv[w]; p = S.wi[w]; }
-    if (!(best > 0.0)) p = c;  // zero (or NaN) column: no interchange
-    if (tid == 0) S.piv[c] = p;
-    if (p != c && tid < jb) {
-      const double t0 = P[c + tid * LU_LDP];
-      P[c + tid * LU_LDP] = P[p + tid * LU_LDP];
-      P[p + tid * LU_LDP] = t0;
+    const int b = c & 1;
+    // a zero or NaN entry never wins, except that the row at position c
+    // stands in when there is no other candidate (then: no interchange)
+    unsigned long long key = 0;
+    if (act) key = fabs(a[0]) > 0.0 ? pivot_key(a[0]) : (pos == c ? 1ull : 0ull);
+    const int wl = warp_argmax_lane(key, act ? (unsigned)pos : 0xffffffffu);
+    if (lane == wl) {
+      S.ckey[b][warp] = key;
+      S.cpos[b][warp] = act ? pos : INT_MAX;
+#pragma unroll
+      for (int k = 0; k < LPW; k += 2)
+        *reinterpret_cast<double2 *>(&S.cand[b][warp][k]) = make_double2(a[k], a[k + 1]);
     }
     __syncthreads();
-    const double piv = P[c + c * LU_LDP];
-    if (piv == 0.0) {
-      if (!fail) fail = c + 1;
-    } else {
-      const double r = 1.0 / piv;
-      const bool use_r = fabs(piv) >= DBL_MIN;
-      for (int i = c + 1 + tid; i < m; i += BT) {
-        const double l = use_r ? P[i + c * LU_LDP] * r : P[i + c * LU_LDP] / piv;
-        P[i + c * LU_LDP] = l;
-        for (int k = c + 1; k < jb; k++) P[i + k * LU_LDP] = fma(-l, P[c + k * LU_LDP], P[i + k * LU_LDP]);
+    int w = 0;
+    if (NW > 1) w = warp_argmax_lane(lane < NW ? S.ckey[b][lane] : 0ull, lane < NW ? (unsigned)S.cpos[b][lane] : 0xffffffffu);
+    const int p = S.cpos[b][w];
+    const double *u = S.cand[b][w];
+    const double piv = u[0];
+    if (tid == 0) {
+      ipiv[j0 + c] = j0 + p;
+      if (piv == 0.0 && !S.fail) S.fail = j0 + c + 1;
+    }
+    if (act) {
+      if (pos == p) {  // the pivot row: it keeps its place in a[] from here on
+        act = false;
+        chosen = true;
+        pos = c;
+      } else {
+        if (pos == c) pos = p;
+        const bool nz = piv != 0.0;  // a zero pivot leaves the column unscaled and the row unchanged
+        const double l = !nz ? a[0] : fabs(piv) >= DBL_MIN ? a[0] * (1.0 / piv) : a[0] / piv;
+        S.P[c * LDP + tid] = l;
+        if (nz) {
+#pragma unroll
+          for (int k = 0; k < LPW; k += 2) {
+            const double2 v = *reinterpret_cast<const double2 *>(u + k);
+            if (k > 0) a[k - 1] = fma(-l, v.x, a[k]);
+            a[k] = fma(-l, v.y, a[k + 1]);
+          }
+        } else {
+#pragma unroll
+          for (int k = 1; k < LPW; k++) a[k - 1] = a[k];
+        }
+        a[LPW - 1] = 0.0;
       }
     }
-    __syncthreads();
   }
-  return fail;
+  if (chosen) {
+#pragma unroll
+    for (int k = 0; k < LPW; k++)
+      if (pos + k < jb) S.P[(pos + k) * LDP + tid] = a[k];
+  }
+  return pos;
 }
 
-__device__ int lu_blocked(const Prob &pr, LuSmem &S) {
+// step 3: C (mt x nt, global, ldc) -= P (mt x 16, shared) U (16 x nt,
+// shared); each warp takes 16 x 32 parts (2 x 4 MMA tiles), accumulators
+// started from C, the next part's C in flight meanwhile
+template <int NT>
+__device__ __forceinline__ void lu_update(const LuSmem<NT> &S, int mt, int nt, double *C, long ldc) {
+  constexpr int LDP = LuSmem<NT>::LDP;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int rb = (mt + 15) / 16, parts = rb * ((nt + 31) / 32);
+  const double *P = S.P + LPW;  // rows below the diagonal block
+  auto load = [&](int s, double (&v)[2][4][2]) {
+    const int r0 = (s % rb) * 16 + g, c0 = (s / rb) * 32 + 2 * t;
+    const bool in0 = r0 < mt, in1 = r0 + 8 < mt;
+    const double *Cp = C + r0 + (long)c0 * ldc;
+#pragma unroll
+    for (int y = 0; y < 4; y++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const bool in = s < parts && c0 + 8 * y + e < nt;
+        const double *q = Cp + (8 * y + e) * ldc;
+        v[0][y][e] = in && in0 ? q[0] : 0.0;
+        v[1][y][e] = in && in1 ? q[8] : 0.0;
+      }
+  };
+  double nx[2][4][2];
+  load(warp, nx);
+#pragma unroll 1
+  for (int s = warp; s < parts; s += NT / 32) {
+    const int r0 = (s % rb) * 16 + g, c0 = (s / rb) * 32;
+    const double *Pr = P + r0 + t * LDP, *Ur = S.U + (c0 + g) * LU_LDU + t;
+    double acc[2][4][2];
+#pragma unroll
+    for (int x = 0; x < 2; x++)
+#pragma unroll
+      for (int y = 0; y < 4; y++) {
+        acc[x][y][0] = nx[x][y][0];
+        acc[x][y][1] = nx[x][y][1];
+      }
+    load(s + NT / 32, nx);
+#pragma unroll
+    for (int q = 0; q < LPW; q += 4) {
+      double av[2], bv[4];
+      av[0] = -Pr[q * LDP];          // rows past mt and columns past nt: not stored
+      av[1] = -Pr[q * LDP + 8];
+#pragma unroll
+      for (int y = 0; y < 4; y++) bv[y] = Ur[8 * y * LU_LDU + q];
+#pragma unroll
+      for (int x = 0; x < 2; x++)
+#pragma unroll
+        for (int y = 0; y < 4; y++) cholb::dmma_8x8x4(acc[x][y], av[x], bv[y]);
+    }
+    const bool in0 = r0 < mt, in1 = r0 + 8 < mt;
+    double *Cp = C + r0 + (long)(c0 + 2 * t) * ldc;
+#pragma unroll
+    for (int y = 0; y < 4; y++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const bool in = c0 + 8 * y + 2 * t + e < nt;
+        double *q = Cp + (8 * y + e) * ldc;
+        if (in && in0) q[0] = acc[0][y][e];
+        if (in && in1) q[8] = acc[1][y][e];
+      }
+  }
+}
+
+// the factorization of one problem, S.xs (nr right-hand sides, row i of
+// column r at r * NT + i) becoming L^-1 P b; returns the first zero pivot
+// (1-based) or 0 and completes either way (LAPACK getrf semantics)
+template <int NT>
+__device__ __forceinline__ int lu_factor(const Prob &pr, int nr, LuSmem<NT> &S) {
+  constexpr int LDP = LuSmem<NT>::LDP;
   const int tid = threadIdx.x, n = pr.n;
   double *A = pr.A;
   const long lda = pr.lda;
   if (tid == 0) S.fail = 0;
+#pragma unroll 1
   for (int j = 0; j < n; j += LPW) {
-    const int jb = min(LPW, n - j), m = n - j, nt = n - j - jb;
-    stage_tile(S.P, LU_LDP, A + j + (long)j * lda, lda, m, jb);
-    __syncthreads();
-    const int f = lu_panel(S, m, jb);
-    if (tid == 0 && f && !S.fail) S.fail = j + f;
-    for (int idx = tid; idx < m * jb; idx += BT) {
-      const int i = idx % m, c = idx / m;
-      A[(j + i) + (long)(j + c) * lda] = S.P[i + c * LU_LDP];
-    }
-    if (tid < jb) pr.ipiv[j + tid] = j + S.piv[tid];
-    // the panel's interchanges as one row permutation: who[r] = the panel
-    // row whose content ends at row r (panel-relative)
-    for (int r = tid; r < m; r += BT) S.who[r] = r;
-    __syncthreads();
-    if (tid == 0) {
-      for (int c = 0; c < jb; c++) {
-        const int p = S.piv[c];
-        const int t0 = S.who[c];
-        S.who[c] = S.who[p];
-        S.who[p] = t0;
-      }
-      int cnt = 0;
-      for (int c = 0; c < jb; c++) {  // moved rows: the first jb rows and the pivot rows
-        if (S.who[c] != c) { S.dst[cnt] = c; S.src[cnt] = S.who[c]; cnt++; }
-        const int p = S.piv[c];
-        if (p >= jb && S.who[p] != p) {
-          bool seen = false;
-          for (int q = 0; q < cnt; q++) seen = seen || S.dst[q] == p;
-          if (!seen) { S.dst[cnt] = p; S.src[cnt] = S.who[p]; cnt++; }
-        }
-      }
-      S.nmove = cnt;
-    }
-    __syncthreads();
-    const int nmove = S.nmove;
-    if (nmove > 0) {  // gather / scatter over the columns outside the panel, LU_CHUNK at a time
-      const int nout = n - jb;
-      for (int c0 = 0; c0 < nout; c0 += LU_CHUNK) {
-        const int cw = min(LU_CHUNK, nout - c0);
-        for (int e = tid; e < nmove * cw; e += BT) {
-          const int q = e % nmove, cc = c0 + e / nmove, col = cc < j ? cc : cc + jb;
-          S.stage[e] = A[(j + S.src[q]) + (long)col * lda];
-        }
-        __syncthreads();
-        for (int e = tid; e < nmove * cw; e += BT) {
-          const int q = e % nmove, cc = c0 + e / nmove, col = cc < j ? cc : cc + jb;
-          A[(j + S.dst[q]) + (long)col * lda] = S.stage[e];
-        }
-        __syncthreads();
-      }
-    }
-    if (nt > 0) {
-      // U12 = L11^-1 A12, one thread per column
-      for (int k = tid; k < nt; k += BT) {
-        double x[LPW];
-        double *col = A + j + (long)(j + jb + k) * lda;
+    const int jb = min(LPW, n - j), m = n - j, nt = m - jb;
+    double a[LPW];
 #pragma unroll
-        for (int q = 0; q < LPW; q++) x[q] = q < jb ? col[q] : 0.0;
+    for (int k = 0; k < LPW; k++) a[k] = (tid < m && k < jb) ? A[j + tid + (long)(j + k) * lda] : 0.0;
+    if (tid < LPW) {  // identity where the panel has fewer rows
+      S.from[tid] = tid;
+      S.to[tid] = tid;
+    }
+    if (tid == 0) S.moved = 0;
+    __syncthreads();
+    const int pos = lu_panel<NT>(S, a, m, jb, j, pr.ipiv);
 #pragma unroll
+    for (int k = 0; k < LPW; k++) a[k] = (tid < m && k < jb) ? S.P[k * LDP + tid] : 0.0;
+    __syncthreads();
+    if (tid < m) {
+#pragma unroll
+      for (int k = 0; k < LPW; k++) {
+        S.P[k * LDP + pos] = a[k];
+        if (k < jb) A[j + pos + (long)(j + k) * lda] = a[k];
+      }
+      if (pos < LPW) S.from[pos] = tid;
+      if (tid < LPW) S.to[tid] = pos;
+      if (pos != tid) S.moved = 1;
+    }
+    __syncthreads();
+    // step 2
+    const int ncol = n - jb + nr;
+#pragma unroll 1
+    for (int cc = tid; cc < ncol; cc += NT) {
+      const bool left = cc < j, rhs = cc >= n - jb;
+      if (left && !S.moved) continue;
+      double *col = rhs ? S.xs + (cc - (n - jb)) * NT + j : A + j + (long)(left ? cc : cc + jb) * lda;
+      double x[LPW];  // shifted below: x[0] is the current row
+#pragma unroll
+      for (int q = 0; q < LPW; q++) x[q] = q < jb ? col[S.from[q]] : 0.0;
+      if (S.moved) {
+#pragma unroll 4
         for (int q = 0; q < LPW; q++) {
-          if (q >= jb) continue;
-#pragma unroll
-          for (int r = q + 1; r < LPW; r++)
-            if (r < jb) x[r] = fma(-S.P[r + q * LU_LDP], x[q], x[r]);
+          const int to = S.to[q];
+          if (to >= LPW) col[to] = col[q];
         }
-#pragma unroll
-        for (int q = 0; q < LPW; q++)
-          if (q < jb) {
-            col[q] = x[q];
-            S.U[k * LU_LDU + q] = x[q];
-          }
       }
-      __syncthreads();
-      if (m > jb) lu_update_dmma(m - jb, nt, jb, S.P + jb, LU_LDP, S.U, LU_LDU, A + (j + jb) + (long)(j + jb) * lda, lda);
-      __syncthreads();
+      double *u = S.U + (cc - j) * LU_LDU;
+#pragma unroll 1
+      for (int q = 0; q < jb; q++) {
+        const double v = x[0];
+        col[q] = v;
+        if (!left && !rhs) u[q] = v;
+        const double *l = S.P + q * LDP + q;
+        const double f = left ? 0.0 : v;  // left of the panel: interchanges only
+#pragma unroll
+        for (int r = 1; r < LPW; r++) x[r - 1] = fma(-l[r], f, x[r]);
+      }
     }
+    __syncthreads();
+    if (nt > 0) {
+      if (tid >= LPW && tid < m)  // the right-hand sides' rows below the panel
+#pragma unroll 1
+        for (int r = 0; r < nr; r++) {
+          double y = S.xs[r * NT + j + tid];
+#pragma unroll
+          for (int q = 0; q < LPW; q++) y = fma(-S.P[q * LDP + tid], S.xs[r * NT + j + q], y);
+          S.xs[r * NT + j + tid] = y;
+        }
+      lu_update<NT>(S, nt, nt, A + (j + jb) + (long)(j + jb) * lda, lda);
+    }
+    __syncthreads();
   }
-  __syncthreads();
   return S.fail;
 }
 
-__global__ void __launch_bounds__(BT)
-batched_getrf_kernel(const Prob *__restrict__ probs, const int *__restrict__ order, int count,
-                     int *__restrict__ next, int *__restrict__ info) {
-  extern __shared__ __align__(16) double sm[];
-  LuSmem &S = *reinterpret_cast<LuSmem *>(sm);
-  __shared__ int s_p;
-  const int tid = threadIdx.x;
-  while (true) {
-    if (tid == 0) {
-      const int t = atomicAdd(next, 1);
-      s_p = t < count ? order[t] : -1;
+// U x = y (UPPER) or L x = y (unit lower) in place on nr <= 8 right-hand
+// sides in S.xs, panel by panel: the panel's 16 columns are in registers, one
+// row per thread, loaded one panel ahead; one warp per right-hand side solves
+// the diagonal block, then every thread updates its row.
+template <int NT, bool UPPER>
+__device__ __forceinline__ void lu_solve(const Prob &pr, int nr, LuSmem<NT> &S) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = pr.n, np = (n + LPW - 1) / LPW;
+  const double *A = pr.A;
+  const long lda = pr.lda;
+  auto load = [&](int s, double (&v)[LPW]) {
+    const int j = (UPPER ? np - 1 - s : s) * LPW, jb = min(LPW, n - j);
+    const bool in = s < np && tid < n && (UPPER ? tid < j + jb : tid >= j);
+#pragma unroll
+    for (int q = 0; q < LPW; q++) v[q] = in && q < jb ? A[tid + (long)(j + q) * lda] : 0.0;
+    if (in && tid >= j && tid < j + jb) {
+#pragma unroll
+      for (int q = 0; q < LPW; q++) S.D[s & 1][q * DLD + tid - j] = v[q];
+    }
+  };
+  double u[LPW];
+  load(0, u);
+#pragma unroll 1
+  for (int s = 0; s < np; s++) {
+    const int j = (UPPER ? np - 1 - s : s) * LPW, jb = min(LPW, n - j);
+    __syncthreads();  // D and the rows updated by the last panel are in place
+    double nx[LPW];
+    load(s + 1, nx);
+#pragma unroll 1
+    for (int r = warp; r < nr; r += NT / 32) {
+      const int c = lane & 15;
+      double v = c < jb ? S.xs[r * NT + j + c] : 0.0;
+      const double *d = S.D[s & 1] + c;  // D(c, q) at q * DLD + c
+      const double ri = UPPER && c < jb ? 1.0 / d[c * DLD] : 1.0;
+      int q = UPPER ? jb - 1 : 0;
+      double dn = d[q * DLD];
+#pragma unroll 1
+      for (int i = 0; i < jb; i++) {
+        const double dq = dn;
+        const int qn = UPPER ? max(q - 1, 0) : min(q + 1, LPW - 1);
+        dn = d[qn * DLD];  // one step ahead of the chain
+        if (UPPER && c == q) v *= ri;
+        const double xq = __shfl_sync(0xffffffffu, v, q);
+        if (UPPER ? c < q : c > q) v = fma(-dq, xq, v);
+        q = qn;
+      }
+      if (lane < jb) S.xs[r * NT + j + c] = v;
     }
     __syncthreads();
-    const int p = s_p;
-    if (p < 0) return;
-    const Prob pr = probs[p];
-    const int fail = lu_blocked(pr, S);
-    if (tid == 0) info[p] = fail;
-    __syncthreads();
+    if (tid < n && (UPPER ? tid < j : tid >= j + jb))
+#pragma unroll 1
+      for (int r = 0; r < nr; r++) {
+        double y = S.xs[r * NT + tid];
+#pragma unroll
+        for (int q = 0; q < LPW; q++)
+          if (q < jb) y = fma(-u[q], S.xs[r * NT + j + q], y);
+        S.xs[r * NT + tid] = y;
+      }
+#pragma unroll
+    for (int q = 0; q < LPW; q++) u[q] = nx[q];
   }
+  __syncthreads();
 }
 
-// P A = L U solves, one right-hand side at a time in shared memory: the
-// interchanges in order, then the blocked unit-lower and upper solves
-__global__ void __launch_bounds__(BT)
-batched_getrs_kernel(const Prob *__restrict__ probs, const int *__restrict__ order, int count,
-                     int *__restrict__ next, const int *__restrict__ info) {
+template <int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB)
+batched_gesv_kernel(const Prob *__restrict__ probs, const int *__restrict__ order, const int *__restrict__ range,
+                    int *__restrict__ next, int *__restrict__ info) {
+  extern __shared__ __align__(16) double sm[];
+  LuSmem<NT> &S = *reinterpret_cast<LuSmem<NT> *>(sm);
   __shared__ int s_p;
-  __shared__ double sbv[MAXN];
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, end = range[1];
   while (true) {
     if (tid == 0) {
-      const int t = atomicAdd(next, 1);
-      s_p = t < count ? order[t] : -1;
+      const int t = range[0] + atomicAdd(next, 1);
+      s_p = t < end ? order[t] : -1;
     }
     __syncthreads();
     const int p = s_p;
     if (p < 0) return;
     const Prob pr = probs[p];
-    if (info[p] == 0) {
-      const int n = pr.n;
-      for (int r = 0; r < pr.nrhs; r++) {
-        double *bg = pr.B + (long)r * pr.ldb;
-        for (int i = tid; i < n; i += BT) sbv[i] = bg[i];
-        __syncthreads();
-        if (tid == 0)
-          for (int k = 0; k < n; k++) {
-            const int q = pr.ipiv[k];
-            if (q != k) { const double t0 = sbv[k]; sbv[k] = sbv[q]; sbv[q] = t0; }
+    int fail = 0;
+    if (pr.n > 0) {
+      const int n = pr.n, nr = min(pr.nrhs, LU_RHS);
+#pragma unroll 1
+      for (int r = 0; r < nr; r++)
+        if (tid < n) S.xs[r * NT + tid] = pr.B[tid + (long)r * pr.ldb];
+      fail = lu_factor<NT>(pr, nr, S);
+      if (!fail)
+#pragma unroll 1
+        for (int r0 = 0; r0 < pr.nrhs; r0 += LU_RHS) {
+          const int nc = min(LU_RHS, pr.nrhs - r0);
+          double *B = pr.B + (long)r0 * pr.ldb;
+          if (r0 > 0) {  // the columns that did not ride along
+#pragma unroll 1
+            for (int r = 0; r < nc; r++)
+              if (tid < n) S.xs[r * NT + tid] = B[tid + (long)r * pr.ldb];
+            __syncthreads();
+            if (tid < nc)
+#pragma unroll 1
+              for (int k = 0; k < n; k++) {
+                const int q = pr.ipiv[k];
+                const double t0 = S.xs[tid * NT + k];
+                S.xs[tid * NT + k] = S.xs[tid * NT + q];
+                S.xs[tid * NT + q] = t0;
+              }
+            lu_solve<NT, false>(pr, nc, S);
           }
-        __syncthreads();
-        tri_solve_smem(pr.A, pr.lda, n, sbv, true, true, false);    // L y = P b
-        tri_solve_smem(pr.A, pr.lda, n, sbv, false, false, false);  // U x = y
-        for (int i = tid; i < n; i += BT) bg[i] = sbv[i];
-        __syncthreads();
-      }
+          lu_solve<NT, true>(pr, nc, S);
+#pragma unroll 1
+          for (int r = 0; r < nc; r++)
+            if (tid < n) B[tid + (long)r * pr.ldb] = S.xs[r * NT + tid];
+          __syncthreads();
+        }
     }
+    if (tid == 0) info[p] = fail;
     __syncthreads();
   }
 }
@@ -491,9 +523,35 @@ void launch_posv(const BatchBufs &b, int bucket, cudaStream_t st) {
   ATLB_CUDA_CHECK(cudaGetLastError());
 }
 
-int grid_size(size_t smem) {
-  int per_sm = smem > 100 * 1024 ? 1 : (smem > 60 * 1024 ? 2 : 4);
-  return num_sms() * per_sm;
+template <int NT, int MINB>
+void launch_gesv(const BatchBufs &b, int bucket, cudaStream_t st) {
+  constexpr int smem = (int)sizeof(LuSmem<NT>);
+  static_assert(MINB * (smem + 1024 + 16) <= 228 * 1024, "the bucket's CTAs do not fit an SM");
+  static bool configured = false;
+  if (!configured) {
+    ATLB_CUDA_CHECK(cudaFuncSetAttribute(batched_gesv_kernel<NT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         smem));
+    ATLB_CUDA_CHECK(cudaFuncSetAttribute(batched_gesv_kernel<NT, MINB>,
+                                         cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    configured = true;
+  }
+  batched_gesv_kernel<NT, MINB><<<num_sms() * MINB, NT, smem, st>>>(b.probs, b.order, b.next + 8 + 2 * bucket,
+                                                                   b.next + bucket, b.info);
+  ATLB_CUDA_CHECK(cudaGetLastError());
+}
+
+// Cuts the sorted list into buckets of orders above lower[0], lower[1], ..;
+// returns the mask of those in use.
+unsigned bucket_ranges(const std::vector<Prob> &P, const BatchBufs &b, const int *lower, int nbuckets) {
+  int *range = b.hnext + 8, at = 0;
+  unsigned used = 0;
+  for (int q = 0; q < nbuckets; q++) {
+    range[2 * q] = at;
+    while (at < (int)P.size() && P[b.horder[at]].n > lower[q]) at++;
+    range[2 * q + 1] = at;
+    if (at > range[2 * q]) used |= 1u << q;
+  }
+  return used;
 }
 
 }  // namespace
@@ -506,16 +564,8 @@ void batched_posv_dev(const std::vector<Prob> &P, int *info_out, cudaStream_t st
   const int count = (int)P.size();
   if (!count) return;
   BatchBufs b = prepare(P, kSlotBatch0);
-  // buckets of the sorted list: tiles per side 12..16, 8..11, 4..7, up to 3
-  static const int lower[4] = {11, 7, 3, -1};
-  int *range = b.hnext + 8, at = 0;
-  unsigned used = 0;
-  for (int q = 0; q < 4; q++) {
-    range[2 * q] = at;
-    while (at < count && cdiv(P[b.horder[at]].n, cholt::TB) > lower[q]) at++;
-    range[2 * q + 1] = at;
-    if (at > range[2 * q]) used |= 1u << q;
-  }
+  static const int lower[4] = {11 * cholt::TB, 7 * cholt::TB, 3 * cholt::TB, -1};
+  const unsigned used = bucket_ranges(P, b, lower, 4);
   const std::vector<unsigned long long> key = {0xBA7C0001ull, (unsigned long long)tune_generation(),
       (unsigned long long)count, (unsigned long long)used, (unsigned long long)(uintptr_t)b.d,
       (unsigned long long)(uintptr_t)b.h, (unsigned long long)(uintptr_t)info_out,
@@ -530,32 +580,22 @@ void batched_posv_dev(const std::vector<Prob> &P, int *info_out, cudaStream_t st
   });
 }
 
-// Batched LU (+ the solve when nrhs > 0 for the problems), the same way.
-void batched_gesv_dev(const std::vector<Prob> &P, bool solve, int *info_out, cudaStream_t st) {
+// Batched LU (+ the solve of each problem's right-hand sides), the same way.
+void batched_gesv_dev(const std::vector<Prob> &P, int *info_out, cudaStream_t st) {
   const int count = (int)P.size();
   if (!count) return;
   BatchBufs b = prepare(P, kSlotBatch0);
-  int maxn = 0;
-  for (auto &p : P) maxn = std::max(maxn, p.n);
-  const size_t smb = sizeof(LuSmem);
-  static bool configured = false;
-  if (!configured) {
-    ATLB_CUDA_CHECK(cudaFuncSetAttribute(batched_getrf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb));
-    configured = true;
-  }
-  const std::vector<unsigned long long> key = {0xBA7C0002ull + (solve ? 1 : 0),
-      (unsigned long long)tune_generation(), (unsigned long long)count, (unsigned long long)maxn,
+  static const int lower[3] = {128, 64, -1};
+  const unsigned used = bucket_ranges(P, b, lower, 3);
+  const std::vector<unsigned long long> key = {0xBA7C0002ull,
+      (unsigned long long)tune_generation(), (unsigned long long)count, (unsigned long long)used,
       (unsigned long long)(uintptr_t)b.d, (unsigned long long)(uintptr_t)b.h,
       (unsigned long long)(uintptr_t)info_out, (unsigned long long)(uintptr_t)st};
   run_graph(key, st, [&]() {
     enqueue_upload(b, st);
-    batched_getrf_kernel<<<grid_size(smb), BT, smb, st>>>(b.probs, b.order, count, b.next, b.info);
-    ATLB_CUDA_CHECK(cudaGetLastError());
-    if (solve) {
-      ATLB_CUDA_CHECK(cudaMemsetAsync(b.next, 0, sizeof(int), st));
-      batched_getrs_kernel<<<num_sms() * 4, BT, 0, st>>>(b.probs, b.order, count, b.next, b.info);
-      ATLB_CUDA_CHECK(cudaGetLastError());
-    }
+    if (used & 1) launch_gesv<256, 2>(b, 0, st);
+    if (used & 2) launch_gesv<128, 4>(b, 1, st);
+    if (used & 4) launch_gesv<64, 8>(b, 2, st);
     ATLB_CUDA_CHECK(cudaMemcpyAsync(info_out, b.info, sizeof(int) * count, cudaMemcpyDeviceToHost, st));
   });
 }
@@ -606,7 +646,7 @@ int atlb_dgesv_batched(int count, const int *n, double *const *A, const int *lda
   }
   cudaStream_t st = stream();
   int *hinfo = (int *)pinned(kSlotBatch1, sizeof(int) * count);
-  batched_gesv_dev(P, B != nullptr, hinfo, st);
+  batched_gesv_dev(P, hinfo, st);
   ATLB_CUDA_CHECK(cudaStreamSynchronize(st));
   memcpy(info, hinfo, sizeof(int) * count);
   return 0;

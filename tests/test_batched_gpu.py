@@ -136,6 +136,83 @@ def test_batched_gesv_matches_oracle(gpu, orc):
         assert orc.resid_slv(a0s[i], np.asfortranarray(x), xt) <= 100
 
 
+@pytest.mark.parametrize("nrhs", [0, 1, 8, 9, 20])
+def test_batched_gesv_panel_edges(gpu, orc, nrhs):
+    """Orders at the edges of the 16-column panels and of the size buckets,
+    leading dimensions above the order, right-hand sides across the eight that
+    ride along, random pivots; ipiv equal to the oracle's, nothing outside A and
+    B's n rows written, |P A - L U| <= (n + 1) u |L||U| and the solve's residual
+    <= (3 n + 2) u |L||U||x| componentwise (Higham, theorems 9.3 and 9.4),
+    u = 2^-53, doubled for the reciprocal pivots."""
+    import torch
+    rng = np.random.default_rng(100 + nrhs)
+    ns = [1, 2, 15, 16, 17, 48, 63, 64, 65, 127, 128, 129, 255, 256, 0]
+    u = 2.0 ** -53
+    As, Bs, Ps, a0s, b0s, lda, ldb = [], [], [], [], [], [], []
+    for n in ns:
+        la, lb = n + 3, n + 5
+        a = np.full((max(n, 1), la), 7.0)             # row = column of the matrix
+        a[:n, :n] = rng.uniform(-1, 1, (n, n))
+        b = np.full((max(nrhs, 1), lb), 9.0)
+        b[:, :n] = rng.uniform(-1, 1, (max(nrhs, 1), n))
+        a0s.append(a)
+        b0s.append(b)
+        lda.append(la)
+        ldb.append(lb)
+        As.append(torch.tensor(a, device="cuda"))
+        Bs.append(torch.tensor(b, device="cuda"))
+        Ps.append(torch.full((n + 1,), -7, dtype=torch.int32, device="cuda"))
+    count = len(ns)
+    info = np.full(count, -1, dtype=np.int32)
+    assert AB.atlb_dgesv_batched(count, _int_array(ns), _ptr_array(As), _int_array(lda), _ptr_array(Ps),
+                                 _ptr_array(Bs), _int_array(ldb), _int_array([nrhs] * count), info) == 0
+    assert np.all(info == 0)
+    for i, n in enumerate(ns):
+        a, b, piv = As[i].cpu().numpy(), Bs[i].cpu().numpy(), Ps[i].cpu().numpy()
+        assert np.array_equal(a[:, n:], a0s[i][:, n:]) and np.array_equal(b[:, n:], b0s[i][:, n:])
+        assert piv[n] == -7
+        if n == 0:
+            continue
+        a0 = np.asfortranarray(a0s[i][:n, :n].T)
+        _, rpiv, _ = orc.dgetrf(a0.copy(order="F"))
+        np.testing.assert_array_equal(piv[:n], rpiv)
+        lu = a[:n, :n].T
+        low, up = np.tril(lu, -1) + np.eye(n), np.triu(lu)
+        pa = a0.copy()
+        for k in range(n):
+            pa[[k, piv[k]]] = pa[[piv[k], k]]
+        mag = np.abs(low) @ np.abs(up)
+        assert np.all(np.abs(low @ up - pa) <= 2 * (n + 2) * u * mag)
+        for r in range(nrhs):
+            pb = b0s[i][r, :n].copy()
+            for k in range(n):
+                pb[[k, piv[k]]] = pb[[piv[k], k]]
+            x = b[r, :n]
+            assert np.all(np.abs(pa @ x - pb) <= 2 * (3 * n + 3) * u * (mag @ np.abs(x)))
+
+
+def test_batched_gesv_singular(gpu):
+    """A zero column, a zero matrix and a repeated row: the first zero pivot's
+    position, the factorization completed, the right-hand side untouched."""
+    import torch
+    n = 40
+    rng = np.random.default_rng(3)
+    a = [rng.uniform(-1, 1, (n, n)) for _ in range(3)]
+    a[0][17] = 0.0                                     # column 17 (stored as a row)
+    a[1][:] = 0.0
+    As = [torch.tensor(m, device="cuda") for m in a] + [torch.eye(n, dtype=torch.float64, device="cuda")]
+    Bs = [torch.ones(1, n, dtype=torch.float64, device="cuda") for _ in As]
+    Ps = [torch.zeros(n, dtype=torch.int32, device="cuda") for _ in As]
+    ns, one = _int_array([n] * 4), _int_array([1] * 4)
+    info = np.zeros(4, dtype=np.int32)
+    assert AB.atlb_dgesv_batched(4, ns, _ptr_array(As), ns, _ptr_array(Ps), _ptr_array(Bs), ns, one, info) == 0
+    assert list(info) == [18, 1, 0, 0]
+    assert np.array_equal(Ps[1].cpu().numpy(), np.arange(n)) and np.array_equal(Ps[3].cpu().numpy(), np.arange(n))
+    for k in (0, 1):
+        assert np.all(Bs[k].cpu().numpy() == 1.0)
+    assert np.all(np.isfinite(As[0].cpu().numpy()))
+
+
 def test_batched_dgemm_uneven(gpu, orc):
     import torch
     rng = np.random.default_rng(2)
