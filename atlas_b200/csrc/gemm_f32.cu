@@ -1,6 +1,6 @@
 // FP32 GEMM on the FP32 FMA pipes (cblas_sgemm and the FP32-exact factor
-// mode of the mixed-precision solvers).  128x128x8 CTA tile, 256 threads,
-// 8x8 outputs per thread; op(A) and op(B) tiles are staged in shared memory
+// mode of the mixed-precision solvers).  128x128x16 CTA tile, 128 threads,
+// 8x16 outputs per thread; op(A) and op(B) tiles are staged in shared memory
 // k-major (m / n contiguous) by a 3-stage cp.async pipeline, whatever their
 // global layout, so the inner loop reads 128-bit vectors.  An output of few
 // tiles with a long K (the Cholesky's diagonal-block updates) is split along
@@ -14,25 +14,66 @@
 namespace atlb {
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 8, THREADS = 256, STAGES = 3, LDS = BM + 4;
+constexpr int BM = 128, BN = 128, BK = 16, THREADS = 128, STAGES = 3, LDS = BM + 4;
+constexpr int SMEM = 2 * STAGES * BK * LDS * (int)sizeof(float);
 
-template <bool TRANS_O>  // operand element (o, k): TRANS_O ? X[k + o*ld] : X[o + k*ld]
+// One 128 x 16 operand tile into shared memory, k-major (o contiguous).
+// Operand element (o, k): TRANS_O ? X[k + o*ld] : X[o + k*ld].  VEC: o is
+// contiguous in global memory and every column starts on 16 bytes, so whole
+// 16-byte pieces are copied; otherwise 4 bytes at a time.
+template <bool TRANS_O, bool VEC>
 __device__ __forceinline__ void load_tile(float *s, const float *X, long ld, int o0, int k0,
                                           int O, int K, int tid) {
+  if (VEC && !TRANS_O) {
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    int c = tid + THREADS * i;
-    int o, k;
-    if (!TRANS_O) { o = c & 127; k = c >> 7; }   // o fastest: coalesced along o
-    else { k = c & 7; o = c >> 3; }              // k fastest: coalesced along k
-    int go = o0 + o, gk = k0 + k;
-    bool p = go < O && gk < K;
-    const float *g = TRANS_O ? X + gk + (long)go * ld : X + go + (long)gk * ld;
-    cp_async4(s + k * LDS + o, p ? g : X, p);
+    for (int i = 0; i < BM * BK / 4 / THREADS; i++) {
+      const int c = tid + THREADS * i, o = (c & 31) * 4, k = c >> 5;
+      const int go = o0 + o, gk = k0 + k;
+      const float *g = X + go + (long)gk * ld;
+      float *d = s + k * LDS + o;
+      if (gk < K && go + 3 < O) cp_async16(d, g, true);
+      else {
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const bool p = gk < K && go + e < O;
+          cp_async4(d + e, p ? g + e : X, p);
+        }
+      }
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < BM * BK / THREADS; i++) {
+      const int c = tid + THREADS * i;
+      int o, k;
+      if (!TRANS_O) { o = c & 127; k = c >> 7; }   // o fastest: coalesced along o
+      else { k = c & 15; o = c >> 4; }             // k fastest: coalesced along k
+      const int go = o0 + o, gk = k0 + k;
+      const bool p = go < O && gk < K;
+      const float *g = TRANS_O ? X + gk + (long)go * ld : X + go + (long)gk * ld;
+      cp_async4(s + k * LDS + o, p ? g : X, p);
+    }
   }
 }
 
-template <bool TA, bool TB>
+// two FP32 fused multiply-adds in one instruction (each rounded as fmaf)
+__device__ __forceinline__ void fma2(unsigned long long &c, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long swap2(unsigned long long x) {
+  unsigned long long r;
+  asm("{\n .reg .b32 lo, hi;\n mov.b64 {lo, hi}, %1;\n mov.b64 %0, {hi, lo};\n}" : "=l"(r) : "l"(x));
+  return r;
+}
+
+// What bounds it: the FP32 pipes (74 TFLOP/s at 1965 MHz), so shared memory
+// and the instructions issued must fit beside them.  A thread holds 8 x 16
+// outputs: a k-step then costs a warp 24 shared-memory passes for 32 cycles of
+// FMAs (with 8 x 8 outputs it was 16 for 16, and shared memory was the bound).
+// Products go two to an instruction (fma.rn.f32x2): a pair of rows times a pair
+// of columns, then the swapped pair of rows times the same, two moves a pair of
+// rows.  4096^3: 3.17 ms with 8 x 8 outputs and single products, 2.76 ms
+// now.
+template <bool TA, bool TB, bool VA, bool VB>
 __global__ void __launch_bounds__(THREADS, 2)
 sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A, long lda,
                   const float *__restrict__ B, long ldb, float beta, float *__restrict__ C,
@@ -47,8 +88,8 @@ sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A,
     alpha = 1.f;
     beta = 0.f;
   }
-  __shared__ __align__(16) float sA[STAGES][BK * LDS];
-  __shared__ __align__(16) float sB[STAGES][BK * LDS];
+  extern __shared__ __align__(16) float sgemm_smem[];
+  float *sA = sgemm_smem, *sB = sgemm_smem + STAGES * BK * LDS;
   const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
   const int bid = blockIdx.x, G = 8;
   const int per_group = G * tiles_n, group = bid / per_group;
@@ -57,20 +98,24 @@ sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A,
   const int m0 = tm * BM, n0 = tn * BN;
   if (tri == 1 && m0 + BM - 1 < n0) return;
   if (tri == 2 && m0 > n0 + BN - 1) return;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // this thread's rows rm + 32 h + 0..3 (h < 2), columns cn + 16 q + 0..3 (q < 4)
+  const int rm = (warp & 1) * 64 + (lane & 7) * 4, cn = (warp >> 1) * 64 + (lane >> 3) * 4;
 
-  float acc[8][8];
+  // row pair i x column pair j: acc[0] holds (row 0, col 0) and (row 1, col 1),
+  // acc[1] (row 1, col 0) and (row 0, col 1)
+  unsigned long long acc[2][4][8];
 #pragma unroll
-  for (int i = 0; i < 8; i++)
+  for (int i = 0; i < 4; i++)
 #pragma unroll
-    for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
+    for (int j = 0; j < 8; j++) acc[0][i][j] = acc[1][i][j] = 0ull;
 
   const int KT = (K + BK - 1) / BK;
 #pragma unroll
   for (int s = 0; s < STAGES - 1; s++) {
     if (s < KT) {
-      load_tile<TA>(sA[s], A, lda, m0, s * BK, M, K, tid);
-      load_tile<!TB>(sB[s], B, ldb, n0, s * BK, N, K, tid);
+      load_tile<TA, VA>(sA + s * BK * LDS, A, lda, m0, s * BK, M, K, tid);
+      load_tile<!TB, VB>(sB + s * BK * LDS, B, ldb, n0, s * BK, N, K, tid);
     }
     cp_async_commit();
   }
@@ -78,43 +123,54 @@ sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A,
     cp_async_wait<STAGES - 2>();
     __syncthreads();
     {
-      int nk = kt + STAGES - 1;
+      const int nk = kt + STAGES - 1;
       if (nk < KT) {
-        load_tile<TA>(sA[nk % STAGES], A, lda, m0, nk * BK, M, K, tid);
-        load_tile<!TB>(sB[nk % STAGES], B, ldb, n0, nk * BK, N, K, tid);
+        load_tile<TA, VA>(sA + nk % STAGES * BK * LDS, A, lda, m0, nk * BK, M, K, tid);
+        load_tile<!TB, VB>(sB + nk % STAGES * BK * LDS, B, ldb, n0, nk * BK, N, K, tid);
       }
       cp_async_commit();
     }
-    const float *as = sA[kt % STAGES], *bs = sB[kt % STAGES];
+    const float *as = sA + kt % STAGES * BK * LDS + rm, *bs = sB + kt % STAGES * BK * LDS + cn;
 #pragma unroll
     for (int k = 0; k < BK; k++) {
-      float4 a0 = *reinterpret_cast<const float4 *>(as + k * LDS + ty * 4);
-      float4 a1 = *reinterpret_cast<const float4 *>(as + k * LDS + 64 + ty * 4);
-      float4 b0 = *reinterpret_cast<const float4 *>(bs + k * LDS + tx * 4);
-      float4 b1 = *reinterpret_cast<const float4 *>(bs + k * LDS + 64 + tx * 4);
-      float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+      const ulonglong2 a0 = *reinterpret_cast<const ulonglong2 *>(as + k * LDS);
+      const ulonglong2 a1 = *reinterpret_cast<const ulonglong2 *>(as + k * LDS + 32);
+      const unsigned long long a[4] = {a0.x, a0.y, a1.x, a1.y};
+      unsigned long long b[8], x[4];
 #pragma unroll
-      for (int i = 0; i < 8; i++)
+      for (int q = 0; q < 4; q++) {
+        const ulonglong2 bq = *reinterpret_cast<const ulonglong2 *>(bs + k * LDS + 16 * q);
+        b[2 * q] = bq.x;
+        b[2 * q + 1] = bq.y;
+        x[q] = swap2(a[q]);
+      }
 #pragma unroll
-        for (int j = 0; j < 8; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+      for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          fma2(acc[0][i][j], a[i], b[j]);
+          fma2(acc[1][i][j], x[i], b[j]);
+        }
     }
   }
   cp_async_wait<0>();
-  // epilogue: each thread owns rows {ty*4 .. +3, 64 + ty*4 .. +3} x columns
-  // {tx*4 .. +3, 64 + tx*4 .. +3}; a row quad of one column is contiguous in C.
-  // All old C values are loaded before any store, so the loads overlap.
+  // epilogue: a row quad of one column is contiguous in C.  Old C values are
+  // loaded eight quads at a time before any of their stores, so the loads overlap.
+  auto val = [&](int h, int j, int e) {  // row rm + 32 h + e, column j of this thread's sixteen
+    // the half that holds row e's product: row 0 leads in acc[0], row 1 in acc[1]
+    const int s = (e ^ j) & 1, half = s ? 1 - (e & 1) : e & 1;
+    return __uint_as_float((unsigned)(acc[s][2 * h + (e >> 1)][j >> 1] >> (32 * half)));
+  };
   const bool vec = tri == 0 && ((uintptr_t)C % 16 == 0) && (ldc % 4 == 0) && m0 + BM <= M && n0 + BN <= N;
   if (vec) {
 #pragma unroll
-    for (int jh = 0; jh < 8; jh += 4) {  // two rounds of 8 float4 loads, then their stores
+    for (int jh = 0; jh < 16; jh += 4) {  // four rounds of 8 float4 loads, then their stores
       float4 cv[4][2];
 #pragma unroll
       for (int jj = 0; jj < 4; jj++)
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-          const int j = jh + jj;
-          const int c = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4), r = m0 + h * 64 + ty * 4;
+          const int c = n0 + cn + 4 * jh + jj, r = m0 + rm + 32 * h;
           cv[jj][h] = beta != 0.f ? *reinterpret_cast<const float4 *>(C + r + (long)c * ldc)
                                   : make_float4(0.f, 0.f, 0.f, 0.f);
         }
@@ -122,13 +178,12 @@ sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A,
       for (int jj = 0; jj < 4; jj++)
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-          const int j = jh + jj;
-          const int c = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4), r = m0 + h * 64 + ty * 4;
+          const int j = jh + jj, c = n0 + cn + 4 * jh + jj, r = m0 + rm + 32 * h;
           float4 o;
-          o.x = alpha * acc[h * 4 + 0][j];
-          o.y = alpha * acc[h * 4 + 1][j];
-          o.z = alpha * acc[h * 4 + 2][j];
-          o.w = alpha * acc[h * 4 + 3][j];
+          o.x = alpha * val(h, j, 0);
+          o.y = alpha * val(h, j, 1);
+          o.z = alpha * val(h, j, 2);
+          o.w = alpha * val(h, j, 3);
           if (beta != 0.f) {
             o.x = fmaf(beta, cv[jj][h].x, o.x);
             o.y = fmaf(beta, cv[jj][h].y, o.y);
@@ -141,22 +196,22 @@ sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A,
     return;
   }
 #pragma unroll
-  for (int j = 0; j < 8; j++) {
-    const int c = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
+  for (int j = 0; j < 16; j++) {
+    const int c = n0 + cn + 16 * (j >> 2) + (j & 3);
     float cv[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-      const int r = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
+      const int r = m0 + rm + (i < 4 ? i : 32 + i - 4);
       const bool ok = r < M && c < N && !(tri == 1 && r < c) && !(tri == 2 && r > c);
       cv[i] = (ok && beta != 0.f) ? C[r + (long)c * ldc] : 0.f;
     }
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-      const int r = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
+      const int r = m0 + rm + (i < 4 ? i : 32 + i - 4);
       if (r >= M || c >= N) continue;
       if (tri == 1 && r < c) continue;
       if (tri == 2 && r > c) continue;
-      float v = alpha * acc[i][j];
+      float v = alpha * val(i >> 2, j, i & 3);
       if (beta != 0.f) v = fmaf(beta, cv[i], v);
       C[r + (long)c * ldc] = v;
     }
@@ -217,10 +272,31 @@ void sgemm_dev(int ta, int tb, int M, int N, int K, float alpha, const float *A,
     else kc = K;
   }
   const dim3 grid(tiles, S);
-  if (!tA && !tB) sgemm_simt_kernel<false, false><<<grid, THREADS, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, tri, kc, W);
-  else if (!tA && tB) sgemm_simt_kernel<false, true><<<grid, THREADS, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, tri, kc, W);
-  else if (tA && !tB) sgemm_simt_kernel<true, false><<<grid, THREADS, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, tri, kc, W);
-  else sgemm_simt_kernel<true, true><<<grid, THREADS, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, tri, kc, W);
+  // 16-byte copies need the outer index contiguous and 16-byte aligned columns
+  const bool va = !tA && (uintptr_t)A % 16 == 0 && lda % 4 == 0, vb = tB && (uintptr_t)B % 16 == 0 && ldb % 4 == 0;
+  auto go = [&](auto kern, bool &configured) {
+    if (!configured) {
+      ATLB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+      ATLB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+      configured = true;
+    }
+    kern<<<grid, THREADS, SMEM, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, tri, kc, W);
+  };
+  static bool set[9] = {};
+  if (!tA && !tB) {
+    if (va) go(sgemm_simt_kernel<false, false, true, false>, set[0]);
+    else go(sgemm_simt_kernel<false, false, false, false>, set[1]);
+  } else if (!tA && tB) {
+    if (va && vb) go(sgemm_simt_kernel<false, true, true, true>, set[2]);
+    else if (va) go(sgemm_simt_kernel<false, true, true, false>, set[3]);
+    else if (vb) go(sgemm_simt_kernel<false, true, false, true>, set[4]);
+    else go(sgemm_simt_kernel<false, true, false, false>, set[5]);
+  } else if (tA && !tB) {
+    go(sgemm_simt_kernel<true, false, false, false>, set[6]);
+  } else {
+    if (vb) go(sgemm_simt_kernel<true, true, false, true>, set[7]);
+    else go(sgemm_simt_kernel<true, true, false, false>, set[8]);
+  }
   ATLB_CUDA_CHECK(cudaGetLastError());
   if (S > 1) {
     const long total = (long)M * N;
