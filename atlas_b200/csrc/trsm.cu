@@ -352,10 +352,141 @@ void eff_update(const Eff<T> &e, int r2, int n2, int r1, int n1, int m, SgemmFn 
   }
 }
 
+// The FP64 solve of an order n <= 256 for all m columns in one launch, on the
+// tensor cores: a CTA keeps its CT columns of B in shared memory and walks
+// T's 64 x 64 tiles, block row after block row -- X_kt's products first, then
+// the block row's inverted diagonal tile -- each tile fetched while the one
+// before is multiplied.  It is what the Cholesky's block columns wait for:
+// the recursion below 256 (inverse times 64 rows, a coupling product, the next
+// inverse) took three launches and 66 us for an order of 128 and 8000 columns,
+// this takes BLK_US.
+constexpr int TBK_N = 256;
+template <int CT>
+constexpr int tri_block_smem(int n) { return 8 * ((n + LEAF - 1) / LEAF * LEAF * (CT + 4) + 2 * LEAF * (LEAF + 4)); }
+
+template <int CT>
+__global__ void __launch_bounds__(256, 1)
+tri_block_kernel(int n, int m, const double *__restrict__ Tp, long tr, long tc, int lower,
+                 const double *__restrict__ W, double *__restrict__ Bp, long br, long bc) {
+  // 4 (mod 16) doubles: the MMA's 8 x 4 fragments fall in distinct banks
+  constexpr int LT = LEAF + 4, LB = CT + 4, NW = CT / 16;  // 8-column groups of a warp
+  extern __shared__ __align__(16) unsigned char tbk_smem[];
+  const int nblk = (n + LEAF - 1) / LEAF, np = nblk * LEAF;
+  double *sB = reinterpret_cast<double *>(tbk_smem);  // [np][LB]
+  double *sT = sB + np * LB;                          // [2][LEAF][LT]: T(i, k) at k * LT + i
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int j0 = blockIdx.x * CT, mc = min(CT, m - j0);
+  const int r0 = (warp & 3) * 16, c0 = (warp >> 2) * 8 * NW;
+  auto block = [&](int s) { return lower ? s : nblk - 1 - s; };  // the s-th block row solved
+  auto fetch = [&](int s, int u, int buf) {  // tile u of block row s (u == s: the inverse)
+    double *d = sT + buf * LEAF * LT;
+    if (s < nblk) {
+      const int ib = block(s), kb = block(u);
+      const double *Tb = u == s ? W + (long)ib * LEAF * LEAF : Tp + (long)ib * LEAF * tr + (long)kb * LEAF * tc;
+      const long si = u == s ? 1 : tr, sk = u == s ? LEAF : tc;
+      for (int e = tid; e < LEAF * LEAF; e += 256) {
+        const int x = e % LEAF, y = e / LEAF, i = si == 1 ? x : y, k = si == 1 ? y : x;
+        const bool ok = u == s || (ib * LEAF + i < n && kb * LEAF + k < n);
+        cp_async8(d + k * LT + i, ok ? Tb + i * si + k * sk : Tp, ok);
+      }
+    }
+    cp_async_commit();
+  };
+  for (int e = tid; e < np * CT; e += 256) {
+    const int i = br == 1 ? e % np : e / CT, j = br == 1 ? e / np : e % CT;
+    const bool ok = i < n && j < mc;
+    cp_async8(sB + i * LB + j, ok ? Bp + i * br + (long)(j0 + j) * bc : Bp, ok);
+  }
+  fetch(0, 0, 0);
+  double acc[2][NW][2];
+  auto clear = [&]() {
+#pragma unroll
+    for (int x = 0; x < 2; x++)
+#pragma unroll
+      for (int y = 0; y < NW; y++) acc[x][y][0] = acc[x][y][1] = 0.0;
+  };
+  clear();
+  int buf = 0;
+  for (int s = 0; s < nblk; s++) {
+    const int ib = block(s);
+    double *Bi = sB + ib * LEAF * LB;
+    for (int u = 0; u <= s; u++, buf ^= 1) {
+      cp_async_wait<0>();
+      __syncthreads();  // this tile is here, and nobody reads the other buffer any more
+      if (u < s) fetch(s, u + 1, buf ^ 1);
+      else fetch(s + 1, 0, buf ^ 1);
+      const double *A = sT + buf * LEAF * LT + t * LT + r0 + g;
+      if (u == s) {  // Y = B_ib - sum, then X_ib = W Y; the inverse's zero half left out
+        if (s > 0) {
+#pragma unroll
+          for (int x = 0; x < 2; x++)
+#pragma unroll
+            for (int y = 0; y < NW; y++)
+#pragma unroll
+              for (int e = 0; e < 2; e++) Bi[(r0 + 8 * x + g) * LB + c0 + 8 * y + 2 * t + e] -= acc[x][y][e];
+          clear();
+          __syncthreads();
+        }
+      }
+      const double *X = sB + block(u) * LEAF * LB + t * LB + c0 + g;
+      const int k0 = u == s && !lower ? r0 : 0, k1 = u == s && lower ? r0 + 16 : LEAF;
+#pragma unroll 4
+      for (int k = k0; k < k1; k += 4) {
+        double a[2], b[NW];
+        a[0] = A[k * LT];
+        a[1] = A[k * LT + 8];
+#pragma unroll
+        for (int y = 0; y < NW; y++) b[y] = X[k * LB + 8 * y];
+#pragma unroll
+        for (int x = 0; x < 2; x++)
+#pragma unroll
+          for (int y = 0; y < NW; y++) cholb::dmma_8x8x4(acc[x][y], a[x], b[y]);
+      }
+      if (u == s) {
+        __syncthreads();
+#pragma unroll
+        for (int x = 0; x < 2; x++)
+#pragma unroll
+          for (int y = 0; y < NW; y++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) Bi[(r0 + 8 * x + g) * LB + c0 + 8 * y + 2 * t + e] = acc[x][y][e];
+        clear();
+      }
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < np * CT; e += 256) {
+    const int i = br == 1 ? e % np : e / CT, j = br == 1 ? e / np : e % CT;
+    if (i < n && j < mc) Bp[i * br + (long)(j0 + j) * bc] = sB[i * LB + j];
+  }
+}
+
+template <int CT>
+void tri_block_launch(int n, int m, const double *Tp, long tr, long tc, int lower, const double *W, double *Bp, long br,
+                      long bc, cudaStream_t st) {
+  static bool configured = false;
+  if (!configured) {
+    static_assert(tri_block_smem<CT>(TBK_N) <= 227 * 1024, "the columns do not fit");
+    ATLB_CUDA_CHECK(cudaFuncSetAttribute(tri_block_kernel<CT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         tri_block_smem<CT>(TBK_N)));
+    configured = true;
+  }
+  tri_block_kernel<CT><<<cdiv(m, CT), 256, tri_block_smem<CT>(n), st>>>(n, m, Tp, tr, tc, lower, W, Bp, br, bc);
+  ATLB_CUDA_CHECK(cudaGetLastError());
+}
+
 template <typename T>
 void eff_solve(const Eff<T> &e, int r0, int n, int m, SgemmFn fn, cudaStream_t st) {
   if (n <= 0 || m <= 0) return;
-  if (n <= LEAF) {
+  if constexpr (sizeof(T) == 8) {
+    if (n <= TBK_N) {
+      const double *Td = e.Tp + r0 * e.tr + r0 * e.tc, *Wd = e.W + (long)(r0 / LEAF) * LEAF * LEAF;
+      // 16 columns a CTA while 64 would leave most SMs idle
+      if (cdiv(m, 64) * 2 <= num_sms()) tri_block_launch<16>(n, m, Td, e.tr, e.tc, e.lower, Wd, e.Bp + r0 * e.br, e.br, e.bc, st);
+      else tri_block_launch<64>(n, m, Td, e.tr, e.tc, e.lower, Wd, e.Bp + r0 * e.br, e.br, e.bc, st);
+      return;
+    }
+  } else if (n <= LEAF) {
     constexpr int smem = 2 * LEAF * (LEAF + 1) * (int)sizeof(T);
     static bool configured = false;
     if (!configured) {

@@ -1,4 +1,4 @@
-// Triangular solve for a few right-hand sides (NRHS <= 8) in ONE launch.
+// Triangular solve for a few right-hand sides (FP32 <= 8, FP64 <= 16) in ONE launch.
 //
 // The recursive TRSM (trsm.cu) issues ~2n/64 launches, which for one
 // right-hand side is all latency.  Here one CTA owns one 128-row block of
@@ -15,7 +15,8 @@
 // published.  In FP32 the block just before is not awaited through its flag:
 // its x also goes out as (value, epoch) 64-bit words, each written by one
 // single-copy-atomic store, and the next block polls those words directly --
-// one round trip to L2 on the chain instead of fence, flag and data load.
+// one round trip to L2 on the chain instead of fence, flag and data load (in
+// FP64, with two words a value, that changed nothing).
 // Every wait is bounded: after ~1 s the kernel records an error in *err and
 // stops waiting (the result is then wrong but the GPU is released).  The
 // launcher clears the ticket counter, the flags and the tagged words before
@@ -23,6 +24,7 @@
 #include <algorithm>
 #include "common.cuh"
 #include "kernels.h"
+#include "chol_blocks.cuh"
 
 namespace atlb {
 namespace {
@@ -231,6 +233,148 @@ trsv_kernel(int n, int nrhs, const T *__restrict__ Tp, long tr, long tc, int low
   }
 }
 
+// The same solve for 5..16 FP64 right-hand sides, 8 NH per launch, with the
+// products on the FP64 tensor cores.  A chain step (the product with the block
+// just before, then the one with the inverted diagonal block) is 128 x 128 x 8
+// twice: with FMAs every term needs its x from shared memory (8192^2, 8
+// right-hand sides: 13.5 us a block), while the MMA's n = 8 columns are the
+// right-hand sides themselves and one fragment of x serves 8 rows.  Warp w
+// owns rows 8 w .. 8 w + 7; its fragments of T come from global memory before
+// the wait.  Two groups of columns share every fragment of T and the chain's
+// latency, hence up to 16 per launch: 8192^2, 16 right-hand sides, one
+// direction 472 us; with FMAs, eight at a time, 2 x 860.
+template <int NH>
+__global__ void __launch_bounds__(TT, 1)
+trsv_mma_kernel(int n, int nrhs, const double *__restrict__ Tp, long tr, long tc, int lower,
+                const double *__restrict__ W, double *X, long ldx, int *counter, int *flags, int epoch, int *err) {
+  constexpr int NR = 8 * NH, LX = NH == 1 ? 12 : 20, LW = CB + 4;  // fragments in distinct banks
+  extern __shared__ __align__(16) unsigned char trsv_smem[];
+  double *sW = reinterpret_cast<double *>(trsv_smem);  // W(r, c) at r * LW + c
+  double *sx = sW + CB * LW;                           // x of a solved block (row k at k * LX), double-buffered
+  double *sb = sx + 2 * CB * LX;                       // this block's b
+  __shared__ int s_bi, s_ready;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nb = (n + CB - 1) / CB;
+  const int g = lane >> 2, t = lane & 3;
+  if (tid == 0) {
+    const int k = atomicAdd(counter, 1);
+    s_bi = lower ? k : nb - 1 - k;
+  }
+  __syncthreads();
+  const int bi = s_bi, r0 = bi * CB, rows = min(CB, n - r0);
+  {
+    const double *Wb = W + (long)bi * CB * CB;
+    for (int base = tid; base < CB * CB; base += 8 * TT) {
+      double v[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) v[q] = Wb[base + q * TT];
+#pragma unroll
+      for (int q = 0; q < 8; q++) sW[(base + q * TT) % CB * LW + (base + q * TT) / CB] = v[q];
+    }
+  }
+  for (int idx = tid; idx < CB * NR; idx += TT) {
+    const int rr = idx % CB, q = idx / CB;
+    sb[rr * LX + q] = (rr < rows && q < nrhs) ? X[r0 + rr + (long)q * ldx] : 0.0;
+  }
+  const int row = 8 * warp + g;
+  const double *trow = Tp + (long)(r0 + row) * tr;
+  const int ndep = lower ? bi : nb - 1 - bi;
+  double acc[NH][2];
+#pragma unroll
+  for (int h = 0; h < NH; h++) acc[h][0] = acc[h][1] = 0.0;
+  auto wait_flag = [&](int bj) {
+    const uint64_t t0 = gtimer();
+    while (ld_acquire(flags + bj) != epoch) {
+      if (gtimer() - t0 > 1000000000ull) { atomicExch(err, 1); break; }
+    }
+  };
+  auto load_t = [&](int bj, double (&a)[CB / 4]) {
+    const int c0 = bj * CB;
+#pragma unroll
+    for (int k = 0; k < CB / 4; k++)
+      a[k] = (row < rows && c0 + 4 * k + t < n) ? trow[(long)(c0 + 4 * k + t) * tc] : 0.0;
+  };
+  auto load_x = [&](int bj, int buf) {
+    const int c0 = bj * CB;
+    for (int idx = tid; idx < CB * NR; idx += TT) {
+      const int cc = idx % CB, q = idx / CB;
+      sx[buf * CB * LX + cc * LX + q] = (c0 + cc < n && q < nrhs) ? __ldcg(X + c0 + cc + (long)q * ldx) : 0.0;
+    }
+  };
+  auto multiply = [&](const double (&a)[CB / 4], int buf) {
+    const double *xs = sx + buf * CB * LX + t * LX + g;
+#pragma unroll
+    for (int k = 0; k < CB / 4; k++)
+#pragma unroll
+      for (int h = 0; h < NH; h++) cholb::dmma_8x8x4(acc[h], a[k], xs[4 * k * LX + 8 * h]);
+  };
+  // 1. solved blocks in bulk: all but the last dependency
+  int d = 0, buf = 0;
+  while (d < ndep - 1) {
+    if (tid < 32) {
+      const int dd = d + lane;
+      const bool ok = dd < ndep - 1 && ld_acquire(flags + (lower ? dd : nb - 1 - dd)) == epoch;
+      const unsigned m = __ballot_sync(0xffffffffu, ok);
+      const int ready = __ffs(~m) - 1;  // leading run of done blocks
+      if (lane == 0) {
+        if (ready == 0) wait_flag(lower ? d : nb - 1 - d);
+        s_ready = ready == 0 ? 1 : ready;
+      }
+    }
+    __syncthreads();
+    const int nr = s_ready;
+    for (int e = 0; e < nr; e++, d++) {
+      const int bj = lower ? d : nb - 1 - d;
+      double a[CB / 4];
+      load_t(bj, a);
+      load_x(bj, buf);
+      __syncthreads();
+      multiply(a, buf);
+      buf ^= 1;
+    }
+    __syncthreads();  // s_ready is read by every thread before it is rewritten
+  }
+  // 2. the block just before this one: its matrix values first, then the wait
+  if (ndep > 0) {
+    const int bj = lower ? ndep - 1 : nb - ndep;
+    double a[CB / 4];
+    load_t(bj, a);
+    if (tid == 0) wait_flag(bj);
+    __syncthreads();
+    load_x(bj, buf);
+    __syncthreads();
+    multiply(a, buf);
+  } else {
+    __syncthreads();  // sb is in place
+  }
+#pragma unroll
+  for (int h = 0; h < NH; h++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) sb[row * LX + 8 * h + 2 * t + e] -= acc[h][e];
+  __syncthreads();
+  // 3. x = inv(T_bb) b, the triangle's zero half left out
+#pragma unroll
+  for (int h = 0; h < NH; h++) acc[h][0] = acc[h][1] = 0.0;
+  const int k0 = lower ? 0 : 2 * warp, k1 = lower ? 2 * warp + 2 : CB / 4;
+#pragma unroll 4
+  for (int k = k0; k < k1; k++) {
+    const double w = sW[row * LW + 4 * k + t];
+#pragma unroll
+    for (int h = 0; h < NH; h++) cholb::dmma_8x8x4(acc[h], w, sb[(4 * k + t) * LX + 8 * h + g]);
+  }
+#pragma unroll
+  for (int h = 0; h < NH; h++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int q = 8 * h + 2 * t + e;
+      if (row < rows && q < nrhs) X[r0 + row + (long)q * ldx] = acc[h][e];
+    }
+  __syncthreads();
+  if (tid == 0) {  // the barrier orders every thread's x stores before this release
+    __threadfence();
+    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(flags + bi), "r"(epoch) : "memory");
+  }
+}
+
 // The 128 x 128 diagonal blocks' inverses from the 64 x 64 ones (W64, as
 // trinv_kernel leaves them): lower [W0 0; -W1 T10 W0  W1], upper
 // [W0  -W0 T01 W1; 0 W1], with W1 = I when the last block has one sub-block.
@@ -264,40 +408,38 @@ trinv128_kernel(int n, const T *__restrict__ Tp, long tr, long tc, int lower, co
     for (int q = 0; q < 8; q++) s[(base + 256 * q) % CB][(base + 256 * q) / CB] = v[q];
   }
   __syncthreads();
-  // off-diagonal quadrant at (oi, ok); the products read the diagonal
-  // quadrants at (ok, ok) (first) and (oi, oi) (second)
-  const int oi = lower ? BS : 0, ok = lower ? 0 : BS;
-  T y[BS * BS / 256];
+  // off-diagonal quadrant at (oi, ok): Y = T W(ok, ok), then -W(oi, oi) Y.
+  // Every thread holds a 4 x 4 part of the 64 x 64 product (rows ti + 16 a,
+  // columns tj + 16 b), so a step of k costs 8 shared-memory loads for 16
+  // FMAs; one load per operand of each FMA took 35 us here, this takes 16.
+  const int oi = lower ? BS : 0, ok = lower ? 0 : BS, ti = tid % 16, tj = tid / 16;
+  T y[4][4];
 #pragma unroll
-  for (int e = 0; e < BS * BS / 256; e++) {
-    const int idx = tid + 256 * e, i = idx % BS, j = idx / BS;
-    T acc = T(0);
-#pragma unroll 16
-    for (int k = 0; k < BS; k++) acc = fma(s[oi + i][ok + k], s[ok + k][ok + j], acc);
-    y[e] = acc;
-  }
-  __syncthreads();
+  for (int pass = 0; pass < 2; pass++) {
+    const T *L = &s[oi + ti][pass ? oi : ok], *R = &s[pass ? oi : ok][ok + tj];
 #pragma unroll
-  for (int e = 0; e < BS * BS / 256; e++) {
-    const int idx = tid + 256 * e;
-    s[oi + idx % BS][ok + idx / BS] = y[e];
-  }
-  __syncthreads();
+    for (int a = 0; a < 4; a++)
 #pragma unroll
-  for (int e = 0; e < BS * BS / 256; e++) {
-    const int idx = tid + 256 * e, i = idx % BS, j = idx / BS;
-    T acc = T(0);
-#pragma unroll 16
-    for (int k = 0; k < BS; k++) acc = fma(s[oi + i][oi + k], s[oi + k][ok + j], acc);
-    y[e] = -acc;
-  }
-  __syncthreads();
+      for (int c = 0; c < 4; c++) y[a][c] = T(0);
+#pragma unroll 4
+    for (int k = 0; k < BS; k++) {
+      T l[4], r[4];
 #pragma unroll
-  for (int e = 0; e < BS * BS / 256; e++) {
-    const int idx = tid + 256 * e;
-    s[oi + idx % BS][ok + idx / BS] = y[e];
+      for (int a = 0; a < 4; a++) l[a] = L[16 * a * (CB + 1) + k];
+#pragma unroll
+      for (int c = 0; c < 4; c++) r[c] = R[k * (CB + 1) + 16 * c];
+#pragma unroll
+      for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) y[a][c] = fma(l[a], r[c], y[a][c]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) s[oi + ti + 16 * a][ok + tj + 16 * c] = pass ? -y[a][c] : y[a][c];
+    __syncthreads();
   }
-  __syncthreads();
   T *Wb = W128 + (long)b * CB * CB;
   for (int idx = tid; idx < CB * CB; idx += 256) Wb[idx] = s[idx % CB][idx / CB];
 }
@@ -330,21 +472,23 @@ template void trsv_inverse_dev<double>(int, int, int, int, const double *, long,
 template void trsv_inverse_dev<float>(int, int, int, int, const float *, long, float *, cudaStream_t);
 
 // Solve op(A) X = B in place (Left side only): the inverted diagonal blocks
-// once, then one launch per 8 right-hand sides.
+// once, then one launch per 16 (FP64) or 8 right-hand sides.
 template <typename T>
 void trsv_dev(int uplo, int trans, int diag, int n, int nrhs, const T *A, long lda, T *B, long ldb,
               cudaStream_t st) {
   if (n <= 0 || nrhs <= 0) return;
   T *W = (T *)scratch(kSlotTrsmW, sizeof(T) * trsv_w_elems(n));
   trsv_inverse_dev<T>(uplo, trans, diag, n, A, lda, W, st);
-  for (int c0 = 0; c0 < nrhs; c0 += 8)
-    trsv_w_dev<T>(uplo, trans, n, std::min(8, nrhs - c0), A, lda, W, B + (long)c0 * ldb, ldb, st);
+  constexpr int step = sizeof(T) == 8 ? 16 : 8;  // right-hand sides of one launch
+  for (int c0 = 0; c0 < nrhs; c0 += step)
+    trsv_w_dev<T>(uplo, trans, n, std::min(step, nrhs - c0), A, lda, W, B + (long)c0 * ldb, ldb, st);
 }
 template void trsv_dev<double>(int, int, int, int, int, const double *, long, double *, long, cudaStream_t);
 template void trsv_dev<float>(int, int, int, int, int, const float *, long, float *, long, cudaStream_t);
 
 // The same solve with the inverted diagonal blocks W already computed
-// (trsv_inverse_dev): for repeated solves with one factor.
+// (trsv_inverse_dev): for repeated solves with one factor; nrhs <= 16 (FP64)
+// or 8.
 template <typename T>
 void trsv_w_dev(int uplo, int trans, int n, int nrhs, const T *A, long lda, const T *W, T *B, long ldb,
                 cudaStream_t st) {
@@ -363,18 +507,36 @@ void trsv_w_dev(int uplo, int trans, int n, int nrhs, const T *A, long lda, cons
   ATLB_CUDA_CHECK(cudaMemsetAsync(ctl, 0, sizeof(int) * nctl + sizeof(unsigned long long) * ntag, st));
   // sW, sxd, sb, sacc (trsv_kernel's layout), for the largest NR
   constexpr int smem = (CB * (CB + 1) + (2 * CB + CB + NQ * CB) * 8) * (int)sizeof(T);
+  if constexpr (sizeof(T) == 8) {
+    if (nrhs > 4) {  // 4 columns and fewer: the MMA's eight would be half empty
+      constexpr int smem1 = (CB * (CB + 4) + 3 * CB * 12) * 8, smem2 = (CB * (CB + 4) + 3 * CB * 20) * 8;
+      static bool configured_m = false;
+      if (!configured_m) {
+        ATLB_CUDA_CHECK(cudaFuncSetAttribute(trsv_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1));
+        ATLB_CUDA_CHECK(cudaFuncSetAttribute(trsv_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2));
+        configured_m = true;
+      }
+      if (nrhs <= 8)
+        trsv_mma_kernel<1><<<nb, TT, smem1, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, err);
+      else
+        trsv_mma_kernel<2><<<nb, TT, smem2, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, err);
+      ATLB_CUDA_CHECK(cudaGetLastError());
+      return;
+    }
+  }
   static bool configured = false;
   if (!configured) {
     ATLB_CUDA_CHECK(cudaFuncSetAttribute(trsv_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     ATLB_CUDA_CHECK(cudaFuncSetAttribute(trsv_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    ATLB_CUDA_CHECK(cudaFuncSetAttribute(trsv_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if constexpr (sizeof(T) == 4)
+      ATLB_CUDA_CHECK(cudaFuncSetAttribute(trsv_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     configured = true;
   }
   if (nrhs == 1)
     trsv_kernel<T, 1><<<nb, TT, smem, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, err, xt);
   else if (nrhs <= 4)
     trsv_kernel<T, 4><<<nb, TT, smem, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, err, xt);
-  else
+  else if constexpr (sizeof(T) == 4)
     trsv_kernel<T, 8><<<nb, TT, smem, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, err, xt);
   ATLB_CUDA_CHECK(cudaGetLastError());
 }

@@ -123,6 +123,50 @@ def test_potrf_vs_oracle(gpu, orc, uplo, n):
     assert np.array_equal(a[:n][other], a0[other])
 
 
+@pytest.mark.parametrize("nrhs", [4, 5, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 300, 520])
+def test_few_rhs_solves_at_block_edges(gpu, n, nrhs):
+    """potrs and getrs across the right-hand sides one launch takes and the
+    128-row blocks: each solve's residual <= gamma |L||U||x| componentwise, with
+    gamma = 4 (n + 128) u for the inverted 128 x 128 diagonal blocks times their
+    largest condition number here (diagonally dominant factors: < 8)."""
+    rng = np.random.default_rng(n * 100 + nrhs)
+    u, ldb = 2.0 ** -53, n + 3
+    g = rng.uniform(-1, 1, (n, n))
+    sym = np.asfortranarray(g @ g.T / n + 4 * np.eye(n))
+    gen = np.asfortranarray(g / np.sqrt(n) + 4 * np.eye(n))
+    b0 = np.full((ldb, nrhs), 3.0, order="F")
+    b0[:n] = rng.uniform(-1, 1, (n, nrhs))
+    for uplo in (121, 122):
+        f = sym.copy(order="F")
+        b = b0.copy(order="F")
+        assert AB.clapack_dpotrf(CM, uplo, n, f, n) == 0
+        assert AB.clapack_dpotrs(CM, uplo, n, nrhs, f, n, b, ldb) == 0
+        low = np.abs(np.tril(f) if uplo == 122 else np.triu(f).T)
+        assert np.array_equal(b[n:], b0[n:])
+        bound = 8 * 4 * (n + 128) * u * (low @ (low.T @ np.abs(b[:n])))
+        assert np.all(np.abs(sym @ b[:n] - b0[:n]) <= bound)
+    lu = gen.copy(order="F")
+    ipiv = np.zeros(n, dtype=np.int32)
+    assert AB.clapack_dgetrf(CM, n, n, lu, n, ipiv) == 0
+    low, up = np.abs(np.tril(lu, -1) + np.eye(n)), np.abs(np.triu(lu))
+    perm = np.arange(n)
+    for k in range(n):
+        perm[[k, ipiv[k]]] = perm[[ipiv[k], k]]
+    for trans in (111, 112):
+        b = b0.copy(order="F")
+        assert AB.clapack_dgetrs(CM, trans, n, nrhs, lu, n, ipiv, b, ldb) == 0
+        assert np.array_equal(b[n:], b0[n:])
+        x = np.abs(b[:n])
+        if trans == 111:
+            mag = np.zeros_like(x)
+            mag[perm] = low @ (up @ x)
+            res = np.abs(gen @ b[:n] - b0[:n])
+        else:
+            mag, res = up.T @ (low.T @ x[perm]), np.abs(gen.T @ b[:n] - b0[:n])
+        assert np.all(res <= 8 * 4 * (n + 128) * u * mag)
+
+
 @pytest.mark.parametrize("uplo", [121, 122])
 @pytest.mark.parametrize("n,bad", [(1, 0), (15, 0), (16, 0), (17, 17), (129, 0), (240, 200), (255, 0), (256, 0),
                                    (256, 241), (256, 256), (257, 0)])
