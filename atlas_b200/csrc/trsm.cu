@@ -359,7 +359,7 @@ void eff_update(const Eff<T> &e, int r2, int n2, int r1, int n1, int m, SgemmFn 
 // before is multiplied.  It is what the Cholesky's block columns wait for:
 // the recursion below 256 (inverse times 64 rows, a coupling product, the next
 // inverse) took three launches and 66 us for an order of 128 and 8000 columns,
-// this takes BLK_US.
+// this takes 24.
 constexpr int TBK_N = 256;
 template <int CT>
 constexpr int tri_block_smem(int n) { return 8 * ((n + LEAF - 1) / LEAF * LEAF * (CT + 4) + 2 * LEAF * (LEAF + 4)); }
