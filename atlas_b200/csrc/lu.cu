@@ -327,9 +327,10 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks(), crank = (int)cl.block_rank();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int TH = blockDim.x, nw = TH >> 5;  // threads (= rows) and warps of a CTA
   const int MN = min(M, ncols);
   extern __shared__ __align__(16) unsigned char fused_smem[];
-  T *Lsm = reinterpret_cast<T *>(fused_smem);  // [NB][PT]: finished row parts
+  T *Lsm = reinterpret_cast<T *>(fused_smem);  // [NB][TH]: finished row parts
   __shared__ Slot slot[2][kMaxPanelCluster];
   __shared__ __align__(8) unsigned long long mbar[2];
   __shared__ __align__(16) T wu[2][PT / 32][NB];  // per-warp copy of the pivot row, by column parity
@@ -351,7 +352,7 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
   cluster_arrive();  // every CTA's barriers exist before anyone sends
   cluster_wait();
 
-  const int r = crank * PT + tid;
+  const int r = crank * TH + tid;
   bool act = r < M;
   int pos = r;
   T a[NB];
@@ -384,8 +385,7 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
     const int wl = warp_argmax_lane(v, p);
     if (lane == wl) { wv[b][warp] = v; wp[b][warp] = p; }
     __syncthreads();
-    const int wc = warp_argmax_lane(lane < PT / 32 ? wv[b][lane] : K(0),
-                                    lane < PT / 32 ? wp[b][lane] : 0xffffffffu);
+    const int wc = warp_argmax_lane(lane < nw ? wv[b][lane] : K(0), lane < nw ? wp[b][lane] : 0xffffffffu);
     if (warp == wc) {  // the warp of the CTA's candidate (or, without one, of a key that never wins)
       const bool owner = act && lane == wl;
       if (owner) {
@@ -404,11 +404,9 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
         stage.pos = -1;
       }
     }
-    // kUnits x C messages of 16 bytes, at most one per thread
-    static_assert(kUnits * kMaxPanelCluster <= PT, "one message per thread");
     __syncthreads();
-    if (tid < kUnits * C) {
-      const int q = tid / kUnits, unit = tid - q * kUnits;
+    for (int i = tid; i < kUnits * C; i += TH) {  // kUnits x C messages of 16 bytes
+      const int q = i / kUnits, unit = i - q * kUnits;
       st_async16(mapa_u32(smem_u32(&slot[b][crank]) + 16 * unit, q), reinterpret_cast<const uint4 *>(&stage)[unit],
                  mapa_u32(mb, q));
     }
@@ -474,7 +472,7 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
         else l = a[0] / piv;
         lm = nz ? l : T(0);
         a[0] = fma(-lm, nz ? u1 : T(0), a[1]);  // the next column first: it decides the next pivot
-        Lsm[j * PT + tid] = l;
+        Lsm[j * TH + tid] = l;
         A[r + (long)j * lda] = l;  // at the row's original place (moved rows are rewritten at the end)
       }
     }
@@ -489,10 +487,10 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
   }
 
   if (piv_row) {  // the U part of a pivot row: columns pos.. of the panel
-    T *dst = Lsm + pos * PT + tid;
+    T *dst = Lsm + pos * TH + tid;
 #pragma unroll
     for (int k = 0; k < NB; k++)
-      if (pos + k < ncols) dst[k * PT] = a[k];
+      if (pos + k < ncols) dst[k * TH] = a[k];
   }
   // Rows that moved register (from, to) in CTA 0's list, for the block's
   // other columns.  After one cluster barrier (which also orders the
@@ -514,7 +512,7 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
   cluster_wait();
   if (in && (pos != r || piv_row)) {
     const int k0 = pos != r ? 0 : pos;
-    for (int k = k0; k < ncols; k++) A[pos + (long)k * lda] = Lsm[k * PT + tid];
+    for (int k = k0; k < ncols; k++) A[pos + (long)k * lda] = Lsm[k * TH + tid];
   }
   if (nother == 0) return;
   // The block's other columns of the rows that moved (at most 2*MN rows):
@@ -522,9 +520,9 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
   // values into shared memory and writes them to their final rows.
   __shared__ int l_from[2 * NB], l_to[2 * NB];
   const int nm = min(*cl.map_shared_rank(&s_nmoved, 0), 2 * NB);
-  if (tid < nm) {
-    l_from[tid] = cl.map_shared_rank(s_from, 0)[tid];
-    l_to[tid] = cl.map_shared_rank(s_to, 0)[tid];
+  for (int i = tid; i < nm; i += TH) {
+    l_from[i] = cl.map_shared_rank(s_from, 0)[i];
+    l_to[i] = cl.map_shared_rank(s_to, 0)[i];
   }
   __syncthreads();  // the list is here and Lsm is free
   // CTA 0's shared memory must outlive the other CTAs' reads of its list: a
@@ -532,12 +530,12 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
   const bool u12 = nright > 0 && MN > 1;
   if (!u12) cluster_arrive();
   const int per = (nother + C - 1) / C, g0 = crank * per, ncol = max(0, min(nother, g0 + per) - g0);
-  const int total = nm * ncol;  // <= 2 NB x NB*PT/(2 NB): fits Lsm
-  for (int base = tid; base < total; base += 4 * PT) {
+  const int total = nm * ncol;  // <= 2 NB x the CTA's share of the columns: fits (launch_fused_panel)
+  for (int base = tid; base < total; base += 4 * TH) {
     T v[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-      const int g = base + q * PT;
+      const int g = base + q * TH;
       if (g < total) {
         const int i = g % nm, c = g0 + g / nm;
         const int col = c < nleft ? c - nleft : ncols + (c - nleft);
@@ -546,10 +544,10 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
     }
 #pragma unroll
     for (int q = 0; q < 4; q++)
-      if (base + q * PT < total) Lsm[base + q * PT] = v[q];
+      if (base + q * TH < total) Lsm[base + q * TH] = v[q];
   }
   __syncthreads();
-  for (int g = tid; g < total; g += PT) {
+  for (int g = tid; g < total; g += TH) {
     const int i = g % nm, c = g0 + g / nm;
     const int col = c < nleft ? c - nleft : ncols + (c - nleft);
     A[l_to[i] + (long)col * lda] = Lsm[g];
@@ -562,7 +560,7 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
   cluster_arrive();  // every row is in place
   cluster_wait();
   // U12 = L11^-1 A12 on the right columns' top MN rows, over all the cluster's warps
-  panel_u12_solve<T, NB>(MN, ncols, nright, crank * (PT / 32) + warp, C * (PT / 32), A, lda);
+  panel_u12_solve<T, NB>(MN, ncols, nright, crank * nw + warp, C * nw, A, lda);
 }
 
 // Fallback for panels taller than a cluster can hold: one CTA, global memory.
@@ -720,12 +718,20 @@ template <typename T>
 bool launch_fused_panel(int M, int ncols, T *A, long lda, int *ipiv, int roff, int *dinfo, int nleft,
                         int nright, cudaStream_t st) {
   if (ncols > 32 || nleft + nright > 256) return false;  // the interchange staging holds 64 x 256
-  const int C = cdiv(M, PT);
-  if (C > max_cluster_fused<T>()) return false;
+  const int most = max_cluster_fused<T>();
+  if (cdiv(M, PT) > most) return false;
+  // As many CTAs as the cluster takes, as few rows in each: what a column costs
+  // inside a CTA grows with its warps, which share the issue slots and the
+  // shared memory that every one of them reads the pivot row from.  At least 128,
+  // below which the messages cost more than the warps (FP64 LU with 512 / 256 /
+  // 128 / 64 / 32: order 500 1.20 / 1.11 / 1.08 / 1.12 / 1.21 ms, order 2000
+  // 4.40 / 3.93 / 3.86 / 3.97 / 4.05).
+  const int rows = std::max(128, cdiv(cdiv(M, most), 32) * 32), C = cdiv(M, rows);
+  const size_t smem = sizeof(T) * std::max(32 * rows, 64 * cdiv(nleft + nright, C));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C, 1, 1);
-  cfg.blockDim = dim3(PT, 1, 1);
-  cfg.dynamicSmemBytes = fused_smem_bytes<T>();
+  cfg.blockDim = dim3(rows, 1, 1);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1002,7 +1008,7 @@ void getrs_dev(int trans, int N, int NRHS, const T *A, long lda, const int *ipiv
                cudaStream_t st, SgemmFn gemm) {
   // ATL_getrs column-major (src/lapack/ATL_getrs.c:34-50)
   if (N <= 0 || NRHS <= 0) return;
-  if (NRHS <= kTrsvMaxRhs) {  // few right-hand sides: blocked solves, one launch per 8 columns
+  if (NRHS <= kTrsvMaxRhs) {  // few right-hand sides: blocked solves, one launch per 8 (FP64: 16) columns
     if (trans == kNoTrans) {
       laswp_dev<T>(NRHS, B, ldb, 0, N, ipiv, 1, st);
       trsv_dev<T>(kLower, kNoTrans, kUnit, N, NRHS, A, lda, B, ldb, st);

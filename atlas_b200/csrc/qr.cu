@@ -30,7 +30,7 @@ namespace cg = cooperative_groups;
 namespace atlb {
 namespace {
 
-constexpr int QT = 512;
+constexpr int QT = 512;  // threads of a panel CTA, at most
 constexpr int NBQ_MAX = 128;  // widest panel factored in one piece (wider panels: two halves)
 
 // lane l returns sum over the warp of v[l % NB]; v is destroyed
@@ -64,11 +64,11 @@ __device__ int g_qr_timeout = 0;
 template <int NB, int RPT>
 __global__ void __launch_bounds__(QT, 1)
 geqr2_cluster_kernel(int M, int ncols, double *__restrict__ A, long lda, double *__restrict__ tau) {
-  static_assert(NB <= 32 && 16 * NB <= QT, "one lane per column, one thread per (CTA, column)");
+  static_assert(NB <= 32, "one lane per column");
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks(), crank = (int)cl.block_rank();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int TOT = C * QT;
+  const int TH = blockDim.x, nw = TH >> 5, TOT = C * TH;
   const int K = min(M, ncols);
 
   __shared__ double part[2][16][NB];           // every CTA's partial dot products, by column parity
@@ -89,7 +89,7 @@ geqr2_cluster_kernel(int M, int ncols, double *__restrict__ A, long lda, double 
   int rows[RPT];
 #pragma unroll
   for (int q = 0; q < RPT; q++) {
-    int r = crank * QT + tid + q * TOT;
+    int r = crank * TH + tid + q * TOT;
     rows[q] = r;
 #pragma unroll
     for (int k = 0; k < NB; k++) a[q][k] = (r < M && k < ncols) ? A[r + (long)k * lda] : 0.0;
@@ -123,11 +123,11 @@ geqr2_cluster_kernel(int M, int ncols, double *__restrict__ A, long lda, double 
       for (int k = 0; k < NB; k++) own_row[b][k] = a[0][k];
     }
     __syncthreads();
-    if (tid < C * NB) {  // thread (CTA, column): this CTA's sum to that CTA
-      const int dst = tid / NB, k = tid % NB;
+    for (int i = tid; i < C * NB; i += TH) {  // (CTA, column): this CTA's sum to that CTA
+      const int dst = i / NB, k = i % NB;
       double t[QT / 32];
 #pragma unroll
-      for (int w = 0; w < QT / 32; w++) t[w] = red[w][k];
+      for (int w = 0; w < QT / 32; w++) t[w] = w < nw ? red[w][k] : 0.0;
 #pragma unroll
       for (int h = QT / 64; h >= 1; h >>= 1)
 #pragma unroll
@@ -271,7 +271,11 @@ int g_qr_max_cluster = 0;
 
 template <int NB, int RPT>
 void launch_geqr2_cluster(int M, int ncols, double *A, long lda, double *tau, cudaStream_t st) {
-  int C = cdiv(M, QT * RPT);
+  // as many CTAs as the cluster takes, as few threads in each, down to 128
+  // (launch_fused_panel in lu.cu has the reason; 300 x 200 with 512 / 256 / 128 /
+  // 64 threads: 0.80 / 0.61 / 0.53 / 0.58 ms, 2000 x 1000 4.31 / 3.39 / 3.57 / 3.78)
+  const int threads = std::min(QT, std::max(128, cdiv(cdiv(M, g_qr_max_cluster * RPT), 32) * 32));
+  const int C = cdiv(M, threads * RPT);
   auto kern = geqr2_cluster_kernel<NB, RPT>;
   static bool configured = false;
   if (!configured) {
@@ -280,7 +284,7 @@ void launch_geqr2_cluster(int M, int ncols, double *A, long lda, double *tau, cu
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C, 1, 1);
-  cfg.blockDim = dim3(QT, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
