@@ -94,12 +94,15 @@ batched_posv_kernel(const Prob *__restrict__ probs, const int *__restrict__ orde
 //      current position on ties = cblas_idamax / ATL_getf2) goes to shared
 //      memory before it, every thread picks the winner after it.  Rows do not
 //      move: each carries its current position;
-//   2. one thread per column outside the panel, right-hand sides included,
+//   2. one thread per column right of the panel, right-hand sides included,
 //      applies the panel's interchanges (only the top 16 rows and the pivot
-//      rows change: one gather, one scatter) and, right of the panel, solves
-//      U12 = L11^-1 A12 in registers;
+//      rows change: one gather, one scatter) and solves U12 = L11^-1 A12 in
+//      registers;
 //   3. A22 -= L21 U12 on the FP64 tensor cores, L21 and U12 from shared
 //      memory, the next part of A22 loaded under the products.
+// The interchanges of the columns left of the panels wait until the end, where
+// they are composed: applied panel by panel they moved as many bytes as step 2,
+// a sector per entry (11.1 ms, with step 2's top rows read column by column).
 // Up to eight right-hand sides ride along in shared memory, which makes the
 // forward substitution part of the factorization.  What bounds it: the chain
 // of columns (about 16 x 500 cycles a panel) and the L2 round trips of steps
@@ -109,7 +112,7 @@ batched_posv_kernel(const Prob *__restrict__ probs, const int *__restrict__ orde
 // 10,000 problems of orders 8..256 with one right-hand side, B200: getrf and
 // getrs kernels 14.5 + 3.0 ms before (two barriers and a shared-memory rank-1
 // update per column, interchanges and U12 as separate passes, a solve with
-// loads of the factor on its chain), 11.1 ms now for both.
+// loads of the factor on its chain), 9.7 ms now for both.
 constexpr int LPW = 16;         // panel width
 constexpr int LU_RHS = 8;       // right-hand sides carried along
 constexpr int LU_LDU = LPW + 4; // U12 copy, U(q, k) at k * LU_LDU + q
@@ -126,7 +129,8 @@ struct LuSmem {
   int cpos[2][NT / 32];
   double D[2][LPW * DLD];             // diagonal blocks of the solves, D(r, q) at q * DLD + r
   int from[LPW], to[LPW];             // row whose content ends at q; where row q's content ends
-  int moved, fail;
+  int piv[NT];                        // ipiv
+  int fail;
 };
 
 // step 1.  a[]: this thread's row of the panel (row tid of m, jb <= 16
@@ -164,6 +168,7 @@ __device__ __forceinline__ int lu_panel(LuSmem<NT> &S, double (&a)[LPW], int m, 
     const double piv = u[0];
     if (tid == 0) {
       ipiv[j0 + c] = j0 + p;
+      S.piv[j0 + c] = j0 + p;
       if (piv == 0.0 && !S.fail) S.fail = j0 + c + 1;
     }
     if (act) {
@@ -283,7 +288,6 @@ __device__ __forceinline__ int lu_factor(const Prob &pr, int nr, LuSmem<NT> &S) 
       S.from[tid] = tid;
       S.to[tid] = tid;
     }
-    if (tid == 0) S.moved = 0;
     __syncthreads();
     const int pos = lu_panel<NT>(S, a, m, jb, j, pr.ipiv);
 #pragma unroll
@@ -297,37 +301,45 @@ __device__ __forceinline__ int lu_factor(const Prob &pr, int nr, LuSmem<NT> &S) 
       }
       if (pos < LPW) S.from[pos] = tid;
       if (tid < LPW) S.to[tid] = pos;
-      if (pos != tid) S.moved = 1;
     }
     __syncthreads();
-    // step 2
-    const int ncol = n - jb + nr;
+    // step 2: the columns right of the panel and the right-hand sides.  Their
+    // top 16 rows come to U and go back from it 16 rows at a time; a column's
+    // thread touches global memory only for the pivot rows below them.
+    double *R = A + j + (long)(j + jb) * lda;
+    for (int e = tid; e < nt * LPW; e += NT) {  // nt > 0: the panel has 16 columns
+      const int q = e & (LPW - 1), k = e / LPW;
+      S.U[k * LU_LDU + q] = R[q + k * lda];
+    }
+    __syncthreads();
 #pragma unroll 1
-    for (int cc = tid; cc < ncol; cc += NT) {
-      const bool left = cc < j, rhs = cc >= n - jb;
-      if (left && !S.moved) continue;
-      double *col = rhs ? S.xs + (cc - (n - jb)) * NT + j : A + j + (long)(left ? cc : cc + jb) * lda;
+    for (int cc = tid; cc < nt + nr; cc += NT) {
+      const bool rhs = cc >= nt;
+      double *col = rhs ? S.xs + (cc - nt) * NT + j : R + cc * lda, *u = rhs ? col : S.U + cc * LU_LDU;
       double x[LPW];  // shifted below: x[0] is the current row
 #pragma unroll
-      for (int q = 0; q < LPW; q++) x[q] = q < jb ? col[S.from[q]] : 0.0;
-      if (S.moved) {
-#pragma unroll 4
-        for (int q = 0; q < LPW; q++) {
-          const int to = S.to[q];
-          if (to >= LPW) col[to] = col[q];
-        }
+      for (int q = 0; q < LPW; q++) {
+        const int from = S.from[q];
+        x[q] = q >= jb ? 0.0 : from < LPW ? u[from] : col[from];
       }
-      double *u = S.U + (cc - j) * LU_LDU;
+#pragma unroll 4
+      for (int q = 0; q < LPW; q++) {
+        const int to = S.to[q];
+        if (to >= LPW) col[to] = u[q];
+      }
 #pragma unroll 1
       for (int q = 0; q < jb; q++) {
         const double v = x[0];
-        col[q] = v;
-        if (!left && !rhs) u[q] = v;
+        u[q] = v;
         const double *l = S.P + q * LDP + q;
-        const double f = left ? 0.0 : v;  // left of the panel: interchanges only
 #pragma unroll
-        for (int r = 1; r < LPW; r++) x[r - 1] = fma(-l[r], f, x[r]);
+        for (int r = 1; r < LPW; r++) x[r - 1] = fma(-l[r], v, x[r]);
       }
+    }
+    __syncthreads();
+    for (int e = tid; e < nt * LPW; e += NT) {
+      const int q = e & (LPW - 1), k = e / LPW;
+      R[q + k * lda] = S.U[k * LU_LDU + q];
     }
     __syncthreads();
     if (nt > 0) {
@@ -341,6 +353,28 @@ __device__ __forceinline__ int lu_factor(const Prob &pr, int nr, LuSmem<NT> &S) 
         }
       lu_update<NT>(S, nt, nt, A + (j + jb) + (long)(j + jb) * lda, lda);
     }
+    __syncthreads();
+  }
+  // The interchanges of the columns left of each panel, all at once: `src` is
+  // the row whose entry ends in this thread's row, composed from the last panel
+  // back; every panel's multipliers are read and written once, in whole rows.
+  int src = tid;
+#pragma unroll 1
+  for (int j = (n - 1) / LPW * LPW; j > 0; j -= LPW) {  // panel j moves the rows of panel j - 16
+#pragma unroll 1
+    for (int c = min(LPW, n - j) - 1; c >= 0; c--) {
+      const int p = S.piv[j + c];
+      src = src == j + c ? p : src == p ? j + c : src;
+    }
+    double *L = A + (long)(j - LPW) * lda;
+    const bool in = tid >= j && tid < n;
+    if (in)
+#pragma unroll
+      for (int q = 0; q < LPW; q++) S.P[q * LDP + tid] = L[tid + q * lda];
+    __syncthreads();
+    if (in && src != tid)
+#pragma unroll
+      for (int q = 0; q < LPW; q++) L[tid + q * lda] = S.P[q * LDP + src];
     __syncthreads();
   }
   return S.fail;
@@ -595,7 +629,7 @@ void batched_gesv_dev(const std::vector<Prob> &P, int *info_out, cudaStream_t st
     enqueue_upload(b, st);
     if (used & 1) launch_gesv<256, 2>(b, 0, st);
     if (used & 2) launch_gesv<128, 4>(b, 1, st);
-    if (used & 4) launch_gesv<64, 8>(b, 2, st);
+    if (used & 4) launch_gesv<64, 7>(b, 2, st);
     ATLB_CUDA_CHECK(cudaMemcpyAsync(info_out, b.info, sizeof(int) * count, cudaMemcpyDeviceToHost, st));
   });
 }
