@@ -144,7 +144,7 @@ __device__ __forceinline__ void dgemm_tile(int M, int N, int K, double alpha, co
 
   const int KT = (K + BK - 1) / BK;
 #pragma unroll
-  for (int s = 0; s < STG; s++) {
+  for (int s = 0; s < STG - 1; s++) {
     if (s < KT) {
       load_tile<TA, VEC, BM>(sA + s * LA::SIZE, A, lda, m0, s * BK, M, K, tid);
       load_tile<!TB, VEC, BNT>(sB + s * LB::SIZE, B, ldb, n0, s * BK, N, K, tid);
@@ -164,9 +164,12 @@ __device__ __forceinline__ void dgemm_tile(int M, int N, int K, double alpha, co
   // copies, waiting for the first fragments behind the barrier.  Fragments
   // are therefore loaded one k-step ahead, the barrier that opens the next k
   // tile stands before the last k-step's products (whose fragments are in
-  // registers already), and the copies that refill the stage just finished
-  // are issued behind those products.  8192^3: 31.5 -> 34.3 TFLOP/s (cuBLAS
-  // 35.5); 8192^2 x K with C read back: K = 128 23.4 -> 25.8, 256 27.6 -> 28.7.
+  // registers already), and the copies that refill the stage finished before
+  // it are issued behind products too, A's and B's behind different k-steps: one
+  // burst of both behind the last k-step needs more address registers than
+  // there are (255 and spills without alignment; 1501 x 1203 x 999, A
+  // transposed, 193 us, now 159).  8192^3: 31.5 -> 34.7 TFLOP/s (cuBLAS 35.5);
+  // 8192^2 x K with C read back: K = 128 23.4 -> 25.8, 256 27.6 -> 28.7.
   const int fr = lane >> 2, fk = lane & 3;
   double a[2][MI], b[2][4];
   auto fragments = [&](int buf, const double *a_s, const double *b_s, int kk) {
@@ -175,18 +178,19 @@ __device__ __forceinline__ void dgemm_tile(int M, int N, int K, double alpha, co
 #pragma unroll
     for (int j = 0; j < 4; j++) b[buf][j] = b_s[LB::at(wn + j * 8 + fr, kk + fk)];
   };
-  cp_async_wait<STG - 1>();
+  cp_async_wait<STG - 2>();
   __syncthreads();
   fragments(0, sA, sB, 0);
-  int stage = 0;
+  int stage = 0, refill = STG - 1;  // the stage read now, the one read before it
   for (int kt = 0; kt < KT; kt++) {
-    double *a_s = sA + stage * LA::SIZE, *b_s = sB + stage * LB::SIZE;
+    const double *a_s = sA + stage * LA::SIZE, *b_s = sB + stage * LB::SIZE;
     stage = stage + 1 == STG ? 0 : stage + 1;
 #pragma unroll
     for (int s = 0; s < BK / 4; s++) {
       if (s < BK / 4 - 1) {
         fragments((s + 1) & 1, a_s, b_s, 4 * (s + 1));
       } else {
+        cp_async_commit();
         cp_async_wait<STG - 2>();
         __syncthreads();  // tile kt + 1 has landed, and nobody reads tile kt's stage any more
         if (kt + 1 < KT) fragments((s + 1) & 1, sA + stage * LA::SIZE, sB + stage * LB::SIZE, 0);
@@ -195,12 +199,13 @@ __device__ __forceinline__ void dgemm_tile(int M, int N, int K, double alpha, co
       for (int i = 0; i < MI; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) dmma(acc[i][j], a[s & 1][i], b[s & 1][j]);
+      if (kt + STG - 1 < KT) {
+        const int k0 = (kt + STG - 1) * BK;
+        if (s == 0) load_tile<TA, VEC, BM>(sA + refill * LA::SIZE, A, lda, m0, k0, M, K, tid);
+        if (s == 1) load_tile<!TB, VEC, BNT>(sB + refill * LB::SIZE, B, ldb, n0, k0, N, K, tid);
+      }
     }
-    if (kt + STG < KT) {
-      load_tile<TA, VEC, BM>(a_s, A, lda, m0, (kt + STG) * BK, M, K, tid);
-      load_tile<!TB, VEC, BNT>(b_s, B, ldb, n0, (kt + STG) * BK, N, K, tid);
-    }
-    cp_async_commit();
+    refill = refill + 1 == STG ? 0 : refill + 1;
   }
   cp_async_wait<0>();
 
