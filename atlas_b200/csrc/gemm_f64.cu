@@ -550,8 +550,16 @@ void launch(int M, int N, int K, double alpha, const double *A, long lda, const 
     ATLB_CUDA_CHECK(cudaGetLastError());
     return;
   }
-  if (K <= SMALL_K) {
-    dgemm_dmma_kernel<TA, TB, VEC, 64><<<cdiv(M, BM) * cdiv(N, 64), THREADS, smem_s, st>>>(
+  // 128 x 64 tiles with long K too where they leave less of the last wave idle:
+  // an SM computes two of them in the time of one 128 x 128 tile and 8 % (900 x
+  // 1500 x 3000, as many waves both ways: 430 and 466 us), so they pay from
+  // there (1700 x 1700 x 700, 196 tiles in 2 waves or 378 in 3 halves: 229 and
+  // 183 us).  Not where a triangle is masked, whose tiles this does not count,
+  // or a cap leaves SMs to another stream.
+  const int tiles_n64 = cdiv(M, BM) * cdiv(N, 64);
+  const bool finer = tri == 0 && cap == 0 && 27 * cdiv(tiles_n64, nsm) < 50 * cdiv(tiles, nsm);
+  if (K <= SMALL_K || finer) {
+    dgemm_dmma_kernel<TA, TB, VEC, 64><<<tiles_n64, THREADS, smem_s, st>>>(
         M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, tri, tune(kTuneGemmGroup));
   } else {
     dgemm_dmma_kernel<TA, TB, VEC, BN><<<tiles, THREADS, smem, st>>>(M, N, K, alpha, A, lda, B, ldb,
