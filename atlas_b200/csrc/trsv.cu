@@ -233,8 +233,8 @@ trsv_kernel(int n, int nrhs, const T *__restrict__ Tp, long tr, long tc, int low
   }
 }
 
-// The same solve for 5..16 FP64 right-hand sides, 8 NH per launch, with the
-// products on the FP64 tensor cores.  A chain step (the product with the block
+// The same solve in FP64 for up to 8 NH right-hand sides, with the products on
+// the FP64 tensor cores.  A chain step (the product with the block
 // just before, then the one with the inverted diagonal block) is 128 x 128 x 8
 // twice: with FMAs every term needs its x from shared memory (8192^2, 8
 // right-hand sides: 13.5 us a block), while the MMA's n = 8 columns are the
@@ -242,7 +242,12 @@ trsv_kernel(int n, int nrhs, const T *__restrict__ Tp, long tr, long tc, int low
 // owns rows 8 w .. 8 w + 7; its fragments of T come from global memory before
 // the wait.  Two groups of columns share every fragment of T and the chain's
 // latency, hence up to 16 per launch: 8192^2, 16 right-hand sides, one
-// direction 472 us; with FMAs, eight at a time, 2 x 860.
+// direction 472 us; with FMAs, eight at a time, 2 x 860.  The step is bound by
+// its latency, so even one right-hand side, with seven of the eight columns
+// zero, is faster than with FMAs: both directions of 8192^2 in 764 us for 1..4
+// right-hand sides (FMAs: 1 one 1054, 2..4 1266), of 3000^2 in 298 (358, 436),
+// of 1000^2 in 144 (157, 183).  Only one right-hand side over one or two blocks,
+// where nothing chains, keeps the FMAs (200^2: 80.7 us, here 84.4).
 template <int NH>
 __global__ void __launch_bounds__(TT, 1)
 trsv_mma_kernel(int n, int nrhs, const double *__restrict__ Tp, long tr, long tc, int lower,
@@ -508,7 +513,7 @@ void trsv_w_dev(int uplo, int trans, int n, int nrhs, const T *A, long lda, cons
   // sW, sxd, sb, sacc (trsv_kernel's layout), for the largest NR
   constexpr int smem = (CB * (CB + 1) + (2 * CB + CB + NQ * CB) * 8) * (int)sizeof(T);
   if constexpr (sizeof(T) == 8) {
-    if (nrhs > 4) {  // 4 columns and fewer: the MMA's eight would be half empty
+    if (nrhs > 1 || n > 2 * CB) {
       constexpr int smem1 = (CB * (CB + 4) + 3 * CB * 12) * 8, smem2 = (CB * (CB + 4) + 3 * CB * 20) * 8;
       static bool configured_m = false;
       if (!configured_m) {
@@ -527,17 +532,19 @@ void trsv_w_dev(int uplo, int trans, int n, int nrhs, const T *A, long lda, cons
   static bool configured = false;
   if (!configured) {
     ATLB_CUDA_CHECK(cudaFuncSetAttribute(trsv_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    ATLB_CUDA_CHECK(cudaFuncSetAttribute(trsv_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    if constexpr (sizeof(T) == 4)
+    if constexpr (sizeof(T) == 4) {
+      ATLB_CUDA_CHECK(cudaFuncSetAttribute(trsv_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       ATLB_CUDA_CHECK(cudaFuncSetAttribute(trsv_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    }
     configured = true;
   }
-  if (nrhs == 1)
-    trsv_kernel<T, 1><<<nb, TT, smem, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, err, xt);
-  else if (nrhs <= 4)
-    trsv_kernel<T, 4><<<nb, TT, smem, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, err, xt);
-  else if constexpr (sizeof(T) == 4)
-    trsv_kernel<T, 8><<<nb, TT, smem, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, err, xt);
+  auto go = [&](auto kern) {
+    kern<<<nb, TT, smem, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, err, xt);
+  };
+  if constexpr (sizeof(T) == 8) go(trsv_kernel<T, 1>);
+  else if (nrhs == 1) go(trsv_kernel<T, 1>);
+  else if (nrhs <= 4) go(trsv_kernel<T, 4>);
+  else go(trsv_kernel<T, 8>);
   ATLB_CUDA_CHECK(cudaGetLastError());
 }
 template void trsv_w_dev<double>(int, int, int, int, const double *, long, const double *, double *, long,

@@ -123,8 +123,8 @@ def test_potrf_vs_oracle(gpu, orc, uplo, n):
     assert np.array_equal(a[:n][other], a0[other])
 
 
-@pytest.mark.parametrize("nrhs", [4, 5, 8, 9, 16, 17, 32])
-@pytest.mark.parametrize("n", [1, 127, 128, 129, 300, 520])
+@pytest.mark.parametrize("nrhs", [1, 2, 3, 4, 5, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 256, 257, 300, 520])
 def test_few_rhs_solves_at_block_edges(gpu, n, nrhs):
     """potrs and getrs across the right-hand sides one launch takes and the
     128-row blocks: each solve's residual <= gamma |L||U||x| componentwise, with
