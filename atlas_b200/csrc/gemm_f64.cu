@@ -92,6 +92,33 @@ __device__ __forceinline__ void load_tile(double *s, const double *X, long ld, i
   }
 }
 
+// The same for 16-byte copies of tiles that lie wholly inside the operand, from a
+// pointer to the thread's first element: no bounds to test, and the addresses of a
+// thread's copies are a fixed stride apart.  Bounds and 64-bit addresses were most
+// of the instructions of a short-K tile (a 128 x 64 tile with K = 128: 38,000 warp
+// instructions, 4,096 of them products); with this and the untested epilogue
+// 8192^2 x 128 goes from 25.8 to 28.3 TFLOP/s, 8192^3 from 34.7 to 35.7.  Eight-byte
+// copies keep the tested form: twice the addresses left the registers short (1501 x
+// 1203 x 999, A transposed: 160 -> 178 us).
+template <bool KC, int BO> struct TileCopy {
+  using L = Lay<KC, BO>;
+  static constexpr int PER = (KC ? BK : BO) / 2;  // copies along the contiguous direction
+  static constexpr int ROWS = THREADS / PER, N = BO * BK / 2 / THREADS;
+  static __device__ __forceinline__ const double *first(const double *X, long ld, int o0, int tid) {
+    const int c = tid % PER * 2, r = tid / PER;
+    return KC ? X + c + (long)(o0 + r) * ld : X + o0 + c + (long)r * ld;
+  }
+  static __device__ __forceinline__ void go(double *s, const double *g, long ld, int tid) {
+    double *d = s + tid / PER * L::LD + tid % PER * 2;
+    const long step = ROWS * ld;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      cp_async16(d + i * ROWS * L::LD, g, true);
+      g += step;
+    }
+  }
+};
+
 // Tile shapes.  BNT = 128: 128 x 128 tiles, 4 stages, one CTA per SM (the
 // long-K GEMMs).  BNT = 64: 128 x 64 tiles, 3 stages, two CTAs per SM, so
 // that one CTA's epilogue (the old C tile in and the new one out) overlaps
@@ -142,12 +169,24 @@ __device__ __forceinline__ void dgemm_tile(int M, int N, int K, double alpha, co
 #pragma unroll
     for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
 
+  using CA = TileCopy<TA, BM>;
+  using CB = TileCopy<!TB, BNT>;
+  const bool fullm = m0 + BM <= M, fulln = n0 + BNT <= N;
+  const double *gA = CA::first(A, lda, m0, tid), *gB = CB::first(B, ldb, n0, tid);
+  auto load_a = [&](int stage, int k0) {
+    if (VEC == 2 && fullm && k0 + BK <= K) CA::go(sA + stage * LA::SIZE, gA + (TA ? k0 : k0 * lda), lda, tid);
+    else load_tile<TA, VEC, BM>(sA + stage * LA::SIZE, A, lda, m0, k0, M, K, tid);
+  };
+  auto load_b = [&](int stage, int k0) {
+    if (VEC == 2 && fulln && k0 + BK <= K) CB::go(sB + stage * LB::SIZE, gB + (TB ? k0 * ldb : k0), ldb, tid);
+    else load_tile<!TB, VEC, BNT>(sB + stage * LB::SIZE, B, ldb, n0, k0, N, K, tid);
+  };
   const int KT = (K + BK - 1) / BK;
-#pragma unroll
+#pragma unroll 1
   for (int s = 0; s < STG - 1; s++) {
     if (s < KT) {
-      load_tile<TA, VEC, BM>(sA + s * LA::SIZE, A, lda, m0, s * BK, M, K, tid);
-      load_tile<!TB, VEC, BNT>(sB + s * LB::SIZE, B, ldb, n0, s * BK, N, K, tid);
+      load_a(s, s * BK);
+      load_b(s, s * BK);
     }
     cp_async_commit();
   }
@@ -168,8 +207,7 @@ __device__ __forceinline__ void dgemm_tile(int M, int N, int K, double alpha, co
   // it are issued behind products too, A's and B's behind different k-steps: one
   // burst of both behind the last k-step needs more address registers than
   // there are (255 and spills without alignment; 1501 x 1203 x 999, A
-  // transposed, 193 us, now 159).  8192^3: 31.5 -> 34.7 TFLOP/s (cuBLAS 35.5);
-  // 8192^2 x K with C read back: K = 128 23.4 -> 25.8, 256 27.6 -> 28.7.
+  // transposed, 193 us, now 159).  8192^3: 31.5 -> 34.7 TFLOP/s (cuBLAS 35.5).
   const int fr = lane >> 2, fk = lane & 3;
   double a[2][MI], b[2][4];
   auto fragments = [&](int buf, const double *a_s, const double *b_s, int kk) {
@@ -201,8 +239,8 @@ __device__ __forceinline__ void dgemm_tile(int M, int N, int K, double alpha, co
         for (int j = 0; j < 4; j++) dmma(acc[i][j], a[s & 1][i], b[s & 1][j]);
       if (kt + STG - 1 < KT) {
         const int k0 = (kt + STG - 1) * BK;
-        if (s == 0) load_tile<TA, VEC, BM>(sA + refill * LA::SIZE, A, lda, m0, k0, M, K, tid);
-        if (s == 1) load_tile<!TB, VEC, BNT>(sB + refill * LB::SIZE, B, ldb, n0, k0, N, K, tid);
+        if (s == 0) load_a(refill, k0);
+        if (s == 1) load_b(refill, k0);
       }
     }
     refill = refill + 1 == STG ? 0 : refill + 1;
@@ -216,12 +254,25 @@ __device__ __forceinline__ void dgemm_tile(int M, int N, int K, double alpha, co
   auto ok = [&](int r, int c) {
     return r < M && c < N && !(tri == 1 && r < c) && !(tri == 2 && r > c);
   };
+  // A tile that is stored whole needs no test per element.
+  const bool whole = fullm && fulln && (tri == 0 || (tri == 1 ? m0 >= n0 + BNT - 1 : n0 >= m0 + BM - 1));
   constexpr int CLD = BM + 4;  // staged C: column-major, ld CLD (fits the pipeline buffers)
   static_assert(BNT * CLD <= STG * (Lay<false, BM>::SIZE + Lay<false, BNT>::SIZE), "C tile does not fit");
   double *sC = smem;
   if (beta != 0.0) {
     __syncthreads();  // every warp is done with the pipeline buffers
-    if (VEC == 2 && (uintptr_t)C % 16 == 0 && ldc % 2 == 0) {
+    const bool vec = VEC == 2 && (uintptr_t)C % 16 == 0 && ldc % 2 == 0;
+    if (whole && vec) {
+      constexpr int COLS = THREADS / (BM / 2);
+      const int rr = tid % (BM / 2) * 2, cc = tid / (BM / 2);
+      const double *g = C + m0 + rr + (long)(n0 + cc) * ldc;
+      double *d = sC + rr + cc * CLD;
+#pragma unroll 8
+      for (int i = 0; i < BNT / COLS; i++) {
+        cp_async16(d + i * COLS * CLD, g, true);
+        g += COLS * ldc;
+      }
+    } else if (vec) {
 #pragma unroll 4
       for (int idx = tid; idx < BM * BNT / 2; idx += THREADS) {
         const int rr = idx % (BM / 2) * 2, cc = idx / (BM / 2), r = m0 + rr, c = n0 + cc;
@@ -241,6 +292,23 @@ __device__ __forceinline__ void dgemm_tile(int M, int N, int K, double alpha, co
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
+  }
+  if (whole) {
+    const double *sc = sC + wm + fr + (wn + fk * 2) * CLD;
+    double *g = C + m0 + wm + fr + (long)(n0 + wn + fk * 2) * ldc;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        double *gc = g + (j * 8 + h) * ldc;
+#pragma unroll
+        for (int i = 0; i < MI; i++) {
+          double v = alpha * acc[i][j][h];
+          if (beta != 0.0) v = fma(beta, sc[i * 8 + (j * 8 + h) * CLD], v);
+          gc[i * 8] = v;
+        }
+      }
+    return;
   }
 #pragma unroll
   for (int i = 0; i < MI; i++) {
