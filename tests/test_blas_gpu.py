@@ -213,6 +213,30 @@ def test_dgemm_few_tiles(gpu, ta, tb, m, n, k, pad):
         assert np.array_equal(c[m:], c0[m:])
 
 
+@pytest.mark.parametrize("beta", [0.0, 1.0])
+@pytest.mark.parametrize("m,n,k", [(1280, 1024, 1), (1281, 1087, 40), (1282, 1088, 256), (1408, 1408, 512), (1280, 1024, 514)])
+@pytest.mark.parametrize("pinned", [False, True])
+def test_dgemm_whole_tiles_by_bulk_copy(gpu, m, n, k, beta, pinned):
+    """beta = 0 and 1, whose whole tiles leave by bulk copies that add in L2: on
+    device memory, next to tiles at the edges, and on pinned host memory, which
+    keeps loads and stores.  |C - C_ref| <= (k + 3) u (|A||B| + |beta||C|)
+    componentwise, doubled for the reference's own rounding; the padding rows of
+    C stay as they are."""
+    import torch
+    g = torch.Generator().manual_seed(m + k)
+    ldc = m + 2 + m % 2
+    rnd = lambda *s: torch.rand(*s, generator=g, dtype=torch.float64) * 2 - 1
+    a, b, c0 = rnd(k, m + m % 2), rnd(n, k + k % 2), rnd(n, ldc)
+    c = c0.clone().pin_memory() if pinned else c0.cuda()
+    AB.atlb_dgemm_dev(111, 111, m, n, k, -1.0, a.cuda(), m + m % 2, b.cuda(), k + k % 2, beta, c, ldc)
+    torch.cuda.synchronize()
+    c = c.cpu()
+    ref = beta * c0[:, :m] - b[:, :k] @ a[:, :m]
+    mag = beta * c0[:, :m].abs() + b[:, :k].abs() @ a[:, :m].abs()
+    assert bool(((c[:, :m] - ref).abs() <= 2 * (k + 3) * 2.0 ** -53 * mag).all())
+    assert torch.equal(c[:, m:], c0[:, m:])
+
+
 @pytest.mark.parametrize("uplo", [121, 122])
 @pytest.mark.parametrize("n,k", [(1, 1), (33, 20), (64, 130), (200, 64), (640, 300)])
 def test_dsyrk_few_tiles(gpu, uplo, n, k):
