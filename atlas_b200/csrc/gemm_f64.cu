@@ -133,7 +133,10 @@ template <int BNT> struct TileCfg {
   template <bool TA, bool TB>
   static constexpr int smem_doubles() { return STG * (Lay<TA, BM>::SIZE + Lay<!TB, BNT>::SIZE); }
 };
-constexpr int SMALL_K = 256;  // K up to this uses the 128 x 64 tiles
+// K up to this uses the 128 x 64 tiles: with bulk copies out the narrow tiles stay
+// ahead for longer (8192^2 x 320 with C read back: 31.5 TFLOP/s wide, 33.5 narrow;
+// x 512 33.0 and 34.1, 2048^2 x 512 28.3 and 28.7; at 640 on 2048^2 29.4 and 29.1)
+constexpr int SMALL_K = 256, SMALL_K_BULK = 512;
 constexpr int SMALL_TILE_K = 512;  // K up to this, with few tiles, uses 64 x 64 or 32 x 32 tiles
 // the grouped (batched) GEMM's tile width: its problems are small (K <= 512,
 // M, N from 16), where the narrower tile wastes less on padding and two CTAs
@@ -675,7 +678,7 @@ void launch(int M, int N, int K, double alpha, const double *A, long lda, const 
   // or a cap leaves SMs to another stream.
   const int tiles_n64 = cdiv(M, BM) * cdiv(N, 64);
   const bool finer = tri == 0 && cap == 0 && 27 * cdiv(tiles_n64, nsm) < 50 * cdiv(tiles, nsm);
-  if (K <= SMALL_K || finer) {
+  if (K <= SMALL_K || (VEC == 2 && bulk && K <= SMALL_K_BULK && tiles > nsm) || finer) {
     dgemm_dmma_kernel<TA, TB, VEC, 64><<<tiles_n64, THREADS, smem_s, st>>>(
         M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, tri, bulk, tune(kTuneGemmGroup));
   } else {
