@@ -20,7 +20,7 @@
 #include "chol_blocks.cuh"
 #include "chol_tiles.cuh"
 #include "kernels.h"
-#include "pivot.cuh"
+#include "lu_panel.cuh"
 #include "staging.h"
 #include "../../include/atlas_b200.h"
 
@@ -113,9 +113,7 @@ batched_posv_kernel(const Prob *__restrict__ probs, const int *__restrict__ orde
 // getrs kernels 14.5 + 3.0 ms before (two barriers and a shared-memory rank-1
 // update per column, interchanges and U12 as separate passes, a solve with
 // loads of the factor on its chain), 9.7 ms now for both.
-constexpr int LPW = 16;         // panel width
 constexpr int LU_RHS = 8;       // right-hand sides carried along
-constexpr int LU_LDU = LPW + 4; // U12 copy, U(q, k) at k * LU_LDU + q
 constexpr int DLD = LPW + 1;
 
 template <int NT>  // threads = largest order
@@ -132,141 +130,6 @@ struct LuSmem {
   int piv[NT];                        // ipiv
   int fail;
 };
-
-// step 1.  a[]: this thread's row of the panel (row tid of m, jb <= 16
-// columns); returns its final position.  The row is shifted as columns are
-// finished -- a[0] is always the current column -- so the loop is one small
-// body (unrolled, the sixteen bodies overflow the instruction cache);
-// multipliers, and the U part of a pivot row, go to S.P at the thread's own
-// row, from where the caller takes the finished row.
-template <int NT>
-__device__ __forceinline__ int lu_panel(LuSmem<NT> &S, double (&a)[LPW], int m, int jb, int j0, int *ipiv) {
-  constexpr int NW = NT / 32, LDP = LuSmem<NT>::LDP;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  bool act = tid < m, chosen = false;
-  int pos = tid;
-#pragma unroll 1
-  for (int c = 0; c < jb; c++) {
-    const int b = c & 1;
-    // a zero or NaN entry never wins, except that the row at position c
-    // stands in when there is no other candidate (then: no interchange)
-    unsigned long long key = 0;
-    if (act) key = fabs(a[0]) > 0.0 ? pivot_key(a[0]) : (pos == c ? 1ull : 0ull);
-    const int wl = warp_argmax_lane(key, act ? (unsigned)pos : 0xffffffffu);
-    if (lane == wl) {
-      S.ckey[b][warp] = key;
-      S.cpos[b][warp] = act ? pos : INT_MAX;
-#pragma unroll
-      for (int k = 0; k < LPW; k += 2)
-        *reinterpret_cast<double2 *>(&S.cand[b][warp][k]) = make_double2(a[k], a[k + 1]);
-    }
-    __syncthreads();
-    int w = 0;
-    if (NW > 1) w = warp_argmax_lane(lane < NW ? S.ckey[b][lane] : 0ull, lane < NW ? (unsigned)S.cpos[b][lane] : 0xffffffffu);
-    const int p = S.cpos[b][w];
-    const double *u = S.cand[b][w];
-    const double piv = u[0];
-    if (tid == 0) {
-      ipiv[j0 + c] = j0 + p;
-      S.piv[j0 + c] = j0 + p;
-      if (piv == 0.0 && !S.fail) S.fail = j0 + c + 1;
-    }
-    if (act) {
-      if (pos == p) {  // the pivot row: it keeps its place in a[] from here on
-        act = false;
-        chosen = true;
-        pos = c;
-      } else {
-        if (pos == c) pos = p;
-        const bool nz = piv != 0.0;  // a zero pivot leaves the column unscaled and the row unchanged
-        const double l = !nz ? a[0] : fabs(piv) >= DBL_MIN ? a[0] * (1.0 / piv) : a[0] / piv;
-        S.P[c * LDP + tid] = l;
-        if (nz) {
-#pragma unroll
-          for (int k = 0; k < LPW; k += 2) {
-            const double2 v = *reinterpret_cast<const double2 *>(u + k);
-            if (k > 0) a[k - 1] = fma(-l, v.x, a[k]);
-            a[k] = fma(-l, v.y, a[k + 1]);
-          }
-        } else {
-#pragma unroll
-          for (int k = 1; k < LPW; k++) a[k - 1] = a[k];
-        }
-        a[LPW - 1] = 0.0;
-      }
-    }
-  }
-  if (chosen) {
-#pragma unroll
-    for (int k = 0; k < LPW; k++)
-      if (pos + k < jb) S.P[(pos + k) * LDP + tid] = a[k];
-  }
-  return pos;
-}
-
-// step 3: C (mt x nt, global, ldc) -= P (mt x 16, shared) U (16 x nt,
-// shared); each warp takes 16 x 32 parts (2 x 4 MMA tiles), accumulators
-// started from C, the next part's C in flight meanwhile
-template <int NT>
-__device__ __forceinline__ void lu_update(const LuSmem<NT> &S, int mt, int nt, double *C, long ldc) {
-  constexpr int LDP = LuSmem<NT>::LDP;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const int rb = (mt + 15) / 16, parts = rb * ((nt + 31) / 32);
-  const double *P = S.P + LPW;  // rows below the diagonal block
-  auto load = [&](int s, double (&v)[2][4][2]) {
-    const int r0 = (s % rb) * 16 + g, c0 = (s / rb) * 32 + 2 * t;
-    const bool in0 = r0 < mt, in1 = r0 + 8 < mt;
-    const double *Cp = C + r0 + (long)c0 * ldc;
-#pragma unroll
-    for (int y = 0; y < 4; y++)
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const bool in = s < parts && c0 + 8 * y + e < nt;
-        const double *q = Cp + (8 * y + e) * ldc;
-        v[0][y][e] = in && in0 ? q[0] : 0.0;
-        v[1][y][e] = in && in1 ? q[8] : 0.0;
-      }
-  };
-  double nx[2][4][2];
-  load(warp, nx);
-#pragma unroll 1
-  for (int s = warp; s < parts; s += NT / 32) {
-    const int r0 = (s % rb) * 16 + g, c0 = (s / rb) * 32;
-    const double *Pr = P + r0 + t * LDP, *Ur = S.U + (c0 + g) * LU_LDU + t;
-    double acc[2][4][2];
-#pragma unroll
-    for (int x = 0; x < 2; x++)
-#pragma unroll
-      for (int y = 0; y < 4; y++) {
-        acc[x][y][0] = nx[x][y][0];
-        acc[x][y][1] = nx[x][y][1];
-      }
-    load(s + NT / 32, nx);
-#pragma unroll
-    for (int q = 0; q < LPW; q += 4) {
-      double av[2], bv[4];
-      av[0] = -Pr[q * LDP];          // rows past mt and columns past nt: not stored
-      av[1] = -Pr[q * LDP + 8];
-#pragma unroll
-      for (int y = 0; y < 4; y++) bv[y] = Ur[8 * y * LU_LDU + q];
-#pragma unroll
-      for (int x = 0; x < 2; x++)
-#pragma unroll
-        for (int y = 0; y < 4; y++) cholb::dmma_8x8x4(acc[x][y], av[x], bv[y]);
-    }
-    const bool in0 = r0 < mt, in1 = r0 + 8 < mt;
-    double *Cp = C + r0 + (long)(c0 + 2 * t) * ldc;
-#pragma unroll
-    for (int y = 0; y < 4; y++)
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const bool in = c0 + 8 * y + 2 * t + e < nt;
-        double *q = Cp + (8 * y + e) * ldc;
-        if (in && in0) q[0] = acc[0][y][e];
-        if (in && in1) q[8] = acc[1][y][e];
-      }
-  }
-}
 
 // the factorization of one problem, S.xs (nr right-hand sides, row i of
 // column r at r * NT + i) becoming L^-1 P b; returns the first zero pivot
@@ -289,7 +152,7 @@ __device__ __forceinline__ int lu_factor(const Prob &pr, int nr, LuSmem<NT> &S) 
       S.to[tid] = tid;
     }
     __syncthreads();
-    const int pos = lu_panel<NT>(S, a, m, jb, j, pr.ipiv);
+    const int pos = lu_panel<NT, false>(S, a, m, jb, j);
 #pragma unroll
     for (int k = 0; k < LPW; k++) a[k] = (tid < m && k < jb) ? S.P[k * LDP + tid] : 0.0;
     __syncthreads();
@@ -351,10 +214,11 @@ __device__ __forceinline__ int lu_factor(const Prob &pr, int nr, LuSmem<NT> &S) 
           for (int q = 0; q < LPW; q++) y = fma(-S.P[q * LDP + tid], S.xs[r * NT + j + q], y);
           S.xs[r * NT + j + tid] = y;
         }
-      lu_update<NT>(S, nt, nt, A + (j + jb) + (long)(j + jb) * lda, lda);
+      lu_update<NT, 4>(S, nt, nt, A + (j + jb) + (long)(j + jb) * lda, lda);
     }
     __syncthreads();
   }
+  if (tid < n) pr.ipiv[tid] = S.piv[tid];
   // The interchanges of the columns left of each panel, all at once: `src` is
   // the row whose entry ends in this thread's row, composed from the last panel
   // back; every panel's multipliers are read and written once, in whole rows.

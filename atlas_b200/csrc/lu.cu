@@ -24,7 +24,7 @@
 #include <cooperative_groups.h>
 #include "common.cuh"
 #include "kernels.h"
-#include "pivot.cuh"
+#include "lu_panel.cuh"
 #include "cluster.cuh"
 
 namespace cg = cooperative_groups;
@@ -312,6 +312,8 @@ __device__ __forceinline__ void stage_row(T *stage, const T (&a)[NB], int off) {
 }
 
 constexpr int kMaxPanelCluster = 16;
+// rows up to which one CTA takes an FP64 panel (getf2_cta_kernel has the times)
+constexpr int kCtaPanelRows = 256;
 __device__ int g_panel_timeout = 0;  // set if a panel wait ever gives up (1 s)
 
 template <typename T, int NB>
@@ -563,6 +565,154 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
   panel_u12_solve<T, NB>(MN, ncols, nright, crank * nw + warp, C * nw, A, lda);
 }
 
+// FP64 panels of at most 256 rows: one CTA of a thread per row, two 16-column
+// panels in registers (lu_panel.cuh).  The fused kernel pays per column for the
+// messages between its CTAs and for 32 columns of the pivot row read by every warp;
+// here a column needs one barrier and 16, and the second half of the panel
+// gets the first half's update at once from the MMA unit.
+// An M x 32 panel, fused kernel and this one: M = 128 43.7 and 29.1 us, 256 43.3
+// and 33.2, 384 44.3 and 42.4, 512 44.1 and 46.6 (a column costs more with every
+// warp), hence the limit; order 500 924 -> 820 us.  What is left is the chain
+// of a column: the search in each warp, one lane's stores of the candidate row,
+// the barrier, the search among the warps, the division.  Every row's reciprocal
+// beside the search instead of the winner's behind it was slower (256: 35.8).
+template <int NT>
+struct alignas(16) CtaPanelSmem {
+  static constexpr int LDP = NT + 4;
+  double P[LPW * LDP];
+  double U[2 * LPW * LU_LDU];  // 16 columns; the update's fragments are read for 16
+  double cand[2][NT / 32][LPW];
+  unsigned long long ckey[2][NT / 32];
+  int cpos[2][NT / 32];
+  int from[LPW], to[LPW];  // row whose content ends at q; where row q's content ends
+  int piv[32];
+  int fail, nm;
+  int mfrom[64], mto[64];  // rows that move in the block's other columns
+};
+
+template <int NT>
+__global__ void __launch_bounds__(NT, 1)
+getf2_cta_kernel(int M, int ncols, double *A, long lda, int *__restrict__ ipiv, int roff, int *__restrict__ dinfo,
+                 int nleft, int nright) {
+  using SM = CtaPanelSmem<NT>;
+  constexpr int LDP = SM::LDP, NE = LPW * LPW / NT > 0 ? LPW * LPW / NT : 1;
+  extern __shared__ __align__(16) unsigned char cta_smem[];
+  SM &S = *reinterpret_cast<SM *>(cta_smem);
+  double *stage = reinterpret_cast<double *>(cta_smem + sizeof(SM));  // 64 x (nleft + nright)
+  const int tid = threadIdx.x;
+  if (tid == 0) S.fail = S.nm = 0;
+#pragma unroll 1
+  for (int j = 0; j < ncols; j += LPW) {
+    const int jb = min(LPW, ncols - j), m = M - j, nt = ncols - j - jb;
+    double *R = A + j + (long)(j + jb) * lda;  // the panel's columns right of this half
+    double a[LPW];
+#pragma unroll
+    for (int k = 0; k < LPW; k++) a[k] = (tid < m && k < jb) ? A[j + tid + (long)(j + k) * lda] : 0.0;
+    if (tid < LPW) S.from[tid] = S.to[tid] = tid;
+    __syncthreads();
+    const int pos = lu_panel<NT, true>(S, a, m, jb, j);
+#pragma unroll
+    for (int k = 0; k < LPW; k++) a[k] = (tid < m && k < jb) ? S.P[k * LDP + tid] : 0.0;
+    __syncthreads();
+    if (tid < m) {
+#pragma unroll
+      for (int k = 0; k < LPW; k++) {
+        S.P[k * LDP + pos] = a[k];
+        if (k < jb) A[j + pos + (long)(j + k) * lda] = a[k];
+      }
+      if (pos < LPW) S.from[pos] = tid;
+      if (tid < LPW) S.to[tid] = pos;
+    }
+    __syncthreads();
+    if (nt > 0) {  // jb = 16: the other half's rows interchanged, its top solved, the rest updated
+      double old[NE];
+#pragma unroll
+      for (int x = 0; x < NE; x++) {
+        const int e = tid + x * NT, q = e & (LPW - 1), k = e / LPW;
+        if (k < nt) {
+          old[x] = R[q + (long)k * lda];
+          S.U[k * LU_LDU + q] = R[S.from[q] + (long)k * lda];
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int x = 0; x < NE; x++) {
+        const int e = tid + x * NT, q = e & (LPW - 1), k = e / LPW;
+        if (k < nt && S.to[q] >= LPW) R[S.to[q] + (long)k * lda] = old[x];
+      }
+      if (tid < nt) {
+        double *u = S.U + tid * LU_LDU, x[LPW];  // shifted below: x[0] is the current row
+#pragma unroll
+        for (int q = 0; q < LPW; q++) x[q] = u[q];
+#pragma unroll 1
+        for (int q = 0; q < LPW; q++) {
+          const double v = x[0], *l = S.P + q * LDP + q;
+          u[q] = v;
+#pragma unroll
+          for (int r = 1; r < LPW; r++) x[r - 1] = fma(-l[r], v, x[r]);
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int x = 0; x < NE; x++) {
+        const int e = tid + x * NT, q = e & (LPW - 1), k = e / LPW;
+        if (k < nt) R[q + (long)k * lda] = S.U[k * LU_LDU + q];
+      }
+      lu_update<NT, 2>(S, m - LPW, nt, R + LPW, lda);
+    }
+    __syncthreads();
+  }
+  if (tid < ncols) ipiv[tid] = roff + S.piv[tid];
+  if (tid == 0 && S.fail) atomicMin(dinfo, roff + S.fail);
+  // the row whose content ends in this thread's row, composed from the last
+  // interchange back: first the second half's, for the first half's columns
+  int src = tid;
+  auto compose = [&](int hi, int lo) {
+#pragma unroll 1
+    for (int c = hi - 1; c >= lo; c--) {
+      const int p = S.piv[c];
+      src = src == c ? p : src == p ? c : src;
+    }
+  };
+  if (ncols > LPW) {
+    compose(ncols, LPW);
+    const bool in = tid >= LPW && tid < M;
+    if (in)
+#pragma unroll
+      for (int q = 0; q < LPW; q++) S.P[q * LDP + tid] = A[tid + (long)q * lda];
+    __syncthreads();
+    if (in && src != tid)
+#pragma unroll
+      for (int q = 0; q < LPW; q++) A[tid + (long)q * lda] = S.P[q * LDP + src];
+  }
+  const int nother = nleft + nright;
+  if (nother == 0) return;
+  compose(min(ncols, LPW), 0);
+  if (tid < M && src != tid) {  // at most two rows for each of 32 interchanges
+    const int i = atomicAdd(&S.nm, 1);
+    S.mfrom[i] = src;
+    S.mto[i] = tid;
+  }
+  __syncthreads();
+  const int nm = S.nm, total = nm * nother;
+  auto other = [&](int c) { return (long)(c < nleft ? c - nleft : ncols + c - nleft) * lda; };
+  for (int base = tid; base < total; base += 8 * NT) {
+    double v[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const int g = base + q * NT;
+      if (g < total) v[q] = A[S.mfrom[g % nm] + other(g / nm)];
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      if (base + q * NT < total) stage[base + q * NT] = v[q];
+  }
+  __syncthreads();
+  for (int g = tid; g < total; g += NT) A[S.mto[g % nm] + other(g / nm)] = stage[g];
+  __syncthreads();
+  if (nright > 0 && ncols > 1) panel_u12_solve<double, 32>(ncols, ncols, nright, tid >> 5, NT / 32, A, lda);
+}
+
 // Fallback for panels taller than a cluster can hold: one CTA, global memory.
 template <typename T>
 __global__ void __launch_bounds__(1024)
@@ -718,6 +868,22 @@ template <typename T>
 bool launch_fused_panel(int M, int ncols, T *A, long lda, int *ipiv, int roff, int *dinfo, int nleft,
                         int nright, cudaStream_t st) {
   if (ncols > 32 || nleft + nright > 256) return false;  // the interchange staging holds 64 x 256
+  if constexpr (sizeof(T) == 8) {
+    if (M <= kCtaPanelRows && M >= ncols) {
+      auto go = [&](auto kern, int nt, int bytes, bool &set) {
+        if (!set) {
+          ATLB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes + 64 * 256 * 8));
+          set = true;
+        }
+        kern<<<1, nt, bytes + 64 * 8 * (nleft + nright), st>>>(M, ncols, A, lda, ipiv, roff, dinfo, nleft, nright);
+        ATLB_CUDA_CHECK(cudaGetLastError());
+      };
+      static bool set1 = false, set2 = false;
+      if (M <= 128) go(getf2_cta_kernel<128>, 128, (int)sizeof(CtaPanelSmem<128>), set1);
+      else go(getf2_cta_kernel<256>, 256, (int)sizeof(CtaPanelSmem<256>), set2);
+      return true;
+    }
+  }
   const int most = max_cluster_fused<T>();
   if (cdiv(M, PT) > most) return false;
   // As many CTAs as the cluster takes, as few rows in each: what a column costs

@@ -123,6 +123,31 @@ def test_potrf_vs_oracle(gpu, orc, uplo, n):
     assert np.array_equal(a[:n][other], a0[other])
 
 
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 31, 32, 33, 100])
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 127, 128, 129, 255, 256, 257, 300])
+def test_getrf_panels_of_one_cta(gpu, m, n):
+    """LU of few rows, whose panels one CTA factors: |PA - LU| <= gamma |L||U|
+    componentwise with gamma = min(m, n) u, doubled for the product's own
+    rounding; multipliers of at most 1; a zero column in each half of a panel is
+    reported and the factorization completes."""
+    rng = np.random.default_rng(m * 1000 + n)
+    mn, u = min(m, n), 2.0 ** -53
+    for zero in ((), (mn // 2,), (mn - 1, mn // 3)):
+        a0 = np.asfortranarray(rng.uniform(-1, 1, (m + 1, n)))
+        a0[:, list(zero)] = 0.0
+        a, ipiv = a0.copy(order="F"), np.full(mn, -1, dtype=np.int32)
+        info = AB.clapack_dgetrf(CM, m, n, a, m + 1, ipiv)
+        assert info == (min(zero) + 1 if zero else 0)
+        assert np.array_equal(a[m], a0[m])
+        p = a0[:m].copy()
+        for k in range(mn):
+            assert k <= ipiv[k] < m
+            p[[k, ipiv[k]]] = p[[ipiv[k], k]]
+        low, up = np.tril(a[:m, :mn], -1) + np.eye(m, mn), np.triu(a[:mn])
+        assert np.max(np.abs(low)) <= 1.0
+        assert np.all(np.abs(p - low @ up) <= 2 * (mn + 1) * u * (np.abs(low) @ np.abs(up)))
+
+
 @pytest.mark.parametrize("nrhs", [1, 2, 3, 4, 5, 8, 9, 16, 17, 32])
 @pytest.mark.parametrize("n", [1, 127, 128, 129, 256, 257, 300, 520])
 def test_few_rhs_solves_at_block_edges(gpu, n, nrhs):
