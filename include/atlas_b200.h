@@ -300,8 +300,8 @@ int atlb_dgemm_ozaki(int TransA, int TransB, int M, int N, int K, double alpha, 
 /* Batched, uneven-size problems (no counterpart in the reference).  All
  * pointers inside the arrays are DEVICE pointers; the arrays themselves are
  * host arrays of `count` entries.  Each batch runs as one persistent launch
- * whose CTAs take work (problems, or GEMM tiles) largest first from an atomic
- * counter.  Column-major; returns 0 or -(bad argument).
+ * (posv, gesv: one per size bucket) whose CTAs take work (problems, or GEMM
+ * tiles) largest first from an atomic counter.  Column-major; returns 0 or -(bad argument).
  *   atlb_dgemm_batched_dev: C[i] = alpha*op(A[i])*op(B[i]) + beta*C[i]; returns
  *     after the launch is enqueued (asynchronous on the library stream).
  *   atlb_dposv_batched: Cholesky (lower triangle) + solve of nrhs[i] right-hand
