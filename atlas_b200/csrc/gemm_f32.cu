@@ -1,6 +1,6 @@
 // FP32 GEMM on the FP32 FMA pipes (cblas_sgemm and the FP32-exact factor
 // mode of the mixed-precision solvers).  128x128x16 CTA tile, 128 threads,
-// 8x16 outputs per thread; op(A) and op(B) tiles are staged in shared memory
+// 8x16 outputs per thread (64x64 and 4x8 for few tiles); op(A) and op(B) tiles are staged in shared memory
 // k-major (m / n contiguous) by a 3-stage cp.async pipeline, whatever their
 // global layout, so the inner loop reads 128-bit vectors.  An output of few
 // tiles with a long K (the Cholesky's diagonal-block updates) is split along
@@ -8,26 +8,29 @@
 // one pass sums the slices into C.
 // Reference semantics: src/blas/reference/level3/ATL_srefgemm.c.
 #include <cstdint>
+#include <type_traits>
 #include "common.cuh"
 #include "kernels.h"
 
 namespace atlb {
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 16, THREADS = 128, STAGES = 3, LDS = BM + 4;
-constexpr int SMEM = 2 * STAGES * BK * LDS * (int)sizeof(float);
+constexpr int BT = 128, BK = 16, THREADS = 128, STAGES = 3;
+template <int T> constexpr int kLds = T + 4;
+template <int T> constexpr int kSmem = 2 * STAGES * BK * kLds<T> * (int)sizeof(float);
 
-// One 128 x 16 operand tile into shared memory, k-major (o contiguous).
+// One T x 16 operand tile into shared memory, k-major (o contiguous).
 // Operand element (o, k): TRANS_O ? X[k + o*ld] : X[o + k*ld].  VEC: o is
 // contiguous in global memory and every column starts on 16 bytes, so whole
 // 16-byte pieces are copied; otherwise 4 bytes at a time.
-template <bool TRANS_O, bool VEC>
+template <int T, bool TRANS_O, bool VEC>
 __device__ __forceinline__ void load_tile(float *s, const float *X, long ld, int o0, int k0,
                                           int O, int K, int tid) {
+  constexpr int LDS = kLds<T>;
   if (VEC && !TRANS_O) {
 #pragma unroll
-    for (int i = 0; i < BM * BK / 4 / THREADS; i++) {
-      const int c = tid + THREADS * i, o = (c & 31) * 4, k = c >> 5;
+    for (int i = 0; i < T * BK / 4 / THREADS; i++) {
+      const int c = tid + THREADS * i, o = c % (T / 4) * 4, k = c / (T / 4);
       const int go = o0 + o, gk = k0 + k;
       const float *g = X + go + (long)gk * ld;
       float *d = s + k * LDS + o;
@@ -42,10 +45,10 @@ __device__ __forceinline__ void load_tile(float *s, const float *X, long ld, int
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < BM * BK / THREADS; i++) {
+    for (int i = 0; i < T * BK / THREADS; i++) {
       const int c = tid + THREADS * i;
       int o, k;
-      if (!TRANS_O) { o = c & 127; k = c >> 7; }   // o fastest: coalesced along o
+      if (!TRANS_O) { o = c % T; k = c / T; }   // o fastest: coalesced along o
       else { k = c & 15; o = c >> 4; }             // k fastest: coalesced along k
       const int go = o0 + o, gk = k0 + k;
       const bool p = go < O && gk < K;
@@ -73,7 +76,13 @@ __device__ __forceinline__ unsigned long long swap2(unsigned long long x) {
 // of columns, then the swapped pair of rows times the same, two moves a pair of
 // rows.  4096^3: 3.17 ms with 8 x 8 outputs and single products, 2.76 ms
 // now.
-template <bool TA, bool TB, bool VA, bool VB>
+//
+// Outputs of fewer 128 x 128 tiles than SMs take 64 x 64 ones (T = 64, 4 x 8 outputs a
+// thread): four times the CTAs, and four warps' latency per tile a quarter as
+// long.  With C read back, 128 x 128 tiles of 8 x 8 outputs and these: 128^3 23.1 and
+// 9.0 us, 2000 x 128 x 128 26.9 and 10.7, 1000^3 140 and 75, 1500 x 1200 x 900 (120
+// tiles) 128 and 122.
+template <int T, bool TA, bool TB, bool VA, bool VB>
 __global__ void __launch_bounds__(THREADS, 2)
 sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A, long lda,
                   const float *__restrict__ B, long ldb, float beta, float *__restrict__ C,
@@ -88,6 +97,7 @@ sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A,
     alpha = 1.f;
     beta = 0.f;
   }
+  constexpr int BM = T, BN = T, LDS = kLds<T>, H = T / 64;  // a warp's part: 32 H x 32 H
   extern __shared__ __align__(16) float sgemm_smem[];
   float *sA = sgemm_smem, *sB = sgemm_smem + STAGES * BK * LDS;
   const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
@@ -99,23 +109,23 @@ sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A,
   if (tri == 1 && m0 + BM - 1 < n0) return;
   if (tri == 2 && m0 > n0 + BN - 1) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // this thread's rows rm + 32 h + 0..3 (h < 2), columns cn + 16 q + 0..3 (q < 4)
-  const int rm = (warp & 1) * 64 + (lane & 7) * 4, cn = (warp >> 1) * 64 + (lane >> 3) * 4;
+  // this thread's rows rm + 32 h + 0..3 (h < H), columns cn + 16 q + 0..3 (q < 2 H)
+  const int rm = (warp & 1) * 32 * H + (lane & 7) * 4, cn = (warp >> 1) * 32 * H + (lane >> 3) * 4;
 
   // row pair i x column pair j: acc[0] holds (row 0, col 0) and (row 1, col 1),
   // acc[1] (row 1, col 0) and (row 0, col 1)
-  unsigned long long acc[2][4][8];
+  unsigned long long acc[2][2 * H][4 * H];
 #pragma unroll
-  for (int i = 0; i < 4; i++)
+  for (int i = 0; i < 2 * H; i++)
 #pragma unroll
-    for (int j = 0; j < 8; j++) acc[0][i][j] = acc[1][i][j] = 0ull;
+    for (int j = 0; j < 4 * H; j++) acc[0][i][j] = acc[1][i][j] = 0ull;
 
   const int KT = (K + BK - 1) / BK;
 #pragma unroll
   for (int s = 0; s < STAGES - 1; s++) {
     if (s < KT) {
-      load_tile<TA, VA>(sA + s * BK * LDS, A, lda, m0, s * BK, M, K, tid);
-      load_tile<!TB, VB>(sB + s * BK * LDS, B, ldb, n0, s * BK, N, K, tid);
+      load_tile<T, TA, VA>(sA + s * BK * LDS, A, lda, m0, s * BK, M, K, tid);
+      load_tile<T, !TB, VB>(sB + s * BK * LDS, B, ldb, n0, s * BK, N, K, tid);
     }
     cp_async_commit();
   }
@@ -125,29 +135,32 @@ sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A,
     {
       const int nk = kt + STAGES - 1;
       if (nk < KT) {
-        load_tile<TA, VA>(sA + nk % STAGES * BK * LDS, A, lda, m0, nk * BK, M, K, tid);
-        load_tile<!TB, VB>(sB + nk % STAGES * BK * LDS, B, ldb, n0, nk * BK, N, K, tid);
+        load_tile<T, TA, VA>(sA + nk % STAGES * BK * LDS, A, lda, m0, nk * BK, M, K, tid);
+        load_tile<T, !TB, VB>(sB + nk % STAGES * BK * LDS, B, ldb, n0, nk * BK, N, K, tid);
       }
       cp_async_commit();
     }
     const float *as = sA + kt % STAGES * BK * LDS + rm, *bs = sB + kt % STAGES * BK * LDS + cn;
 #pragma unroll
     for (int k = 0; k < BK; k++) {
-      const ulonglong2 a0 = *reinterpret_cast<const ulonglong2 *>(as + k * LDS);
-      const ulonglong2 a1 = *reinterpret_cast<const ulonglong2 *>(as + k * LDS + 32);
-      const unsigned long long a[4] = {a0.x, a0.y, a1.x, a1.y};
-      unsigned long long b[8], x[4];
+      unsigned long long a[2 * H], b[4 * H], x[2 * H];
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
+      for (int h = 0; h < H; h++) {
+        const ulonglong2 ah = *reinterpret_cast<const ulonglong2 *>(as + k * LDS + 32 * h);
+        a[2 * h] = ah.x;
+        a[2 * h + 1] = ah.y;
+      }
+#pragma unroll
+      for (int q = 0; q < 2 * H; q++) {
         const ulonglong2 bq = *reinterpret_cast<const ulonglong2 *>(bs + k * LDS + 16 * q);
         b[2 * q] = bq.x;
         b[2 * q + 1] = bq.y;
         x[q] = swap2(a[q]);
       }
 #pragma unroll
-      for (int j = 0; j < 8; j++)
+      for (int j = 0; j < 4 * H; j++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < 2 * H; i++) {
           fma2(acc[0][i][j], a[i], b[j]);
           fma2(acc[1][i][j], x[i], b[j]);
         }
@@ -156,7 +169,7 @@ sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A,
   cp_async_wait<0>();
   // epilogue: a row quad of one column is contiguous in C.  Old C values are
   // loaded eight quads at a time before any of their stores, so the loads overlap.
-  auto val = [&](int h, int j, int e) {  // row rm + 32 h + e, column j of this thread's sixteen
+  auto val = [&](int h, int j, int e) {  // row rm + 32 h + e, column j of this thread's 8 H
     // the half that holds row e's product: row 0 leads in acc[0], row 1 in acc[1]
     const int s = (e ^ j) & 1, half = s ? 1 - (e & 1) : e & 1;
     return __uint_as_float((unsigned)(acc[s][2 * h + (e >> 1)][j >> 1] >> (32 * half)));
@@ -164,12 +177,12 @@ sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A,
   const bool vec = tri == 0 && ((uintptr_t)C % 16 == 0) && (ldc % 4 == 0) && m0 + BM <= M && n0 + BN <= N;
   if (vec) {
 #pragma unroll
-    for (int jh = 0; jh < 16; jh += 4) {  // four rounds of 8 float4 loads, then their stores
-      float4 cv[4][2];
+    for (int jh = 0; jh < 8 * H; jh += 4) {  // rounds of 4 H float4 loads, then their stores
+      float4 cv[4][H];
 #pragma unroll
       for (int jj = 0; jj < 4; jj++)
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
+        for (int h = 0; h < H; h++) {
           const int c = n0 + cn + 4 * jh + jj, r = m0 + rm + 32 * h;
           cv[jj][h] = beta != 0.f ? *reinterpret_cast<const float4 *>(C + r + (long)c * ldc)
                                   : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -177,7 +190,7 @@ sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A,
 #pragma unroll
       for (int jj = 0; jj < 4; jj++)
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
+        for (int h = 0; h < H; h++) {
           const int j = jh + jj, c = n0 + cn + 4 * jh + jj, r = m0 + rm + 32 * h;
           float4 o;
           o.x = alpha * val(h, j, 0);
@@ -196,17 +209,17 @@ sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A,
     return;
   }
 #pragma unroll
-  for (int j = 0; j < 16; j++) {
+  for (int j = 0; j < 8 * H; j++) {
     const int c = n0 + cn + 16 * (j >> 2) + (j & 3);
-    float cv[8];
+    float cv[4 * H];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
+    for (int i = 0; i < 4 * H; i++) {
       const int r = m0 + rm + (i < 4 ? i : 32 + i - 4);
       const bool ok = r < M && c < N && !(tri == 1 && r < c) && !(tri == 2 && r > c);
       cv[i] = (ok && beta != 0.f) ? C[r + (long)c * ldc] : 0.f;
     }
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
+    for (int i = 0; i < 4 * H; i++) {
       const int r = m0 + rm + (i < 4 ? i : 32 + i - 4);
       if (r >= M || c >= N) continue;
       if (tri == 1 && r < c) continue;
@@ -259,7 +272,7 @@ void sgemm_dev(int ta, int tb, int M, int N, int K, float alpha, const float *A,
     ATLB_CUDA_CHECK(cudaGetLastError());
     return;
   }
-  int tiles = cdiv(M, BM) * cdiv(N, BN);
+  const int tiles = cdiv(M, BT) * cdiv(N, BT);
   const bool tA = ta != kNoTrans, tB = tb != kNoTrans;
   // few output tiles and a long K: split K so that about two CTAs per SM run
   int S = 1, kc = K;
@@ -271,32 +284,37 @@ void sgemm_dev(int ta, int tb, int M, int N, int K, float alpha, const float *A,
     if (S > 1) W = (float *)scratch(kSlotGemmSplit, sizeof(float) * (size_t)S * M * N);
     else kc = K;
   }
-  const dim3 grid(tiles, S);
   // 16-byte copies need the outer index contiguous and 16-byte aligned columns
   const bool va = !tA && (uintptr_t)A % 16 == 0 && lda % 4 == 0, vb = tB && (uintptr_t)B % 16 == 0 && ldb % 4 == 0;
-  auto go = [&](auto kern, bool &configured) {
-    if (!configured) {
-      ATLB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-      ATLB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-      configured = true;
+  auto with = [&](auto tile) {
+    constexpr int T = decltype(tile)::value;
+    auto go = [&](auto kern, bool &configured) {
+      if (!configured) {
+        ATLB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem<T>));
+        ATLB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+        configured = true;
+      }
+      kern<<<dim3(cdiv(M, T) * cdiv(N, T), S), THREADS, kSmem<T>, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc,
+                                                                         tri, kc, W);
+    };
+    static bool set[9] = {};
+    if (!tA && !tB) {
+      if (va) go(sgemm_simt_kernel<T, false, false, true, false>, set[0]);
+      else go(sgemm_simt_kernel<T, false, false, false, false>, set[1]);
+    } else if (!tA && tB) {
+      if (va && vb) go(sgemm_simt_kernel<T, false, true, true, true>, set[2]);
+      else if (va) go(sgemm_simt_kernel<T, false, true, true, false>, set[3]);
+      else if (vb) go(sgemm_simt_kernel<T, false, true, false, true>, set[4]);
+      else go(sgemm_simt_kernel<T, false, true, false, false>, set[5]);
+    } else if (tA && !tB) {
+      go(sgemm_simt_kernel<T, true, false, false, false>, set[6]);
+    } else {
+      if (vb) go(sgemm_simt_kernel<T, true, true, false, true>, set[7]);
+      else go(sgemm_simt_kernel<T, true, true, false, false>, set[8]);
     }
-    kern<<<grid, THREADS, SMEM, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, tri, kc, W);
   };
-  static bool set[9] = {};
-  if (!tA && !tB) {
-    if (va) go(sgemm_simt_kernel<false, false, true, false>, set[0]);
-    else go(sgemm_simt_kernel<false, false, false, false>, set[1]);
-  } else if (!tA && tB) {
-    if (va && vb) go(sgemm_simt_kernel<false, true, true, true>, set[2]);
-    else if (va) go(sgemm_simt_kernel<false, true, true, false>, set[3]);
-    else if (vb) go(sgemm_simt_kernel<false, true, false, true>, set[4]);
-    else go(sgemm_simt_kernel<false, true, false, false>, set[5]);
-  } else if (tA && !tB) {
-    go(sgemm_simt_kernel<true, false, false, false>, set[6]);
-  } else {
-    if (vb) go(sgemm_simt_kernel<true, true, false, true>, set[7]);
-    else go(sgemm_simt_kernel<true, true, false, false>, set[8]);
-  }
+  if (S == 1 && tiles < num_sms()) with(std::integral_constant<int, 64>{});
+  else with(std::integral_constant<int, BT>{});
   ATLB_CUDA_CHECK(cudaGetLastError());
   if (S > 1) {
     const long total = (long)M * N;

@@ -237,6 +237,29 @@ def test_dgemm_whole_tiles_by_bulk_copy(gpu, m, n, k, beta, pinned):
     assert torch.equal(c[:, m:], c0[:, m:])
 
 
+@pytest.mark.parametrize("ta,tb", [(111, 111), (111, 112), (112, 111), (112, 112)])
+@pytest.mark.parametrize("m,n,k,pad", [(1, 1, 1, 0), (63, 65, 17, 1), (64, 64, 16, 0), (65, 132, 33, 3), (128, 256, 128, 0),
+                                       (500, 708, 300, 0), (1500, 1200, 40, 0), (1664, 1537, 20, 1)])
+def test_sgemm_few_tiles(gpu, ta, tb, m, n, k, pad):
+    """64 x 64 tiles (fewer 128 x 128 tiles than SMs) and the first size beyond:
+    sizes around the tiles, aligned and unaligned columns; |C - C_ref| <=
+    (k + 3) u (|alpha||A||B| + |beta||C|) componentwise with FP32's u, against
+    FP64."""
+    rng = np.random.default_rng(m + n + k)
+    mat = lambda r, c: np.asfortranarray(rng.uniform(-1, 1, (r + pad, c)).astype(np.float32))
+    a, b = mat(*((m, k) if ta == 111 else (k, m))), mat(*((k, n) if tb == 111 else (n, k)))
+    c0 = mat(m, n)
+    opa = (a[:m] if ta == 111 else a[:k].T).astype(np.float64)
+    opb = (b[:k] if tb == 111 else b[:n].T).astype(np.float64)
+    for beta in (0.0, -0.5):
+        c = c0.copy(order="F")
+        AB.cblas_sgemm(102, ta, tb, m, n, k, 1.5, a, a.shape[0], b, b.shape[0], beta, c, c.shape[0])
+        ref = 1.5 * (opa @ opb) + beta * c0[:m]
+        mag = 1.5 * (np.abs(opa) @ np.abs(opb)) + abs(beta) * np.abs(c0[:m])
+        assert np.all(np.abs(c[:m] - ref) <= (k + 3) * 2.0 ** -24 * mag)
+        assert np.array_equal(c[m:], c0[m:])
+
+
 @pytest.mark.parametrize("uplo", [121, 122])
 @pytest.mark.parametrize("n,k", [(1, 1), (33, 20), (64, 130), (200, 64), (640, 300)])
 def test_dsyrk_few_tiles(gpu, uplo, n, k):
