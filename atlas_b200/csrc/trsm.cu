@@ -875,22 +875,27 @@ namespace {
 // the U12 = L11^-1 A12 step of the blocked LU in ONE launch (the recursive
 // trsm_dev issues a TRSM/GEMM cascade of ~8 kernels for it).
 //
-// FP64, on the tensor cores.  It stands on the factorization's critical chain
-// (the look-ahead block's U12), so what counts is the latency of one CTA: all
-// diagonal 32 x 32 tiles are inverted at once, a warp each (one lane per
-// column, the column shifted through registers), and block row ib is then
-//   X_ib = inv(L_ib,ib) (B_ib - sum_{kt < ib} L_ib,kt X_kt),
-// two runs of MMAs with the next block row of L on its way to shared memory
-// (for m <= 192, where two fit).  CTAs of 32 columns, or of 8 with the k range
-// split between two halves of the warps when the columns are few.  The forward
-// substitution by shuffles that this replaces took 47 us at m = 192; this takes
-// 20 us (192 columns) and 33 us (up to 8000).
+// FP64.  It stands on the factorization's critical chain (the look-ahead
+// block's U12), so what counts is the latency of one CTA.  Block row ib is
+//   X_ib = L_ib,ib^-1 (B_ib - sum_{kt < ib} L_ib,kt X_kt):
+// the sum in one run of MMAs on the tensor cores, with the next block row of L
+// on its way to shared memory (for m <= 192, where two fit), then forward
+// substitution with the 32 x 32 diagonal tile, a lane per row, the solved
+// entries passed by shuffle.  Substitution and not a product with the inverted
+// tile: partial pivoting bounds the multipliers by one, the tile's inverse only by
+// 2^30, and |PA - LU| would grow with it (multipliers of -0.9: 4e4 times the
+// bound of substitution).  CTAs of 32 columns, four a warp, or of 8 when the
+// columns are few: one a warp, the sum's k range split between two halves of the
+// warps, and four entries passed at a time, whose own 4 x 4 corner every lane
+// solves (a shuffle for four rows on the chain instead of one for each).
+// At m = 192: 18.7 us (192 columns), 35.0 us (up to 8000); by products with the
+// inverted tiles 20.1 and 33.7, by substitution alone, shuffles for every entry, 47.
 constexpr int LLU_MAX = 256, LLU_LD = 36;  // 4 (mod 16): the MMA's fragments fall in distinct banks
 constexpr int LLU_TILE = 32 * LLU_LD;      // a 32 x 32 tile, (r, k) at k * LLU_LD + r
 
 constexpr int llu_smem(int m, int ncol) {
   const int nblk = (m + 31) / 32, nbuf = m <= 192 ? 2 : 1;
-  return 8 * (ncol * (32 * nblk + 4) + nblk * LLU_TILE + 64 + nbuf * (nblk - 1) * LLU_TILE + 256);
+  return 8 * (ncol * (32 * nblk + 4) + nblk * LLU_TILE + nbuf * (nblk - 1) * LLU_TILE + 256);
 }
 
 template <int NCOL>
@@ -899,8 +904,8 @@ trsm_llu_mma_kernel(int m, int n, const double *__restrict__ L, long lda, double
   extern __shared__ __align__(16) unsigned char llu_smem_raw[];
   const int nblk = (m + 31) / 32, LDX = 32 * nblk + 4, nbuf = m <= 192 ? 2 : 1;
   double *sX = reinterpret_cast<double *>(llu_smem_raw);  // [NCOL][LDX]: B, then X
-  double *sD = sX + NCOL * LDX;                           // the diagonal tiles, then their inverses
-  double *sL = sD + nblk * LLU_TILE + 64;                 // block rows of L, k-major
+  double *sD = sX + NCOL * LDX;                           // the diagonal tiles
+  double *sL = sD + nblk * LLU_TILE;                      // block rows of L, k-major
   double *sP = sL + nbuf * (nblk - 1) * LLU_TILE;         // the second half's sums (NCOL = 8)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int c0 = blockIdx.x * NCOL, nc = min(NCOL, n - c0);
@@ -928,22 +933,7 @@ trsm_llu_mma_kernel(int m, int n, const double *__restrict__ L, long lda, double
   fetch_row(1);
   cp_async_wait<1>();
   __syncthreads();
-  if (warp < nblk) {  // lane j: column j of the inverse, by forward substitution
-    double *D = sD + warp * LLU_TILE;
-    double x[32];
-#pragma unroll
-    for (int r = 0; r < 32; r++) x[r] = r == lane ? 1.0 : 0.0;
-#pragma unroll 1
-    for (int q = 0; q < 32; q++) {
-      const double v = x[0], *l = D + q * LLU_LD + q;  // column q of L is not needed after this step
-#pragma unroll
-      for (int r = 1; r < 32; r++) x[r - 1] = fma(-l[r], v, x[r]);  // past the tile: values nobody uses
-      __syncwarp();
-      if (lane <= q) D[lane * LLU_LD + q] = v;
-      __syncwarp();
-    }
-  }
-  constexpr int NH = NCOL == 8 ? 1 : NCOL / 16;  // 8-column groups of a warp
+  constexpr int NH = NCOL == 8 ? 1 : NCOL / 16;  // 8-column groups of a warp in the sum
   const int rt = 8 * (warp & 3), half = warp >> 2, n0 = NCOL == 8 ? 0 : half * 8 * NH;
   auto mma = [&](const double *T, const double *X, int k0, int k1, double (&acc)[NH][2]) {
     const double *a = T + t * LLU_LD + rt + g, *x = X + (n0 + g) * LDX + t;
@@ -955,9 +945,9 @@ trsm_llu_mma_kernel(int m, int n, const double *__restrict__ L, long lda, double
     }
   };
   for (int ib = 0; ib < nblk; ib++) {
-    double acc[NH][2];
-    double *Xr = sX + 32 * ib + rt + g;  // this warp's rows of the block
     if (ib > 0) {
+      double acc[NH][2];
+      double *Xr = sX + 32 * ib + rt + g;  // this warp's rows of the block
       cp_async_wait<0>();
       __syncthreads();
       if (nbuf == 2) fetch_row(ib + 1);
@@ -981,21 +971,35 @@ trsm_llu_mma_kernel(int m, int n, const double *__restrict__ L, long lda, double
 #pragma unroll
           for (int e = 0; e < 2; e++) Xr[(n0 + 8 * h + 2 * t + e) * LDX] -= acc[h][e];
       }
-      if (nbuf == 1) {
-        __syncthreads();
-        fetch_row(ib + 1);
+      __syncthreads();
+      if (nbuf == 1) fetch_row(ib + 1);
+    }
+    // forward substitution: this lane's row of the warp's columns
+    constexpr int NC = NCOL / 8, G = NCOL == 8 ? 4 : 1;
+    const double *D = sD + ib * LLU_TILE;
+    double x[NC], *Xs = sX + NC * warp * LDX + 32 * ib + lane;
+#pragma unroll
+    for (int c = 0; c < NC; c++) x[c] = Xs[c * LDX];
+#pragma unroll
+    for (int k = 0; k < 32; k += G) {
+      double l[G];
+#pragma unroll
+      for (int u = 0; u < G; u++) l[u] = D[(k + u) * LLU_LD + lane];
+#pragma unroll
+      for (int c = 0; c < NC; c++) {
+        double xs[G];
+#pragma unroll
+        for (int u = 0; u < G; u++) xs[u] = __shfl_sync(0xffffffffu, x[c], k + u);
+#pragma unroll
+        for (int u = 0; u < G; u++) {
+#pragma unroll
+          for (int v = 0; v < u; v++) xs[u] = fma(-D[(k + v) * LLU_LD + k + u], xs[v], xs[u]);
+          if (lane > k + u) x[c] = fma(-l[u], xs[u], x[c]);
+        }
       }
     }
-    __syncthreads();
 #pragma unroll
-    for (int h = 0; h < NH; h++) acc[h][0] = acc[h][1] = 0.0;
-    mma(sD + ib * LLU_TILE, sX + 32 * ib, 0, rt + 8, acc);  // the inverse is lower triangular
-    __syncthreads();
-    if (NCOL > 8 || !half)
-#pragma unroll
-      for (int h = 0; h < NH; h++)
-#pragma unroll
-        for (int e = 0; e < 2; e++) Xr[(n0 + 8 * h + 2 * t + e) * LDX] = acc[h][e];
+    for (int c = 0; c < NC; c++) Xs[c * LDX] = x[c];
   }
   __syncthreads();
   for (int e = tid; e < NCOL * 32 * nblk; e += 256) {

@@ -148,6 +148,36 @@ def test_getrf_panels_of_one_cta(gpu, m, n):
         assert np.all(np.abs(p - low @ up) <= 2 * (mn + 1) * u * (np.abs(low) @ np.abs(up)))
 
 
+@pytest.mark.parametrize("m,n,nb", [(193, 193, 192), (300, 300, 192), (500, 500, 192), (400, 1100, 192),
+                                    (250, 1000, 64), (500, 500, 256), (300, 1000, 256)])
+def test_getrf_of_ill_conditioned_multipliers(gpu, m, n, nb):
+    """A = L U with every multiplier the same: the diagonal tiles of L11 are then
+    far worse conditioned than the matrix, and |PA - LU| <= gamma |L||U| has to
+    hold all the same, through the U12 solve between block columns of nb.  gamma =
+    (m + 2) u (Higham, theorem 9.3, with multipliers by the reciprocal pivot) and m u
+    for the check's own product."""
+    rng = np.random.default_rng(m + n)
+    u = 2.0 ** -53
+    old = AB.atlb_tune_get("getrf_nb")
+    try:
+        assert AB.atlb_tune_set("getrf_nb", nb) == nb
+        for mult in (-0.5, -0.9, -1.0):
+            low = np.eye(m) + mult * np.tril(np.ones((m, m)), -1)
+            up = np.triu(rng.uniform(-1, 1, (m, n)))
+            up[np.arange(m), np.arange(m)] = 1.0
+            a0 = np.asfortranarray(low @ up)
+            a = a0.copy(order="F")
+            ipiv, info = _getrf_gpu(a, m, n)
+            assert info == 0
+            for k in range(m):
+                a0[[k, ipiv[k]]] = a0[[ipiv[k], k]]
+            low, up = np.tril(a[:, :m], -1) + np.eye(m), np.triu(a)
+            assert np.max(np.abs(low)) <= 1.0
+            assert np.all(np.abs(a0 - low @ up) <= 2 * (m + 1) * u * (np.abs(low) @ np.abs(up))), mult
+    finally:
+        AB.atlb_tune_set("getrf_nb", old)
+
+
 @pytest.mark.parametrize("nrhs", [1, 2, 3, 4, 5, 8, 9, 16, 17, 32])
 @pytest.mark.parametrize("n", [1, 127, 128, 129, 256, 257, 300, 520])
 def test_few_rhs_solves_at_block_edges(gpu, n, nrhs):
