@@ -276,7 +276,7 @@ __device__ __forceinline__ void lu_solve(const Prob &pr, int nr, LuSmem<NT> &S) 
       const int c = lane & 15;
       double v = c < jb ? S.xs[r * NT + j + c] : 0.0;
       const double *d = S.D[s & 1] + c;  // D(c, q) at q * DLD + c
-      const double ri = UPPER && c < jb ? 1.0 / d[c * DLD] : 1.0;
+      const double piv = UPPER && c < jb ? d[c * DLD] : 1.0;
       int q = UPPER ? jb - 1 : 0;
       double dn = d[q * DLD];
 #pragma unroll 1
@@ -284,7 +284,7 @@ __device__ __forceinline__ void lu_solve(const Prob &pr, int nr, LuSmem<NT> &S) 
         const double dq = dn;
         const int qn = UPPER ? max(q - 1, 0) : min(q + 1, LPW - 1);
         dn = d[qn * DLD];  // one step ahead of the chain
-        if (UPPER && c == q) v *= ri;
+        if (UPPER && c == q) v /= piv;  // a subnormal pivot's reciprocal would be infinite
         const double xq = __shfl_sync(0xffffffffu, v, q);
         if (UPPER ? c < q : c > q) v = fma(-dq, xq, v);
         q = qn;

@@ -213,6 +213,32 @@ def test_batched_gesv_singular(gpu):
     assert np.all(np.isfinite(As[0].cpu().numpy()))
 
 
+@pytest.mark.parametrize("nrhs", [1, 10])
+def test_batched_gesv_divides_by_its_pivots(gpu, nrhs):
+    """Diagonal systems, subnormal pivots among them, whose reciprocals are
+    infinite: every solution is the one correctly rounded quotient, zero where the
+    right-hand side is zero."""
+    import torch
+    rng = np.random.default_rng(nrhs)
+    ns = [1, 5, 17, 40, 64, 100, 129, 256]
+    As, Bs, Ps, want = [], [], [], []
+    for n in ns:
+        d = rng.uniform(-2, 2, n)
+        d[::3] = rng.integers(1, 9, d[::3].size) * 2.0 ** -1070
+        x = rng.integers(-3, 4, (nrhs, n)).astype(np.float64)
+        b = np.where(np.abs(d) < 1e-300, x * d, x)
+        want.append(b / d)
+        As.append(torch.tensor(np.diag(d), device="cuda"))
+        Bs.append(torch.tensor(b, device="cuda"))
+        Ps.append(torch.zeros(n, dtype=torch.int32, device="cuda"))
+    info = np.full(len(ns), -1, dtype=np.int32)
+    assert AB.atlb_dgesv_batched(len(ns), _int_array(ns), _ptr_array(As), _int_array(ns), _ptr_array(Ps),
+                                 _ptr_array(Bs), _int_array(ns), _int_array([nrhs] * len(ns)), info) == 0
+    assert np.all(info == 0)
+    for b, w in zip(Bs, want):
+        np.testing.assert_array_equal(b.cpu().numpy(), w)
+
+
 def test_batched_dgemm_uneven(gpu, orc):
     import torch
     rng = np.random.default_rng(2)
