@@ -162,7 +162,7 @@ void potrf_dev(int uplo, int N, T *A, long lda, int *dinfo, cudaStream_t st, Sge
       (unsigned long long)uplo,
       (unsigned long long)N, (unsigned long long)lda, (unsigned long long)(uintptr_t)A,
       (unsigned long long)(uintptr_t)dinfo, (unsigned long long)(uintptr_t)gemm,
-      (unsigned long long)(uintptr_t)st};
+      (unsigned long long)(uintptr_t)st, (unsigned long long)(sizeof(T) == 8 && own_memory(A))};
   run_graph(key, st, [&]() {
     set_info_kernel_launch(dinfo, st);
     const bool up = uplo == kUpper;

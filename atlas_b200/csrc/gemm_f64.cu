@@ -584,9 +584,12 @@ int splitk_count(int tiles, int K, int nsm) {
   return 1;
 }
 
+}  // namespace
+
 // Memory of the current device: the bulk copies' additions take place in its L2.
 // Host, managed and other devices' memory keeps the loads and stores.  (0.3 us on
-// the host, and no state: an address says nothing about the next call's.)
+// the host, and no state: an address says nothing about the next call's, so a
+// graph of launches that write a caller's matrix has the answer in its key.)
 bool own_memory(const void *p) {
   cudaPointerAttributes a;
   int dev = -1;
@@ -596,6 +599,8 @@ bool own_memory(const void *p) {
   }
   return a.type == cudaMemoryTypeDevice && a.device == dev;
 }
+
+namespace {
 
 template <bool TA, bool TB, int VEC>
 void launch(int M, int N, int K, double alpha, const double *A, long lda, const double *B,

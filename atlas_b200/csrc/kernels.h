@@ -14,6 +14,10 @@ void sgemm_dev(int ta, int tb, int M, int N, int K, float alpha, const float *A,
                const float *B, long ldb, float beta, float *C, long ldc, cudaStream_t st,
                int tri = 0);
 
+// Whether p lies in the current device's own memory (dgemm_dev writes it by bulk
+// copies, other memory by stores).
+bool own_memory(const void *p);
+
 // One problem of a grouped (batched, uneven) DGEMM: C = alpha*op(A)*op(B) + beta*C.
 struct GemmProb {
   const double *A, *B;

@@ -1096,14 +1096,15 @@ bool lookahead_enabled() { return tune(kTuneLookahead) != 0; }
 template <typename T>
 void getrf_dev(int M, int N, T *A, long lda, int *ipiv, int *dinfo, cudaStream_t st,
                SgemmFn gemm) {
-  // the launch sequence depends only on (M, N, lda, pointers): replayed as a graph
+  // the launch sequence depends only on (M, N, lda, pointers) and on whose memory A is
+  // in (dgemm_dev): replayed as a graph
   // multiple of 32, <= 256 (the fused panel's limit); the FP32 factorization has its own
   const int NBO = tune(sizeof(T) == 4 ? kTuneSgetrfNB : kTuneGetrfNB);
   const std::vector<unsigned long long> key = {1ull + sizeof(T), (unsigned long long)tune_generation(),
       (unsigned long long)M,
       (unsigned long long)N, (unsigned long long)lda, (unsigned long long)(uintptr_t)A,
       (unsigned long long)(uintptr_t)ipiv, (unsigned long long)(uintptr_t)dinfo,
-      (unsigned long long)(uintptr_t)gemm, (unsigned long long)(uintptr_t)st};
+      (unsigned long long)(uintptr_t)gemm, (unsigned long long)(uintptr_t)st, (unsigned long long)(sizeof(T) == 8 && own_memory(A))};
   run_graph(key, st, [&]() {
     set_info_kernel_launch(dinfo, st);
     const int MN = std::min(M, N), nblk = cdiv(MN, NBO);
@@ -1288,7 +1289,7 @@ template <typename T>
 void getrf_nopiv_dev(int N, T *A, long lda, int *dinfo, cudaStream_t st, SgemmFn gemm) {
   const std::vector<unsigned long long> key = {11ull + sizeof(T), (unsigned long long)N,
       (unsigned long long)lda, (unsigned long long)(uintptr_t)A, (unsigned long long)(uintptr_t)dinfo,
-      (unsigned long long)(uintptr_t)gemm, (unsigned long long)(uintptr_t)st};
+      (unsigned long long)(uintptr_t)gemm, (unsigned long long)(uintptr_t)st, (unsigned long long)(sizeof(T) == 8 && own_memory(A))};
   run_graph(key, st, [&]() {
     set_info_kernel_launch(dinfo, st);
     for (int j = 0; j < N; j += NBD) {

@@ -463,3 +463,89 @@ def test_geqrf_panel_widths_vs_oracle(gpu, orc, nb, la):
     finally:
         AB.atlb_tune_set("qr_nb", 128)
         AB.atlb_tune_set("lookahead", 1)
+
+
+def _ok(result):
+    assert result[0] == 0, result[0]
+    return result[1] if len(result) > 1 else None
+
+
+@pytest.mark.parametrize("kind", ["getrf", "potrf"])
+def test_replayed_factorizations_follow_the_memory_behind_an_address(gpu, kind):
+    """The factorizations' graphs are kept by address.  Here the same address is
+    device memory for the calls that record and replay one, and host memory for
+    the call after: the updates are then not those that add in the device's own L2.
+    |PA - LU| or |A - LL^T| <= gamma |L||U| with gamma = (n + 2) u, doubled for the
+    check's own product."""
+    import torch
+    from cuda.bindings import driver as d
+    from cuda.bindings import runtime as rt
+    dev = _ok(d.cuDeviceGet(0))
+    host_vmm = d.CUdevice_attribute.CU_DEVICE_ATTRIBUTE_HOST_NUMA_VIRTUAL_MEMORY_MANAGEMENT_SUPPORTED
+    if not _ok(d.cuDeviceGetAttribute(host_vmm, dev)):
+        pytest.skip("no host memory in the driver's virtual memory management here")
+    numa = _ok(d.cuDeviceGetAttribute(d.CUdevice_attribute.CU_DEVICE_ATTRIBUTE_HOST_NUMA_ID, dev))
+    n, u = 1536, 2.0 ** -53
+    rng = np.random.default_rng(9)
+    a0 = rng.uniform(-1, 1, (n, n))
+    if kind == "potrf":
+        a0 = a0 @ a0.T + n * np.eye(n)
+    src = torch.tensor(np.ascontiguousarray(a0.T), device="cuda")
+    out, ipiv, info = torch.empty_like(src), torch.zeros(n, dtype=torch.int32, device="cuda"), \
+        torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    loc = d.CUmemLocation()
+    access = d.CUmemAccessDesc()
+    access.location.type = d.CUmemLocationType.CU_MEM_LOCATION_TYPE_DEVICE
+    access.location.id = 0
+    access.flags = d.CUmemAccess_flags.CU_MEM_ACCESS_FLAGS_PROT_READWRITE
+    size, addr = 0, None
+
+    def memory(where, index):
+        nonlocal size, addr
+        prop = d.CUmemAllocationProp()
+        prop.type = d.CUmemAllocationType.CU_MEM_ALLOCATION_TYPE_PINNED
+        loc.type, loc.id = where, index
+        prop.location = loc
+        gran = _ok(d.cuMemGetAllocationGranularity(
+            prop, d.CUmemAllocationGranularity_flags.CU_MEM_ALLOC_GRANULARITY_RECOMMENDED))
+        if addr is None:
+            size = (8 * n * n + gran - 1) // gran * gran
+            addr = _ok(d.cuMemAddressReserve(size, 0, 0, 0))
+        assert size % gran == 0
+        return _ok(d.cuMemCreate(size, prop, 0))
+
+    def factor():
+        st = torch.cuda.current_stream().cuda_stream
+        _ok(d.cuMemcpyAsync(addr, src.data_ptr(), 8 * n * n, st))
+        if kind == "getrf":
+            assert AB.atlb_dgetrf_dev(n, n, int(addr), n, ipiv, info) == 0
+        else:
+            assert AB.atlb_dpotrf_dev(122, n, int(addr), n, info) == 0
+        _ok(d.cuMemcpyAsync(out.data_ptr(), addr, 8 * n * n, st))
+        assert AB.atlb_sync() == 0 and int(info.item()) == 0
+        f = out.cpu().numpy().T
+        if kind == "getrf":
+            want = a0.copy()
+            for k, p in enumerate(ipiv.cpu().numpy()):
+                want[[k, p]] = want[[p, k]]
+            low, up = np.tril(f, -1) + np.eye(n), np.triu(f)
+        else:
+            want, low = a0, np.tril(f)
+            up = low.T
+        assert np.all(np.abs(want - low @ up) <= 2 * (n + 2) * u * (np.abs(low) @ np.abs(up)))
+
+    for where, index, calls in ((d.CUmemLocationType.CU_MEM_LOCATION_TYPE_DEVICE, 0, 3),
+                                (d.CUmemLocationType.CU_MEM_LOCATION_TYPE_HOST_NUMA, numa, 1)):
+        handle = memory(where, index)
+        _ok(d.cuMemMap(addr, size, 0, handle, 0))
+        _ok(d.cuMemSetAccess(addr, size, [access], 1))
+        own = _ok(rt.cudaPointerGetAttributes(int(addr))).type == rt.cudaMemoryType.cudaMemoryTypeDevice
+        device = where == d.CUmemLocationType.CU_MEM_LOCATION_TYPE_DEVICE
+        if own == device:
+            for _ in range(calls):
+                factor()
+        _ok(d.cuMemUnmap(addr, size))
+        _ok(d.cuMemRelease(handle))
+        assert own == device
+    _ok(d.cuMemAddressFree(addr, size))
