@@ -407,11 +407,17 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
       }
     }
     __syncthreads();
-    for (int i = tid; i < kUnits * C; i += TH) {  // kUnits x C messages of 16 bytes
+    // kUnits x C messages of 16 bytes
+    auto send = [&](int i) {
       const int q = i / kUnits, unit = i - q * kUnits;
       st_async16(mapa_u32(smem_u32(&slot[b][crank]) + 16 * unit, q), reinterpret_cast<const uint4 *>(&stage)[unit],
                  mapa_u32(mb, q));
-    }
+    };
+    if (tid < kUnits * C) send(tid);
+    // not unrolled: the trip count would be a division by TH in every column's chain
+    // (8192 x 32: FP64 47.7 us unrolled, 45.0 now; 8192 x 256 FP32 366, 358)
+#pragma unroll 1
+    for (int i = tid + TH; i < kUnits * C; i += TH) send(i);
   };
   // wait until column c's C messages are in this CTA's slots
   auto receive = [&](int c) {
@@ -891,8 +897,10 @@ bool launch_fused_panel(int M, int ncols, T *A, long lda, int *ipiv, int roff, i
   // shared memory that every one of them reads the pivot row from.  At least 128,
   // below which the messages cost more than the warps (FP64 LU with 512 / 256 /
   // 128 / 64 / 32: order 500 1.20 / 1.11 / 1.08 / 1.12 / 1.21 ms, order 2000
-  // 4.40 / 3.93 / 3.86 / 3.97 / 4.05).
-  const int rows = std::max(128, cdiv(cdiv(M, most), 32) * 32), C = cdiv(M, rows);
+  // 4.40 / 3.93 / 3.86 / 3.97 / 4.05).  In FP32 up to 256 rows one CTA without
+  // messages is ahead of two (order 256: 465 us in two, 440 in one; 500: 881 with
+  // two CTAs of 256 rows, 866 with four of 128).
+  const int rows = std::max(sizeof(T) == 4 && M <= 256 ? 256 : 128, cdiv(cdiv(M, most), 32) * 32), C = cdiv(M, rows);
   const size_t smem = sizeof(T) * std::max(32 * rows, 64 * cdiv(nleft + nright, C));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C, 1, 1);
