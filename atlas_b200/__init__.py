@@ -56,6 +56,7 @@ _SIGS = {
     "atlb_get_stream": (_P, []),
     "atlb_set_stream": (None, [_P]),
     "atlb_sync": (_I, []),
+    "atlb_wait_word": (_P, []),
     "atlb_dgemm_dev": (_I, [_I, _I, _I, _I, _I, _D, _P, _I, _P, _I, _D, _P, _I]),
     "atlb_sgemm_dev": (_I, [_I, _I, _I, _I, _I, _F, _P, _I, _P, _I, _F, _P, _I]),
     "atlb_sgemm_tc_dev": (_I, [_I, _I, _I, _I, _I, _I, _F, _P, _I, _P, _I, _F, _P, _I]),

@@ -523,7 +523,7 @@ int atlb_dposv_batched(int count, const int *n, double *const *A, const int *lda
   cudaStream_t st = stream();
   int *hinfo = (int *)pinned(kSlotBatch1, sizeof(int) * count);
   batched_posv_dev(P, hinfo, st);
-  ATLB_CUDA_CHECK(cudaStreamSynchronize(st));
+  sync_stream(st);
   memcpy(info, hinfo, sizeof(int) * count);
   return 0;
 }
@@ -545,7 +545,7 @@ int atlb_dgesv_batched(int count, const int *n, double *const *A, const int *lda
   cudaStream_t st = stream();
   int *hinfo = (int *)pinned(kSlotBatch1, sizeof(int) * count);
   batched_gesv_dev(P, hinfo, st);
-  ATLB_CUDA_CHECK(cudaStreamSynchronize(st));
+  sync_stream(st);
   memcpy(info, hinfo, sizeof(int) * count);
   return 0;
 }

@@ -19,8 +19,6 @@ void xerbla(int pos, const char *rout);
 
 namespace {
 
-void sync(cudaStream_t st) { ATLB_CUDA_CHECK(cudaStreamSynchronize(st)); }
-
 __global__ void reflect_upper_kernel(int n, double *C, long ldc) {
   long total = (long)n * n;
   for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
@@ -119,7 +117,7 @@ void cblas_dgemm(const enum CBLAS_ORDER Order, const enum CBLAS_TRANSPOSE TA,
   DMat<double> dC = stage_in(kSlotC, C, m, n, ldc, beta != 0.0, st);
   dgemm_core(ta, tb, m, n, K, alpha, dA.d, dA.ld, dB.d, dB.ld, beta, dC.d, dC.ld, st, shortcut);
   stage_out(C, ldc, dC, m, n, st);
-  sync(st);
+  sync_stream(st);
 }
 
 void cblas_sgemm(const enum CBLAS_ORDER Order, const enum CBLAS_TRANSPOSE TA,
@@ -156,7 +154,7 @@ void cblas_sgemm(const enum CBLAS_ORDER Order, const enum CBLAS_TRANSPOSE TA,
   DMat<float> dC = stage_in(kSlotC, C, m, n, ldc, beta != 0.f, st);
   sgemm_dev(ta, tb, m, n, K, alpha, dA.d, dA.ld, dB.d, dB.ld, beta, dC.d, dC.ld, st, 0);
   stage_out(C, ldc, dC, m, n, st);
-  sync(st);
+  sync_stream(st);
 }
 
 static int trsm_like_checks(const char *name, int Order, int Side, int Uplo, int TA, int Diag,
@@ -199,7 +197,7 @@ void cblas_dtrsm(const enum CBLAS_ORDER Order, const enum CBLAS_SIDE Side,
   trsm_dev<double>(side, uplo, (int)TA == kNoTrans ? kNoTrans : kTrans, Diag, m, n, alpha, dA.d, dA.ld,
                    dB.d, dB.ld, st);
   stage_out(B, ldb, dB, m, n, st);
-  sync(st);
+  sync_stream(st);
 }
 
 void cblas_dtrmm(const enum CBLAS_ORDER Order, const enum CBLAS_SIDE Side,
@@ -221,7 +219,7 @@ void cblas_dtrmm(const enum CBLAS_ORDER Order, const enum CBLAS_SIDE Side,
   dtrmm_dev(side, uplo, (int)TA == kNoTrans ? kNoTrans : kTrans, Diag, m, n, alpha, dA.d, dA.ld, dB.d,
             dB.ld, st);
   stage_out(B, ldb, dB, m, n, st);
-  sync(st);
+  sync_stream(st);
 }
 
 void cblas_dsyrk(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo,
@@ -258,7 +256,7 @@ void cblas_dsyrk(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo,
   else
     dgemm_dev(kTrans, kNoTrans, N, N, K, alpha, dA.d, dA.ld, dA.d, dA.ld, beta, dC.d, dC.ld, st, tri);
   stage_out(C, ldc, dC, N, N, st);
-  sync(st);
+  sync_stream(st);
 }
 
 // ---------------------------------------------------------------- LAPACK
@@ -287,8 +285,8 @@ int clapack_dgetrf(const enum CBLAS_ORDER Order, const int M, const int N, doubl
   stage_vec_out<int>(ipiv, dip, mn, st);
   int *hinfo = (int *)pinned(kSlotInfo, 64);
   ATLB_CUDA_CHECK(cudaMemcpyAsync(hinfo, dinfo, sizeof(int), cudaMemcpyDeviceToHost, st));
-  sync(st);
-  return *hinfo;
+  const int lost = sync_stream(st);
+  return *hinfo ? *hinfo : lost;
 }
 
 int clapack_dgetrs(const enum CBLAS_ORDER Order, const enum CBLAS_TRANSPOSE Trans, const int N,
@@ -313,8 +311,7 @@ int clapack_dgetrs(const enum CBLAS_ORDER Order, const enum CBLAS_TRANSPOSE Tran
   DMat<double> dB = stage_in(kSlotB, B, N, NRHS, ldb, true, st);
   getrs_dev<double>(tr, N, NRHS, dA.d, dA.ld, dip, dB.d, dB.ld, st);
   stage_out(B, ldb, dB, N, NRHS, st);
-  sync(st);
-  return 0;
+  return sync_stream(st);
 }
 
 int clapack_dgesv(const enum CBLAS_ORDER Order, const int N, const int NRHS, double *A,
@@ -337,14 +334,14 @@ int clapack_dgesv(const enum CBLAS_ORDER Order, const int N, const int NRHS, dou
   ATLB_CUDA_CHECK(cudaMemcpyAsync(hinfo, dinfo, sizeof(int), cudaMemcpyDeviceToHost, st));
   stage_out(A, lda, dA, N, N, st);
   stage_vec_out<int>(ipiv, dip, N, st);
-  sync(st);
-  int info = *hinfo;
+  const int lost = sync_stream(st);
+  int info = *hinfo ? *hinfo : lost;
   if (info == 0 && NRHS > 0) {
     int tr = Order == CblasColMajor ? kNoTrans : kTrans;
     DMat<double> dB = stage_in(kSlotB, B, N, NRHS, ldb, true, st);
     getrs_dev<double>(tr, N, NRHS, dA.d, dA.ld, dip, dB.d, dB.ld, st);
     stage_out(B, ldb, dB, N, NRHS, st);
-    sync(st);
+    info = sync_stream(st);
   }
   return info;
 }
@@ -375,8 +372,8 @@ int clapack_dpotrf(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo, con
   stage_out(A, lda, dA, N, N, st);
   int *hinfo = (int *)pinned(kSlotInfo, 64);
   ATLB_CUDA_CHECK(cudaMemcpyAsync(hinfo, dinfo, sizeof(int), cudaMemcpyDeviceToHost, st));
-  sync(st);
-  return *hinfo;
+  const int lost = sync_stream(st);
+  return *hinfo ? *hinfo : lost;
 }
 
 int clapack_dpotrs(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo, const int N,
@@ -398,8 +395,7 @@ int clapack_dpotrs(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo, con
   DMat<double> dB = stage_in(kSlotB, B, N, NRHS, ldb, true, st);
   potrs_dev<double>(uplo, N, NRHS, dA.d, dA.ld, dB.d, dB.ld, st);
   stage_out(B, ldb, dB, N, NRHS, st);
-  sync(st);
-  return 0;
+  return sync_stream(st);
 }
 
 int clapack_dposv(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo, const int N,
@@ -423,13 +419,13 @@ int clapack_dposv(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo, cons
   int *hinfo = (int *)pinned(kSlotInfo, 64);
   ATLB_CUDA_CHECK(cudaMemcpyAsync(hinfo, dinfo, sizeof(int), cudaMemcpyDeviceToHost, st));
   stage_out(A, lda, dA, N, N, st);
-  sync(st);
-  int info = *hinfo;
+  const int lost = sync_stream(st);
+  int info = *hinfo ? *hinfo : lost;
   if (info == 0 && NRHS > 0) {
     DMat<double> dB = stage_in(kSlotB, B, N, NRHS, ldb, true, st);
     potrs_dev<double>(uplo, N, NRHS, dA.d, dA.ld, dB.d, dB.ld, st);
     stage_out(B, ldb, dB, N, NRHS, st);
-    sync(st);
+    info = sync_stream(st);
   }
   return info;
 }
@@ -452,8 +448,7 @@ int ATL_dgeqrf(const int M, const int N, double *A, const int lda, double *TAU, 
   dgeqrf_dev(M, N, dA.d, dA.ld, dtau, st);
   stage_out(A, lda, dA, M, N, st);
   stage_vec_out<double>(TAU, dtau, mn, st);
-  sync(st);
-  return 0;
+  return sync_stream(st);
 }
 
 int clapack_dgeqrf(const enum CBLAS_ORDER Order, const int M, const int N, double *A,
@@ -482,8 +477,7 @@ int clapack_dgeqrf(const enum CBLAS_ORDER Order, const int M, const int N, doubl
   transpose_dev(M, N, T, M, dV.d, dV.ld, st);
   stage_out(A, lda, dV, N, M, st);
   stage_vec_out<double>(TAU, dtau, mn, st);
-  sync(st);
-  return 0;
+  return sync_stream(st);
 }
 
 // ---------------------------------------------------------------- device API

@@ -29,6 +29,13 @@ enum { kLeft = 141, kRight = 142 };
 
 void set_cuda_error(cudaError_t e);
 cudaStream_t stream();           // the library's stream for the calling thread
+// The calling thread's word in pinned host memory, null if there is none, that a
+// kernel sets to 1 when one of its bounded waits gives up (its results are then marked
+// or wrong).  sync_stream() waits for a stream and reports the word, then clears
+// it: 0, or a CUDA error (cudaErrorLaunchTimeout for a wait that gave up), which is
+// recorded too.
+int *wait_word();
+int sync_stream(cudaStream_t st);
 int num_sms();
 
 // Device memory cache: grow-only buffers keyed by slot, reused across calls
@@ -98,6 +105,11 @@ void run_graph(const std::vector<unsigned long long> &key, cudaStream_t st,
 
 // ---------------------------------------------------------------------------
 // Device helpers
+// a bounded wait gave up: tell the host (wait_word())
+__device__ __forceinline__ void report_lost_wait(int *word) {
+  if (word) *(volatile int *)word = 1;
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

@@ -28,8 +28,6 @@ void xerbla(int pos, const char *rout);
 
 namespace {
 
-void sync_st(cudaStream_t st) { ATLB_CUDA_CHECK(cudaStreamSynchronize(st)); }
-
 int grid_of(long n) { return (int)std::min<long>((n + 255) / 256, 8192); }
 
 // W (n x n, ld n) = I
@@ -99,7 +97,7 @@ int first_zero_diag(int n, const double *A, long lda, cudaStream_t st) {
   double *h = (double *)pinned(kSlotExt3, sizeof(double) * n);
   ATLB_CUDA_CHECK(cudaMemcpy2DAsync(h, sizeof(double), A, (lda + 1) * sizeof(double), sizeof(double), n,
                                     cudaMemcpyDeviceToHost, st));
-  sync_st(st);
+  ATLB_CUDA_CHECK(cudaStreamSynchronize(st));
   for (int i = 0; i < n; i++)
     if (h[i] == 0.0) return i + 1;
   return 0;
@@ -294,7 +292,7 @@ void cblas_dsymm(const enum CBLAS_ORDER Order, const enum CBLAS_SIDE Side, const
   DMat<double> dC = stage_in(kSlotC, (const double *)C, m, n, ldc, beta != 0.0, st);
   dsymm_dev(side, uplo, m, n, alpha, dA.d, dA.ld, dB.d, dB.ld, beta, dC.d, dC.ld, st);
   stage_out(C, ldc, dC, m, n, st);
-  sync_st(st);
+  sync_stream(st);
 }
 
 void cblas_dsyr2k(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo, const enum CBLAS_TRANSPOSE Trans,
@@ -327,7 +325,7 @@ void cblas_dsyr2k(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo, cons
   DMat<double> dC = stage_in(kSlotC, (const double *)C, N, N, ldc, true, st);
   dsyr2k_dev(uplo, trans, N, K, alpha, dA.d, dA.ld, dB.d, dB.ld, beta, dC.d, dC.ld, st);
   stage_out(C, ldc, dC, N, N, st);
-  sync_st(st);
+  sync_stream(st);
 }
 
 void cblas_zgemm(const enum CBLAS_ORDER Order, const enum CBLAS_TRANSPOSE TransA,
@@ -372,7 +370,7 @@ void cblas_zgemm(const enum CBLAS_ORDER Order, const enum CBLAS_TRANSPOSE TransA
   DMat<double> dC = stage_in(kSlotC, (const double *)C, 2 * m, n, 2L * ldc, readc, st);
   zgemm_dev(ta, tb, m, n, K, al, dA.d, dA.ld / 2, dB.d, dB.ld / 2, be, dC.d, dC.ld / 2, st);
   stage_out((double *)C, 2L * ldc, dC, 2 * m, n, st);
-  sync_st(st);
+  sync_stream(st);
 }
 
 int clapack_dgetri(const enum CBLAS_ORDER Order, const int N, double *A, const int lda, const int *ipiv) {
@@ -389,8 +387,8 @@ int clapack_dgetri(const enum CBLAS_ORDER Order, const int N, double *A, const i
   int *dip = stage_vec_in<int>(kSlotIpiv, ipiv, N, true, st);
   const int info = dgetri_dev(N, dA.d, dA.ld, dip, st);
   stage_out(A, lda, dA, N, N, st);
-  sync_st(st);
-  return info;
+  const int lost = sync_stream(st);
+  return info ? info : lost;
 }
 
 int clapack_dtrtri(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo, const enum CBLAS_DIAG Diag,
@@ -411,8 +409,8 @@ int clapack_dtrtri(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo, con
   DMat<double> dA = stage_in(kSlotA, A, N, N, lda, true, st);
   const int info = dtrtri_dev(uplo, Diag, N, dA.d, dA.ld, st);
   stage_out(A, lda, dA, N, N, st);
-  sync_st(st);
-  return info;
+  const int lost = sync_stream(st);
+  return info ? info : lost;
 }
 
 int clapack_dlauum(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo, const int N, double *A,
@@ -430,8 +428,7 @@ int clapack_dlauum(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo, con
   DMat<double> dA = stage_in(kSlotA, A, N, N, lda, true, st);
   dlauum_dev(uplo, N, dA.d, dA.ld, st);
   stage_out(A, lda, dA, N, N, st);
-  sync_st(st);
-  return 0;
+  return sync_stream(st);
 }
 
 int clapack_dpotri(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo, const int N, double *A,
@@ -450,8 +447,8 @@ int clapack_dpotri(const enum CBLAS_ORDER Order, const enum CBLAS_UPLO Uplo, con
   const int info = dtrtri_dev(uplo, kNonUnit, N, dA.d, dA.ld, st);
   if (!info) dlauum_dev(uplo, N, dA.d, dA.ld, st);
   stage_out(A, lda, dA, N, N, st);
-  sync_st(st);
-  return info;
+  const int lost = sync_stream(st);
+  return info ? info : lost;
 }
 
 int clapack_dgels(const enum CBLAS_ORDER Order, const enum CBLAS_TRANSPOSE TA, const int M, const int N,
@@ -481,8 +478,8 @@ int clapack_dgels(const enum CBLAS_ORDER Order, const enum CBLAS_TRANSPOSE TA, c
   const int info = dgels_dev(ta, m, n, NRHS, dA.d, dA.ld, dB.d, dB.ld, st);
   stage_out(A, lda, dA, m, n, st);
   stage_out(B, ldb, dB, rb, NRHS, st);
-  sync_st(st);
-  return info;
+  const int lost = sync_stream(st);
+  return info ? info : lost;
 }
 
 int clapack_dgelqf(const enum CBLAS_ORDER Order, const int M, const int N, double *A, const int lda,
@@ -513,8 +510,7 @@ int clapack_dgelqf(const enum CBLAS_ORDER Order, const int M, const int N, doubl
     stage_out(A, lda, dA, M, N, st);
   }
   stage_vec_out<double>(TAU, dtau, mn, st);
-  sync_st(st);
-  return 0;
+  return sync_stream(st);
 }
 
 int ATL_dormqr(const enum CBLAS_SIDE SIDE, const enum CBLAS_TRANSPOSE TRANS, const int M, const int N,
@@ -543,8 +539,7 @@ int ATL_dormqr(const enum CBLAS_SIDE SIDE, const enum CBLAS_TRANSPOSE TRANS, con
   DMat<double> dC = stage_in(kSlotC, (const double *)C, M, N, ldc, true, st);
   dormqr_dev(SIDE, TRANS == CblasNoTrans ? kNoTrans : kTrans, M, N, K, dA.d, dA.ld, dtau, dC.d, dC.ld, st);
   stage_out(C, ldc, dC, M, N, st);
-  sync_st(st);
-  return 0;
+  return sync_stream(st);
 }
 
 int atlb_dormqr_dev(int Side, int Trans, int M, int N, int K, const double *A, int lda, const double *tau,

@@ -314,7 +314,6 @@ __device__ __forceinline__ void stage_row(T *stage, const T (&a)[NB], int off) {
 constexpr int kMaxPanelCluster = 16;
 // rows up to which one CTA takes an FP64 panel (getf2_cta_kernel has the times)
 constexpr int kCtaPanelRows = 256;
-__device__ int g_panel_timeout = 0;  // set if a panel wait ever gives up (1 s)
 
 template <typename T, int NB>
 __global__ void __launch_bounds__(PT, 1)
@@ -427,7 +426,17 @@ getf2_fused_kernel(int M, int ncols, T *__restrict__ A, long lda, int *__restric
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
       while (!mbar_try_wait(mb, parity)) {
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-        if (t - t0 > 1000000000ull) { atomicExch(&g_panel_timeout, 1); break; }
+        if (t - t0 > 1000000000ull) {
+          // 1 s: recorded for finish_info_kernel, and the column goes on without an
+          // interchange, whatever of the messages still arrives (a position comes with
+          // its key, and any key beats zero)
+          atomicMin(dinfo, INT_MIN + roff + c + 1);
+          for (int q = 0; q < C; q++) {
+            slot[c & 1][q].key = K(0);
+            slot[c & 1][q].pos = c;
+          }
+          break;
+        }
       }
     }
   };

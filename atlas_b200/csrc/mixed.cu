@@ -846,8 +846,8 @@ int atlb_dsgesv_ex(int N, int NRHS, double *A, int lda, int *ipiv, double *B, in
     stage_out(A, lda, dA, N, N, st);
     stage_vec_out<int>(ipiv, dip, N, st);
   }
-  ATLB_CUDA_CHECK(cudaStreamSynchronize(st));
-  return info;
+  const int lost = sync_stream(st);
+  return info ? info : lost;
 }
 
 int atlb_mixed_krylov_steps(void) { return tl_krylov_steps; }
@@ -927,8 +927,8 @@ int atlb_dsposv(int Uplo, int N, int NRHS, double *A, int lda, double *B, int ld
                     nullptr, krylov_mode(prec));
   stage_out(X, ldx, dX, N, NRHS, st);
   if (fell_back) stage_out(A, lda, dA, N, N, st);
-  ATLB_CUDA_CHECK(cudaStreamSynchronize(st));
-  return info;
+  const int lost = sync_stream(st);
+  return info ? info : lost;
 }
 
 }  // extern "C"

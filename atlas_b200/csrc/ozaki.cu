@@ -189,7 +189,7 @@ int atlb_dgemm_ozaki(int TA, int TB, int M, int N, int K, double alpha, const do
   dgemm_ozaki_dev(tA ? kTrans : kNoTrans, tB ? kTrans : kNoTrans, M, N, K, alpha, dA.d, dA.ld, dB.d,
                   dB.ld, beta, dC.d, dC.ld, slices, st);
   stage_out(C, ldc, dC, M, N, st);
-  ATLB_CUDA_CHECK(cudaStreamSynchronize(st));
+  sync_stream(st);
   return 0;
 }
 

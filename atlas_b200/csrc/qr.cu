@@ -58,12 +58,13 @@ __device__ __forceinline__ double warp_reduce_scatter(double (&v)[NB], int lane)
 // mbarrier): a cluster barrier there also waits for the multipliers' global
 // stores, and remote reads after it cost another round trip.  One warp then
 // forms beta, tau and the update row w, and every thread applies it.  Waits
-// are bounded (1 s, g_qr_timeout).  16 columns of 16384 rows: 72 us with the
-// barrier, the remote reads and the columns unrolled; 34 us now.
-__device__ int g_qr_timeout = 0;
+// are bounded (1 s): a CTA that gives up reports it (wait_word()) and continues with
+// NaN, which the other CTAs get with its next message and tau carries out.  16
+// columns of 16384 rows: 72 us with the barrier, the remote reads and the columns
+// unrolled; 34 us now.
 template <int NB, int RPT>
 __global__ void __launch_bounds__(QT, 1)
-geqr2_cluster_kernel(int M, int ncols, double *__restrict__ A, long lda, double *__restrict__ tau) {
+geqr2_cluster_kernel(int M, int ncols, double *__restrict__ A, long lda, double *__restrict__ tau, int *word) {
   static_assert(NB <= 32, "one lane per column");
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks(), crank = (int)cl.block_rank();
@@ -143,7 +144,11 @@ geqr2_cluster_kernel(int M, int ncols, double *__restrict__ A, long lda, double 
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
         while (!mbar_try_wait(mbj, parity)) {
           asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-          if (t1 - t0 > 1000000000ull) { atomicExch(&g_qr_timeout, 1); break; }
+          if (t1 - t0 > 1000000000ull) {
+            report_lost_wait(word);
+            for (int r = 0; r < C; r++) part[b][r][lane % NB] = __longlong_as_double(-1LL);
+            break;
+          }
         }
       }
       __syncwarp();
@@ -293,7 +298,7 @@ void launch_geqr2_cluster(int M, int ncols, double *A, long lda, double *tau, cu
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  ATLB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, M, ncols, A, lda, tau));
+  ATLB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, M, ncols, A, lda, tau, wait_word()));
 }
 
 void init_qr_cluster() {

@@ -23,6 +23,7 @@ struct ThreadState {
   bool own_stream = false;
   cudaStream_t side = nullptr;
   cudaStream_t copy = nullptr;
+  int *lost_wait = nullptr;  // wait_word()
   cudaEvent_t events[8] = {};
   std::vector<cudaEvent_t> chunk_events;
   Buf dev[2 * kNumSlots];   // second half: buffers of work on the side stream
@@ -73,12 +74,42 @@ int num_sms() {
 
 cudaStream_t stream() {
   ensure_device();
+  wait_word();
   if (!tl.stream) {
     ATLB_CUDA_CHECK(cudaSetDevice(g_device));
     ATLB_CUDA_CHECK(cudaStreamCreateWithFlags(&tl.stream, cudaStreamNonBlocking));
     tl.own_stream = true;
   }
   return tl.stream;
+}
+
+int *wait_word() {
+  if (!tl.lost_wait) {
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    tl.lost_wait = (int *)p;
+    *tl.lost_wait = 0;
+  }
+  return tl.lost_wait;
+}
+
+int sync_stream(cudaStream_t st) {
+  cudaError_t e = cudaStreamSynchronize(st);
+  volatile int *w = tl.lost_wait;
+  if (e == cudaSuccess && w && *w) {
+    *w = 0;
+    e = cudaErrorLaunchTimeout;
+    fprintf(stderr, "atlas_b200: a kernel gave up a wait for its peers; the results since the last "
+                    "synchronization are not valid\n");
+  } else if (e != cudaSuccess) {
+    fprintf(stderr, "atlas_b200: CUDA error %s at a synchronization: %s\n", cudaGetErrorName(e),
+            cudaGetErrorString(e));
+  }
+  if (e != cudaSuccess) set_cuda_error(e);
+  return (int)e;
 }
 
 cudaStream_t side_stream() {
@@ -328,11 +359,8 @@ void atlb_set_stream(void *s) {
   tl.own_stream = false;
   if (!s) stream();
 }
-int atlb_sync(void) {
-  cudaError_t e = cudaStreamSynchronize(stream());
-  if (e != cudaSuccess) tl_cuda_error = e;
-  return (int)e;
-}
+int atlb_sync(void) { return sync_stream(stream()); }
+int *atlb_wait_word(void) { return (stream(), wait_word()); }
 
 void cblas_xerbla(int p, const char *rout, const char *form, ...) {
   va_list ap;

@@ -9,8 +9,8 @@
 // tiles with TMA (each CTA loads its own tiles), one thread of warp 1 issues tcgen05.mma into
 // a TMEM accumulator and releases each stage with tcgen05.commit, and all
 // four warps drain TMEM (tcgen05.ld 32x32b) into the epilogue.  Every
-// mbarrier wait is bounded: on timeout the kernel records an error code in
-// *err, stops, frees its TMEM and returns.
+// mbarrier wait is bounded: on timeout the kernel reports it (wait_word()), stops,
+// frees its TMEM and returns.
 //
 // Epilogues: FP32 column-major C = alpha*D + beta*C (optionally one triangle
 // only), and the split-integer (Ozaki) accumulation C_fp64 += w * rs[m] *
@@ -130,7 +130,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 template <int KIND, int BN, int STAGES, int EPI, int MS = 1, int SPLIT = 0>
 __global__ void __launch_bounds__(THREADS, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-               int M, int N, int K, EpiParams ep, int *err) {
+               int M, int N, int K, EpiParams ep, int *word) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // 1024-byte aligned base for the swizzled tiles
   unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -183,7 +183,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     for (int kb = 0; kb < nkb; kb++) {
       const int s = kb % STAGES;
       const uint32_t ph = (kb / STAGES) & 1;
-      if (kb >= STAGES && !mbar_wait(bar_empty + 8 * s, ph ^ 1, TO)) { atomicExch(err, 1); break; }
+      if (kb >= STAGES && !mbar_wait(bar_empty + 8 * s, ph ^ 1, TO)) { report_lost_wait(word); break; }
       mbar_expect_tx(bar_full + 8 * s, STAGE);
 #pragma unroll
       for (int p = 0; p < NP; p++) {
@@ -195,11 +195,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   } else if (warp == 1 && lane == 0) {
     // MMA issuer
     constexpr uint32_t idesc = instr_desc<KIND, BN>();
-    bool ok = true;
     for (int kb = 0; kb < nkb; kb++) {
       const int s = kb % STAGES;
       const uint32_t ph = (kb / STAGES) & 1;
-      if (!mbar_wait(bar_full + 8 * s, ph, TO)) { atomicExch(err, 2); ok = false; break; }
+      if (!mbar_wait(bar_full + 8 * s, ph, TO)) { report_lost_wait(word); break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t a_addr = sbase + s * STAGE, b_addr = a_addr + NP * A_BYTES;
 #pragma unroll
@@ -216,7 +215,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                    ::"r"(bar_empty + 8 * s) : "memory");
     }
-    (void)ok;
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                  ::"r"(bar_done) : "memory");
   }
@@ -227,7 +225,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   done = __all_sync(0xffffffffu, done);
   __syncwarp();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (!done) atomicExch(err, 3);
+  if (!done) report_lost_wait(word);
 #pragma unroll 1
   for (int ms = 0; ms < MS; ms++) {
   const int m = m0 + ms * BM + warp * 32 + lane;
@@ -328,15 +326,6 @@ bool make_map(CUtensorMap *map, int kind, const void *base, int rows, int K, lon
   return r == CUDA_SUCCESS;
 }
 
-int *err_flag() {
-  static int *d = nullptr;
-  if (!d) {
-    ATLB_CUDA_CHECK(cudaMalloc(&d, sizeof(int)));
-    ATLB_CUDA_CHECK(cudaMemset(d, 0, sizeof(int)));
-  }
-  return d;
-}
-
 // SPLIT: A and B rows hold two K-element planes (K a multiple of 32)
 template <int KIND, int BN, int STAGES, int EPI, int MS = 1, int SPLIT = 0>
 void launch_t(const void *A, long lda, const void *B, long ldb, int M, int N, int K,
@@ -356,7 +345,7 @@ void launch_t(const void *A, long lda, const void *B, long ldb, int M, int N, in
     configured = true;
   }
   const int tiles = cdiv(M, BM * MS) * cdiv(N, BN);
-  kern<<<tiles, THREADS, smem, st>>>(ma, mb, M, N, K, ep, err_flag());
+  kern<<<tiles, THREADS, smem, st>>>(ma, mb, M, N, K, ep, wait_word());
   ATLB_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -386,14 +375,6 @@ void tc_gemm_split(const float *A2, const float *B2, long ldk, int M, int N, con
   // CTA's epilogue runs under the other's products, and each CTA retires
   // after one tile, which keeps SMs turning over for the look-ahead stream
   launch_t<kKindTF32, 64, 2, kEpiF32, 1, 1>(A2, 2 * ldk, B2, 2 * ldk, M, N, (int)ldk, ep, st);
-}
-
-int read_and_clear_error(cudaStream_t st) {
-  int h = 0;
-  ATLB_CUDA_CHECK(cudaMemcpyAsync(&h, err_flag(), sizeof(int), cudaMemcpyDeviceToHost, st));
-  ATLB_CUDA_CHECK(cudaStreamSynchronize(st));
-  if (h) ATLB_CUDA_CHECK(cudaMemsetAsync(err_flag(), 0, sizeof(int), st));
-  return h;
 }
 
 // ---------------------------------------------------------------- FP32 GEMM on tensor cores

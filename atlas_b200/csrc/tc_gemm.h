@@ -22,9 +22,5 @@ struct EpiParams {
 // elements, 16-byte aligned rows); the epilogue consumes D.
 void tc_gemm(int kind, int epi, const void *A, long lda, const void *B, long ldb, int M, int N,
              int K, const EpiParams &ep, cudaStream_t st);
-// Error code recorded by a kernel whose bounded wait timed out (0 = none);
-// reading it synchronises the stream and clears it.
-int read_and_clear_error(cudaStream_t st);
-
 }  // namespace tc
 }  // namespace atlb

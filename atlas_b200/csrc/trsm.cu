@@ -9,6 +9,7 @@
 // solve T*X = B with T and B addressed through (row, column) strides, so one
 // leaf kernel serves all eight cases.
 #include <algorithm>
+#include <climits>
 #include "common.cuh"
 #include "kernels.h"
 #include "chol_blocks.cuh"
@@ -798,7 +799,15 @@ __global__ void fill_zero_kernel(T *A, int M, int N, long lda) {
 }
 
 __global__ void set_info_kernel(int *d) { *d = 0x7fffffff; }
-__global__ void finish_info_kernel(int *d) { if (*d == 0x7fffffff) *d = 0; }
+// also reports a panel's wait that gave up, which left INT_MIN + its column (lu.cu)
+__global__ void finish_info_kernel(int *d, int *word) {
+  if (*d < 0) {
+    *d -= INT_MIN;
+    report_lost_wait(word);
+  } else if (*d == 0x7fffffff) {
+    *d = 0;
+  }
+}
 
 }  // namespace
 
@@ -1353,6 +1362,6 @@ template void fill_zero_dev<double>(double *, int, int, long, cudaStream_t);
 template void fill_zero_dev<float>(float *, int, int, long, cudaStream_t);
 
 void set_info_kernel_launch(int *d, cudaStream_t st) { set_info_kernel<<<1, 1, 0, st>>>(d); }
-void finish_info_kernel_launch(int *d, cudaStream_t st) { finish_info_kernel<<<1, 1, 0, st>>>(d); }
+void finish_info_kernel_launch(int *d, cudaStream_t st) { finish_info_kernel<<<1, 1, 0, st>>>(d, wait_word()); }
 
 }  // namespace atlb

@@ -17,8 +17,8 @@
 // single-copy-atomic store, and the next block polls those words directly --
 // one round trip to L2 on the chain instead of fence, flag and data load (in
 // FP64, with two words a value, that changed nothing).
-// Every wait is bounded: after ~1 s the kernel records an error in *err and
-// stops waiting (the result is then wrong but the GPU is released).  The
+// Every wait is bounded: after ~1 s the kernel reports it (wait_word()), stops
+// waiting, and marks its block of x, and so all that follow from it, with NaN.  The
 // launcher clears the ticket counter, the flags and the tagged words before
 // each launch.
 #include <algorithm>
@@ -50,18 +50,19 @@ __device__ __forceinline__ int ld_acquire(const int *p) {
 template <typename T, int NR>
 __global__ void __launch_bounds__(TT, 1)
 trsv_kernel(int n, int nrhs, const T *__restrict__ Tp, long tr, long tc, int lower,
-            const T *__restrict__ W, T *X, long ldx, int *counter, int *flags, int epoch, int *err,
+            const T *__restrict__ W, T *X, long ldx, int *counter, int *flags, int epoch, int *word,
             unsigned long long *xt) {
   extern __shared__ __align__(16) unsigned char trsv_smem[];
   T(*sW)[CB + 1] = reinterpret_cast<T(*)[CB + 1]>(trsv_smem);   // [CB]: the inverted diagonal block
   T(*sxd)[CB][NR] = reinterpret_cast<T(*)[CB][NR]>(sW + CB);    // x of a solved block, double-buffered
   T(*sb)[NR] = reinterpret_cast<T(*)[NR]>(sxd + 2);             // this block's b
   T(*sacc)[CB][NR] = reinterpret_cast<T(*)[CB][NR]>(sb + CB);   // [NQ]: the parts' sums
-  __shared__ int s_bi, s_ready;
+  __shared__ int s_bi, s_ready, s_late[2];
   const int tid = threadIdx.x, lane = tid & 31, nb = (n + CB - 1) / CB;
   if (tid == 0) {
     const int t = atomicAdd(counter, 1);
     s_bi = lower ? t : nb - 1 - t;
+    s_late[0] = s_late[1] = 0;
   }
   __syncthreads();
   const int bi = s_bi, r0 = bi * CB, rows = min(CB, n - r0);
@@ -87,10 +88,14 @@ trsv_kernel(int n, int nrhs, const T *__restrict__ Tp, long tr, long tc, int low
   T acc[NR], acc2[NR];  // even and odd columns: two independent FMA chains
 #pragma unroll
   for (int q = 0; q < NR; q++) acc[q] = acc2[q] = T(0);
+  auto give_up = [&]() {  // one thread: b, and with it x, becomes NaN
+    report_lost_wait(word);
+    for (int idx = 0; idx < CB * NR; idx++) sb[idx / NR][idx % NR] = (T)__longlong_as_double(-1LL);
+  };
   auto wait_flag = [&](int bj) {
     const uint64_t t0 = gtimer();
     while (ld_acquire(flags + bj) != epoch) {
-      if (gtimer() - t0 > 1000000000ull) { atomicExch(err, 1); break; }
+      if (gtimer() - t0 > 1000000000ull) { give_up(); break; }
     }
   };
   // x of block bj into sxd[buf] (all threads), then the products
@@ -153,6 +158,7 @@ trsv_kernel(int n, int nrhs, const T *__restrict__ Tp, long tr, long tc, int low
       // single-copy-atomic store, so a word whose tag is current carries its
       // value: one round trip to L2 instead of flag, fence and data
       const uint64_t t0 = gtimer();
+      int poll = 0;
       while (true) {
         bool ok = true;
         for (int idx = tid; idx < CB * NR; idx += TT) {
@@ -166,10 +172,12 @@ trsv_kernel(int n, int nrhs, const T *__restrict__ Tp, long tr, long tc, int low
           sxd[buf][cc][q] = v;
         }
         if (__syncthreads_and(ok)) break;
-        if (gtimer() - t0 > 1000000000ull) {  // bounded: record and go on (the result is then wrong)
-          if (tid == 0) atomicExch(err, 1);
+        if (s_late[poll & 1]) {  // thread 0's clock as of the poll before, so that all leave together
+          if (tid == 0) give_up();
           break;
         }
+        poll++;
+        if (tid == 0 && gtimer() - t0 > 1000000000ull) s_late[poll & 1] = 1;
       }
     } else {
       if (tid == 0) wait_flag(bj);
@@ -251,7 +259,7 @@ trsv_kernel(int n, int nrhs, const T *__restrict__ Tp, long tr, long tc, int low
 template <int NH>
 __global__ void __launch_bounds__(TT, 1)
 trsv_mma_kernel(int n, int nrhs, const double *__restrict__ Tp, long tr, long tc, int lower,
-                const double *__restrict__ W, double *X, long ldx, int *counter, int *flags, int epoch, int *err) {
+                const double *__restrict__ W, double *X, long ldx, int *counter, int *flags, int epoch, int *word) {
   constexpr int NR = 8 * NH, LX = NH == 1 ? 12 : 20, LW = CB + 4;  // fragments in distinct banks
   extern __shared__ __align__(16) unsigned char trsv_smem[];
   double *sW = reinterpret_cast<double *>(trsv_smem);  // W(r, c) at r * LW + c
@@ -286,10 +294,14 @@ trsv_mma_kernel(int n, int nrhs, const double *__restrict__ Tp, long tr, long tc
   double acc[NH][2];
 #pragma unroll
   for (int h = 0; h < NH; h++) acc[h][0] = acc[h][1] = 0.0;
+  auto give_up = [&]() {  // one thread: b, and with it x, becomes NaN
+    report_lost_wait(word);
+    for (int idx = 0; idx < CB * LX; idx++) sb[idx] = __longlong_as_double(-1LL);
+  };
   auto wait_flag = [&](int bj) {
     const uint64_t t0 = gtimer();
     while (ld_acquire(flags + bj) != epoch) {
-      if (gtimer() - t0 > 1000000000ull) { atomicExch(err, 1); break; }
+      if (gtimer() - t0 > 1000000000ull) { give_up(); break; }
     }
   };
   auto load_t = [&](int bj, double (&a)[CB / 4]) {
@@ -502,12 +514,12 @@ void trsv_w_dev(int uplo, int trans, int n, int nrhs, const T *A, long lda, cons
   const long tstr = tr ? lda : 1, tcol = tr ? 1 : lda;  // effective T(i,k) = A[i*tstr + k*tcol]
   const int lower = (uplo == kLower) != tr;
   const int nb = cdiv(n, CB);
-  // workspace: ticket counter, error word, flags, and (FP32) the tagged copy
+  // workspace: ticket counter, flags, and (FP32) the tagged copy
   // of x, 8 words per row
   const size_t nctl = (size_t)cdiv(nb + 64, 2) * 2, ntag = sizeof(T) == 4 ? (size_t)nb * CB * 8 : 0;
   int *ctl = (int *)scratch(kSlotTrsvCtl, sizeof(int) * nctl + sizeof(unsigned long long) * ntag);
   const int epoch = 1;
-  int *counter = ctl, *err = ctl + 1, *flags = ctl + 64;
+  int *counter = ctl, *flags = ctl + 64, *word = wait_word();
   unsigned long long *xt = (unsigned long long *)(ctl + nctl);
   ATLB_CUDA_CHECK(cudaMemsetAsync(ctl, 0, sizeof(int) * nctl + sizeof(unsigned long long) * ntag, st));
   // sW, sxd, sb, sacc (trsv_kernel's layout), for the largest NR
@@ -522,9 +534,9 @@ void trsv_w_dev(int uplo, int trans, int n, int nrhs, const T *A, long lda, cons
         configured_m = true;
       }
       if (nrhs <= 8)
-        trsv_mma_kernel<1><<<nb, TT, smem1, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, err);
+        trsv_mma_kernel<1><<<nb, TT, smem1, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, word);
       else
-        trsv_mma_kernel<2><<<nb, TT, smem2, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, err);
+        trsv_mma_kernel<2><<<nb, TT, smem2, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, word);
       ATLB_CUDA_CHECK(cudaGetLastError());
       return;
     }
@@ -539,7 +551,7 @@ void trsv_w_dev(int uplo, int trans, int n, int nrhs, const T *A, long lda, cons
     configured = true;
   }
   auto go = [&](auto kern) {
-    kern<<<nb, TT, smem, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, err, xt);
+    kern<<<nb, TT, smem, st>>>(n, nrhs, A, tstr, tcol, lower, W, B, ldb, counter, flags, epoch, word, xt);
   };
   if constexpr (sizeof(T) == 8) go(trsv_kernel<T, 1>);
   else if (nrhs == 1) go(trsv_kernel<T, 1>);

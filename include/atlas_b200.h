@@ -189,6 +189,13 @@ int atlb_last_cuda_error(void);
 void *atlb_get_stream(void);
 void atlb_set_stream(void *stream);
 int atlb_sync(void);
+/* Waits between a kernel's blocks are bounded (1 to 4 s).  One that gives up sets
+ * the calling thread's word (host memory, 1 set, 0 clear) and marks its results:
+ * LU by *dinfo > 0, the solves and QR by NaN.  The thread's next synchronising call
+ * (atlb_sync, or any entry point that returns results in host memory) reports it:
+ * it prints a message, clears the word, records cudaErrorLaunchTimeout for
+ * atlb_last_cuda_error(), and returns it unless it has an info value to return. */
+int *atlb_wait_word(void);
 
 /* Device-pointer variants: column-major, all pointers in device memory,
  * enqueued on the library stream and NOT synchronised.  Integer arguments

@@ -549,3 +549,26 @@ def test_replayed_factorizations_follow_the_memory_behind_an_address(gpu, kind):
         _ok(d.cuMemRelease(handle))
         assert own == device
     _ok(d.cuMemAddressFree(addr, size))
+
+
+def test_a_wait_that_gave_up_is_reported_by_the_next_synchronization(gpu, orc):
+    """The word that a kernel sets, set here: the synchronising call after it returns
+    cudaErrorLaunchTimeout, unless it has an info value to return, and clears it."""
+    import ctypes
+    timeout = 702
+    word = ctypes.cast(AB.atlb_wait_word(), ctypes.POINTER(ctypes.c_int))
+    assert word[0] == 0 and AB.atlb_sync() == 0
+    n = 40
+    a, tau, ipiv = orc.lu_matrix(n, 3), np.zeros(n), np.zeros(n, dtype=np.int32)
+    b = np.asfortranarray(np.ones((n, 1)))
+    singular = np.zeros((n, n), order="F")
+    calls = [(AB.atlb_sync, timeout),
+             (lambda: AB.ATL_dgeqrf(n, n, a.copy(order="F"), n, tau, None, 0), timeout),
+             (lambda: AB.clapack_dgesv(CM, n, 1, a.copy(order="F"), n, ipiv, b.copy(order="F"), n), timeout),
+             (lambda: AB.clapack_dpotrf(CM, 122, n, np.asfortranarray(np.eye(n)), n), timeout),
+             (lambda: AB.clapack_dgetrf(CM, n, n, singular, n, ipiv), 1)]
+    for call, want in calls:
+        word[0] = 1
+        assert call() == want
+        assert word[0] == 0 and AB.atlb_last_cuda_error() == timeout
+        assert AB.atlb_sync() == 0
