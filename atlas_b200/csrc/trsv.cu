@@ -251,11 +251,14 @@ trsv_kernel(int n, int nrhs, const T *__restrict__ Tp, long tr, long tc, int low
 // the wait.  Two groups of columns share every fragment of T and the chain's
 // latency, hence up to 16 per launch: 8192^2, 16 right-hand sides, one
 // direction 472 us; with FMAs, eight at a time, 2 x 860.  The step is bound by
-// its latency, so even one right-hand side, with seven of the eight columns
-// zero, is faster than with FMAs: both directions of 8192^2 in 764 us for 1..4
-// right-hand sides (FMAs: 1 one 1054, 2..4 1266), of 3000^2 in 298 (358, 436),
-// of 1000^2 in 144 (157, 183).  Only one right-hand side over one or two blocks,
-// where nothing chains, keeps the FMAs (200^2: 80.7 us, here 84.4).
+// its latency, so 1..4 right-hand sides, with most of the eight columns zero,
+// take it too: both directions of 8192^2 in 764 us (FMAs: 2..4 1266), of 3000^2 in
+// 298 (436), of 1000^2 in 144 (183).  One right-hand side keeps the FMAs where a
+// column of T is contiguous in memory: their lanes run down it, while the fragments
+// take eight rows of four columns (getrs, both factors, without transposition, 8192^2:
+// 1106 us here, 862 with FMAs, 2000^2 304 and 249, 400^2 122 and 111; transposed 1096
+// here and 1970 with FMAs, 307 and 503, 123 and 178), and over one or two blocks, where
+// nothing chains (200^2: 80.7 us, here 84.4).
 template <int NH>
 __global__ void __launch_bounds__(TT, 1)
 trsv_mma_kernel(int n, int nrhs, const double *__restrict__ Tp, long tr, long tc, int lower,
@@ -525,7 +528,7 @@ void trsv_w_dev(int uplo, int trans, int n, int nrhs, const T *A, long lda, cons
   // sW, sxd, sb, sacc (trsv_kernel's layout), for the largest NR
   constexpr int smem = (CB * (CB + 1) + (2 * CB + CB + NQ * CB) * 8) * (int)sizeof(T);
   if constexpr (sizeof(T) == 8) {
-    if (nrhs > 1 || n > 2 * CB) {
+    if (nrhs > 1 || (n > 2 * CB && tstr != 1)) {
       constexpr int smem1 = (CB * (CB + 4) + 3 * CB * 12) * 8, smem2 = (CB * (CB + 4) + 3 * CB * 20) * 8;
       static bool configured_m = false;
       if (!configured_m) {
