@@ -77,11 +77,15 @@ __device__ __forceinline__ unsigned long long swap2(unsigned long long x) {
 // rows.  4096^3: 3.17 ms with 8 x 8 outputs and single products, 2.76 ms
 // now.
 //
-// Outputs of fewer 128 x 128 tiles than SMs take 64 x 64 ones (T = 64, 4 x 8 outputs a
+// Outputs of few 128 x 128 tiles take 64 x 64 ones (T = 64, 4 x 8 outputs a
 // thread): four times the CTAs, and four warps' latency per tile a quarter as
 // long.  With C read back, 128 x 128 tiles of 8 x 8 outputs and these: 128^3 23.1 and
-// 9.0 us, 2000 x 128 x 128 26.9 and 10.7, 1000^3 140 and 75, 1500 x 1200 x 900 (120
-// tiles) 128 and 122.
+// 9.0 us, 2000 x 128 x 128 26.9 and 10.7, 1000^3 140 and 75.  The line is at three
+// small tiles an SM (111 large ones): with four, an SM is no sooner done than with
+// one large tile.  Time with large tiles over that with small ones, K = 1000, A and B
+// as they are / A transposed: 1.19 / 1.05 at 100 and 110 tiles, 0.91 / 0.81 at 121 to 144.
+// Up to K = 128, where a tile's start and end count most, the small ones stay ahead
+// to the last (121 tiles, K = 32 1.21 / 1.00, 128 1.00 / 0.91, unaligned 1.34 and 1.21).
 template <int T, bool TA, bool TB, bool VA, bool VB>
 __global__ void __launch_bounds__(THREADS, 2)
 sgemm_simt_kernel(int M, int N, int K, float alpha, const float *__restrict__ A, long lda,
@@ -313,7 +317,8 @@ void sgemm_dev(int ta, int tb, int M, int N, int K, float alpha, const float *A,
       else go(sgemm_simt_kernel<T, true, true, false, false>, set[8]);
     }
   };
-  if (S == 1 && tiles < num_sms()) with(std::integral_constant<int, 64>{});
+  const bool few = 4 * tiles <= 3 * num_sms() || (K <= 128 && tiles < num_sms());
+  if (S == 1 && few) with(std::integral_constant<int, 64>{});
   else with(std::integral_constant<int, BT>{});
   ATLB_CUDA_CHECK(cudaGetLastError());
   if (S > 1) {

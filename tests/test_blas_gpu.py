@@ -239,10 +239,11 @@ def test_dgemm_whole_tiles_by_bulk_copy(gpu, m, n, k, beta, pinned):
 
 @pytest.mark.parametrize("ta,tb", [(111, 111), (111, 112), (112, 111), (112, 112)])
 @pytest.mark.parametrize("m,n,k,pad", [(1, 1, 1, 0), (63, 65, 17, 1), (64, 64, 16, 0), (65, 132, 33, 3), (128, 256, 128, 0),
-                                       (500, 708, 300, 0), (1500, 1200, 40, 0), (1664, 1537, 20, 1)])
+                                       (500, 708, 300, 0), (1500, 1200, 40, 0), (1664, 1537, 20, 1),
+                                       (4730, 300, 130, 0), (4737, 300, 130, 1), (1400, 1290, 128, 0), (1400, 1290, 129, 0)])
 def test_sgemm_few_tiles(gpu, ta, tb, m, n, k, pad):
-    """64 x 64 tiles (fewer 128 x 128 tiles than SMs) and the first size beyond:
-    sizes around the tiles, aligned and unaligned columns; |C - C_ref| <=
+    """64 x 64 tiles (up to 111 tiles of 128 x 128, 147 up to K = 128) and the first
+    sizes beyond: sizes around the tiles, aligned and unaligned columns; |C - C_ref| <=
     (k + 3) u (|alpha||A||B| + |beta||C|) componentwise with FP32's u, against
     FP64."""
     rng = np.random.default_rng(m + n + k)
