@@ -137,7 +137,7 @@ template <int BNT> struct TileCfg {
 // ahead for longer (8192^2 x 320 with C read back: 31.5 TFLOP/s wide, 33.5 narrow;
 // x 512 33.0 and 34.1, 2048^2 x 512 28.3 and 28.7; at 640 on 2048^2 29.4 and 29.1)
 constexpr int SMALL_K = 256, SMALL_K_BULK = 512;
-constexpr int SMALL_TILE_K = 512;  // K up to this, with few tiles, uses 64 x 64 or 32 x 32 tiles
+constexpr int SMALL_TILE_K = 512;  // K up to this, with few tiles, uses 32 x 32 or 64 x 64 tiles
 // the grouped (batched) GEMM's tile width: its problems are small (K <= 512,
 // M, N from 16), where the narrower tile wastes less on padding and two CTAs
 // per SM overlap their epilogues
@@ -383,8 +383,8 @@ dgemm_dmma_kernel(int M, int N, int K, double alpha, const double *__restrict__ 
 
 // GEMMs whose output has too few 128 x 128 tiles for the SMs and whose K is
 // short (the small updates inside the factorizations, a user's small
-// products): BT x BT tiles (64, or 32 when even those are fewer than the SMs),
-// four warps, old C fetched into registers before the main loop.  Split K
+// products): BT x BT tiles (32, or 64 for many of them without alignment), four
+// warps, old C fetched into registers before the main loop.  Split K
 // needs a second launch and a round trip of the partials through memory,
 // which is most of the time of such a product.  Against split K (device time,
 // launches included): 128^3 14.4 -> 7.5 us, 96 x 80 x 112 16.2 -> 8.9,
@@ -620,11 +620,17 @@ void launch(int M, int N, int K, double alpha, const double *A, long lda, const 
   }
   int tiles = cdiv(M, BM) * cdiv(N, BN);
   const int nsm = num_sms();
-  // too few tiles for the 148 SMs: smaller tiles while K is short, else split
-  // K (partials + reduction).  At K = 500 the two are level on few tiles
-  // (300 x 300: 16.5 us both ways) and the smaller tiles ahead on many; beyond,
-  // the serial K loop of one tile is the longer.
-  if (tiles * 2 <= nsm && K <= SMALL_TILE_K) {
+  // Too few tiles for the 148 SMs: smaller tiles while K is short, else split K
+  // (partials + reduction).  Where an SM has one 32 x 32 tile or less, that tile's
+  // serial K loop becomes the longer towards K = 512, without alignment from 450 on
+  // (200 x 200 with C read back, split and small: K = 400 16.6 and 12.5 us, 450 16.6 and
+  // 14.5, 512 14.6 and 14.5, A transposed 14.6 and 16.6; unaligned 16.6 and 14.6, 16.6
+  // and 16.6, 14.6 and 17.4).  With more tiles than SMs the small ones are ahead at 512
+  // too (500 x 500 20.7 and 17.6, 800 x 800 43.3 and 35.0).
+  const long t32 = (long)cdiv(M, 32) * cdiv(N, 32), t64 = (long)cdiv(M, 64) * cdiv(N, 64);
+  const bool can_split = tune(kTuneSplitK) && !no_alloc_active();
+  const int most_k = !can_split || t32 > nsm ? SMALL_TILE_K : VEC == 2 ? 480 : 400;
+  if (tiles * 2 <= nsm && K <= most_k) {
     auto go = [&](auto kern, int bt, int bytes, bool &set) {
       if (!set) {
         ATLB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
@@ -634,13 +640,24 @@ void launch(int M, int N, int K, double alpha, const double *A, long lda, const 
       kern<<<cdiv(M, bt) * cdiv(N, bt), SM_THREADS, bytes, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, tri);
       ATLB_CUDA_CHECK(cudaGetLastError());
     };
-    static bool set64 = false, set32 = false;
-    if (cdiv(M, 64) * cdiv(N, 64) >= nsm) go(dgemm_small_kernel<TA, TB, VEC, 64>, 64, small_smem<TA, TB, 64>(), set64);
-    else go(dgemm_small_kernel<TA, TB, VEC, 32>, 32, small_smem<TA, TB, 32>(), set32);
+    // 64 x 64 tiles cost four of 32 x 32 each and leave more of the last wave idle
+    // (800 x 800 x 512, 169 tiles: 47.4 us, 32 x 32 35.1).  With 16-byte copies the small
+    // ones are ahead throughout (1000^2 x 512 47.2 and 51.4); with 8-byte copies, which
+    // cost them 1.25 times as much, where the waves say so (1000^2 x 512 59.6 and 53.5,
+    // 900^2 47.3 and 53.4).
+    if constexpr (VEC == 1) {
+      if (t64 >= nsm && 16 * cdiv(t64, nsm) <= 5 * cdiv(t32, nsm)) {
+        static bool set64 = false;
+        go(dgemm_small_kernel<TA, TB, VEC, 64>, 64, small_smem<TA, TB, 64>(), set64);
+        return;
+      }
+    }
+    static bool set32 = false;
+    go(dgemm_small_kernel<TA, TB, VEC, 32>, 32, small_smem<TA, TB, 32>(), set32);
     return;
   }
   int S = 1;
-  if (tune(kTuneSplitK) && tiles * 2 <= nsm && K >= 4 * BK && !no_alloc_active()) S = splitk_count(tiles, K, nsm);
+  if (can_split && tiles * 2 <= nsm && K >= 4 * BK) S = splitk_count(tiles, K, nsm);
   if (S > 1) {
     const int kc = cdiv(cdiv(K, S), BK) * BK;
     S = cdiv(K, kc);

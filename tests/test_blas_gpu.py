@@ -192,10 +192,11 @@ def test_syrk_golden_cases(gpu, orc, gold):
 @pytest.mark.parametrize("ta,tb", [(111, 111), (111, 112), (112, 111), (112, 112)])
 @pytest.mark.parametrize("m,n,k,pad", [(1, 1, 1, 0), (31, 33, 7, 1), (32, 32, 16, 0), (33, 31, 17, 0), (64, 96, 48, 1),
                                        (96, 80, 112, 0), (700, 640, 512, 0), (700, 640, 513, 1), (513, 65, 300, 1),
-                                       (1665, 1700, 529, 1), (1664, 1666, 528, 0)])
+                                       (1665, 1700, 529, 1), (1664, 1666, 528, 0), (250, 300, 480, 0), (250, 300, 481, 0),
+                                       (250, 301, 400, 1), (250, 301, 401, 1), (1000, 1000, 60, 0), (999, 1000, 60, 1)])
 def test_dgemm_few_tiles(gpu, ta, tb, m, n, k, pad):
-    """Products with few output tiles (32 x 32 and 64 x 64 tiles up to K = 512,
-    split K above; 128 x 64 where 128 x 128 ones leave much of the last wave idle): sizes around the tiles and the K steps, aligned and
+    """Products with few output tiles (32 x 32 and 64 x 64 tiles up to K = 512, 400 or
+    480 with one tile an SM or less, split K above; 128 x 64 where 128 x 128 ones leave much of the last wave idle): sizes around the tiles and the K steps, aligned and
     unaligned leading dimensions; |C - C_ref| <= (k + 3) u (|alpha||A||B| + |beta||C|)
     componentwise, doubled for the reference's own rounding."""
     rng = np.random.default_rng(m + n + k)
