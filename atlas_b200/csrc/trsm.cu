@@ -339,17 +339,20 @@ void eff_update(const Eff<T> &e, int r2, int n2, int r1, int n1, int m, SgemmFn 
   const T *T21 = e.Tp + r2 * e.tr + r1 * e.tc;
   T *B2 = e.Bp + r2 * e.br;
   const T *X1 = e.Bp + r1 * e.br;
-  const bool small = n1 <= SK_K && n2 <= 2 * SK_T;  // the coupling product of an order <= 128 solve
+  // the coupling product of an order <= 128 solve (FP32 only: the FP64 recursion ends there)
+  const bool small = sizeof(T) == 4 && n1 <= SK_K && n2 <= 2 * SK_T;
   if (e.br == 1) {  // B column-major (ld = bc)
     int ta = (e.tr == 1) ? kNoTrans : kTrans;
     long ldt = (e.tr == 1) ? e.tc : e.tr;
-    if (small) gemm_smallk<T>(ta, kNoTrans, n2, m, n1, T21, ldt, X1, e.bc, B2, e.bc, st);
-    else gemm_call<T>(fn, ta, kNoTrans, n2, m, n1, T(-1), T21, ldt, X1, e.bc, T(1), B2, e.bc, st);
+    if constexpr (sizeof(T) == 4)
+      if (small) return gemm_smallk<T>(ta, kNoTrans, n2, m, n1, T21, ldt, X1, e.bc, B2, e.bc, st);
+    gemm_call<T>(fn, ta, kNoTrans, n2, m, n1, T(-1), T21, ldt, X1, e.bc, T(1), B2, e.bc, st);
   } else {  // B^T column-major (m x n) with ld = br: B2^T -= X1^T * T21^T
     int tb = (e.tc == 1) ? kNoTrans : kTrans;
     long ldt = (e.tc == 1) ? e.tr : e.tc;
-    if (small) gemm_smallk<T>(kNoTrans, tb, m, n2, n1, X1, e.br, T21, ldt, B2, e.br, st);
-    else gemm_call<T>(fn, kNoTrans, tb, m, n2, n1, T(-1), X1, e.br, T21, ldt, T(1), B2, e.br, st);
+    if constexpr (sizeof(T) == 4)
+      if (small) return gemm_smallk<T>(kNoTrans, tb, m, n2, n1, X1, e.br, T21, ldt, B2, e.br, st);
+    gemm_call<T>(fn, kNoTrans, tb, m, n2, n1, T(-1), X1, e.br, T21, ldt, T(1), B2, e.br, st);
   }
 }
 
@@ -361,12 +364,18 @@ void eff_update(const Eff<T> &e, int r2, int n2, int r1, int n1, int m, SgemmFn 
 // the recursion below 256 (inverse times 64 rows, a coupling product, the next
 // inverse) took three launches and 66 us for an order of 128 and 8000 columns,
 // this takes 24.
-constexpr int TBK_N = 256;
+// With more columns than two CTAs of 64 an SM, what counts is no longer one CTA's
+// latency but how many share an SM: order <= 128 takes CTAs of 32 columns, two an SM,
+// and larger orders go through the recursion down to that (order 128, 100,000
+// columns: 220 us with 64 columns and one CTA an SM, 181 now; order 65 220 and 158,
+// order 256 598 and 469; the recursion to 64 rows took 218, 201 and 577).  At order <= 64
+// 64 columns have room twice and stay (100,000: 68 us, with 32 columns 73).
+constexpr int TBK_N = 256, TBK_WIDE_N = 128;
 template <int CT>
 constexpr int tri_block_smem(int n) { return 8 * ((n + LEAF - 1) / LEAF * LEAF * (CT + 4) + 2 * LEAF * (LEAF + 4)); }
 
 template <int CT>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(256, CT == 32 ? 2 : 1)
 tri_block_kernel(int n, int m, const double *__restrict__ Tp, long tr, long tc, int lower,
                  const double *__restrict__ W, double *__restrict__ Bp, long br, long bc) {
   // 4 (mod 16) doubles: the MMA's 8 x 4 fragments fall in distinct banks
@@ -430,7 +439,12 @@ tri_block_kernel(int n, int m, const double *__restrict__ Tp, long tr, long tc, 
         }
       }
       const double *X = sB + block(u) * LEAF * LB + t * LB + c0 + g;
-      const int k0 = u == s && !lower ? r0 : 0, k1 = u == s && lower ? r0 + 16 : LEAF;
+      const int k0 = u == s && !lower ? r0 : 0;
+      // CT = 32: nothing for rows and columns past the order
+      const int k1 = CT == 32 && ib * LEAF + r0 >= n ? 0
+                     : u == s && lower               ? r0 + 16
+                     : CT == 32                      ? min(LEAF, (n - block(u) * LEAF + 3) / 4 * 4)
+                                                     : LEAF;
 #pragma unroll 4
       for (int k = k0; k < k1; k += 4) {
         double a[2], b[NW];
@@ -480,10 +494,12 @@ template <typename T>
 void eff_solve(const Eff<T> &e, int r0, int n, int m, SgemmFn fn, cudaStream_t st) {
   if (n <= 0 || m <= 0) return;
   if constexpr (sizeof(T) == 8) {
-    if (n <= TBK_N) {
+    const bool wide = cdiv(m, 64) > 2 * num_sms();
+    if (n <= (wide ? TBK_WIDE_N : TBK_N)) {
       const double *Td = e.Tp + r0 * e.tr + r0 * e.tc, *Wd = e.W + (long)(r0 / LEAF) * LEAF * LEAF;
       // 16 columns a CTA while 64 would leave most SMs idle
       if (cdiv(m, 64) * 2 <= num_sms()) tri_block_launch<16>(n, m, Td, e.tr, e.tc, e.lower, Wd, e.Bp + r0 * e.br, e.br, e.bc, st);
+      else if (wide && n > LEAF) tri_block_launch<32>(n, m, Td, e.tr, e.tc, e.lower, Wd, e.Bp + r0 * e.br, e.br, e.bc, st);
       else tri_block_launch<64>(n, m, Td, e.tr, e.tc, e.lower, Wd, e.Bp + r0 * e.br, e.br, e.bc, st);
       return;
     }

@@ -275,3 +275,31 @@ def test_dsyrk_few_tiles(gpu, uplo, n, k):
     mag = np.abs(a) @ np.abs(a.T) + np.abs(c0)
     assert np.all((np.abs(c - (c0 - a @ a.T)) <= 2 * (k + 3) * 2.0 ** -53 * mag)[part])
     assert np.array_equal(c[~part], c0[~part])
+
+
+@pytest.mark.parametrize("m", [18944, 18945, 19100])
+@pytest.mark.parametrize("n", [16, 64, 65, 100, 128, 129, 200, 256, 300])
+def test_dtrsm_many_columns(gpu, n, m):
+    """Solves around the number of columns from which CTAs of 32 columns and an
+    order of at most 128 take over, all sides and triangles: |T X - B| <= 2 (n + 64) u
+    (|T||T^-1||T||X| + |T||X|) componentwise, for the inverted 64 x 64 diagonal tiles
+    and the check's own product."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n + m)
+    u = 2.0 ** -53
+    t = (torch.rand(n, n, generator=g, dtype=torch.float64, device="cuda") * 2 - 1) / n ** 0.5
+    t += 2 * torch.eye(n, dtype=torch.float64, device="cuda")
+    for side in (141, 142):
+        b0 = torch.rand(*((m, n) if side == 141 else (n, m)), generator=g, dtype=torch.float64, device="cuda") * 2 - 1
+        for uplo in (121, 122):
+            for trans in (111, 112):
+                b = b0.clone()
+                assert AB.atlb_dtrsm_dev(side, uplo, trans, 131, *((n, m) if side == 141 else (m, n)), 1.0, t, n, b,
+                                         n if side == 141 else m) == 0
+                T = torch.triu(t.T) if uplo == 121 else torch.tril(t.T)
+                T = T if trans == 111 else T.T
+                X, B = (b.T, b0.T) if side == 141 else (b, b0)      # T X = B or X^T T = B^T
+                T = T if side == 141 else T.T
+                aT, aX = T.abs(), X.abs()
+                mag = aT @ (torch.linalg.inv(T).abs() @ (aT @ aX) + aX)
+                assert bool(((T @ X - B).abs() <= 2 * (n + 64) * u * mag).all()), (side, uplo, trans)
