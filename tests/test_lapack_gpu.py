@@ -420,6 +420,34 @@ def test_geqrf_lookahead_shapes_vs_oracle(gpu, orc, m, n):
     assert orc.resid_qr(a0, a.copy(order="F"), tau) <= 100.0
 
 
+@pytest.mark.parametrize("m,n", [(300, 70), (2048, 70), (2049, 70), (4097, 33), (8193, 40), (16384, 20),
+                                 (16385, 20), (40000, 10)])
+def test_geqrf_panel_rows_and_reflectors_that_vanish(gpu, orc, m, n):
+    """Rows around the limits of a panel's CTAs and of its rows a thread; random
+    columns, zero columns at the start, in the middle and at the end of a leaf, and
+    leading columns that are triangular already: tau = 0 there, R, V and tau the
+    oracle's, and |A - QR| <= m n u |A| (Higham, theorem 19.4)."""
+    for kind in ("random", "zero", "triangular"):
+        a0 = orc.normal((m, n), 5 * m + n)
+        if kind == "zero":
+            a0[:, [c for c in (0, 7, 15, 16, 31, 32, 47, n - 1) if c < n]] = 0.0
+        if kind == "triangular":
+            a0[:, :n // 2] = np.triu(a0[:, :n // 2])
+        a = a0.copy(order="F")
+        tau = np.zeros(n)
+        assert AB.clapack_dgeqrf(CM, m, n, a, m, tau) == 0
+        qr, rtau = orc.dgeqrf(a0.copy(order="F"))
+        np.testing.assert_array_equal(tau == 0.0, rtau == 0.0)
+        np.testing.assert_allclose(tau, rtau, rtol=1e-9, atol=1e-11)
+        np.testing.assert_allclose(np.triu(a), np.triu(qr), rtol=1e-9, atol=1e-10)
+        np.testing.assert_allclose(np.tril(a, -1), np.tril(qr, -1), rtol=1e-8, atol=1e-10)
+        back = np.triu(a)
+        for c in range(n - 1, -1, -1):
+            v = np.concatenate([[1.0], a[c + 1:, c]])
+            back[c:] -= tau[c] * np.outer(v, v @ back[c:])
+        assert np.linalg.norm(back - a0) <= m * n * 2.0 ** -53 * np.linalg.norm(a0)
+
+
 @pytest.mark.parametrize("n", [129, 300, 513])
 @pytest.mark.parametrize("uplo", [121, 122])
 def test_potrf_lookahead_sizes_vs_oracle(gpu, orc, n, uplo):
