@@ -192,23 +192,27 @@ def test_batched_gesv_panel_edges(gpu, orc, nrhs):
 
 
 def test_batched_gesv_singular(gpu):
-    """A zero column, a zero matrix and a repeated row: the first zero pivot's
-    position, the factorization completed, the right-hand side untouched."""
+    """A zero column, a zero matrix and a row repeated in a matrix whose elimination
+    is exact (entries 0 and +-1, pivots of +-1): the first zero pivot's position, the
+    factorization completed, the right-hand side untouched."""
     import torch
     n = 40
     rng = np.random.default_rng(3)
-    a = [rng.uniform(-1, 1, (n, n)) for _ in range(3)]
+    a = [rng.uniform(-1, 1, (n, n)), np.zeros((n, n)), None]
     a[0][17] = 0.0                                     # column 17 (stored as a row)
-    a[1][:] = 0.0
+    rep = np.triu(rng.integers(-1, 2, (n, n)).astype(np.float64), 1) + np.eye(n)
+    rep[25] = rep[7]
+    a[2] = np.ascontiguousarray(rep.T)
     As = [torch.tensor(m, device="cuda") for m in a] + [torch.eye(n, dtype=torch.float64, device="cuda")]
     Bs = [torch.ones(1, n, dtype=torch.float64, device="cuda") for _ in As]
     Ps = [torch.zeros(n, dtype=torch.int32, device="cuda") for _ in As]
     ns, one = _int_array([n] * 4), _int_array([1] * 4)
     info = np.zeros(4, dtype=np.int32)
     assert AB.atlb_dgesv_batched(4, ns, _ptr_array(As), ns, _ptr_array(Ps), _ptr_array(Bs), ns, one, info) == 0
-    assert list(info) == [18, 1, 0, 0]
+    _, _, rinfo = O.dgetrf(np.asfortranarray(rep))
+    assert list(info) == [18, 1, rinfo, 0] and rinfo == 26
     assert np.array_equal(Ps[1].cpu().numpy(), np.arange(n)) and np.array_equal(Ps[3].cpu().numpy(), np.arange(n))
-    for k in (0, 1):
+    for k in (0, 1, 2):
         assert np.all(Bs[k].cpu().numpy() == 1.0)
     assert np.all(np.isfinite(As[0].cpu().numpy()))
 
@@ -267,41 +271,34 @@ def test_batched_dgemm_uneven(gpu, orc):
         assert orc.resid_gemm(111, 111, int(M[i]), int(N[i]), int(K[i]), 1.5, a, b, -0.5, c0, c) < 50
 
 
-@pytest.mark.parametrize("small,pw", [(96, 32), (128, 16), (64, 64)])
-def test_batched_posv_buckets_and_graph_replays(gpu, small, pw):
-    """Every size bucket setting of the tuner gives the same solves, and the
-    third and later calls of one batch shape (replayed from a CUDA graph) solve
-    the new data each call carries."""
+@pytest.mark.parametrize("edges", [(48, 49), (112, 113), (176, 177)])
+def test_batched_posv_graph_replays(gpu, edges):
+    """Batches with orders on both sides of a size bucket's edge: the third and
+    later calls of one batch shape (replayed from a CUDA graph) solve the new data
+    each call carries."""
     import torch
-    old = (AB.atlb_tune_get("batch_posv_small"), AB.atlb_tune_get("batch_posv_pw"))
-    AB.atlb_tune_set("batch_posv_small", small)
-    AB.atlb_tune_set("batch_posv_pw", pw)
-    try:
-        rng = np.random.default_rng(small + pw)
-        count, nr = 64, 2
-        ns = rng.integers(8, 257, count)
-        ns[:4] = [small, small + 1, 8, 256]
-        for call in range(4):
-            As, Bs, a0s, b0s = [], [], [], []
-            for n in ns:
-                g = rng.standard_normal((n, n))
-                a = g @ g.T + n * np.eye(n)
-                b = rng.uniform(-1, 1, (n, nr))
-                a0s.append(a)
-                b0s.append(b)
-                As.append(torch.tensor(a, device="cuda"))            # symmetric: either order
-                Bs.append(torch.tensor(np.ascontiguousarray(b.T), device="cuda"))
-            info = np.zeros(count, dtype=np.int32)
-            assert AB.atlb_dposv_batched(count, _int_array(ns), _ptr_array(As), _int_array(ns), _ptr_array(Bs),
-                                         _int_array(ns), _int_array([nr] * count), info) == 0
-            assert np.all(info == 0)
-            for i in range(count):
-                x = Bs[i].cpu().numpy().T
-                res = np.abs(a0s[i] @ x - b0s[i]).max() / (np.abs(a0s[i]).sum(1).max() * np.abs(x).max())
-                assert res < 1e-14, (call, i, ns[i], res)
-    finally:
-        AB.atlb_tune_set("batch_posv_small", old[0])
-        AB.atlb_tune_set("batch_posv_pw", old[1])
+    rng = np.random.default_rng(edges[1])
+    count, nr = 64, 2
+    ns = rng.integers(8, 257, count)
+    ns[:4] = [*edges, 8, 256]
+    for call in range(4):
+        As, Bs, a0s, b0s = [], [], [], []
+        for n in ns:
+            g = rng.standard_normal((n, n))
+            a = g @ g.T + n * np.eye(n)
+            b = rng.uniform(-1, 1, (n, nr))
+            a0s.append(a)
+            b0s.append(b)
+            As.append(torch.tensor(a, device="cuda"))            # symmetric: either order
+            Bs.append(torch.tensor(np.ascontiguousarray(b.T), device="cuda"))
+        info = np.zeros(count, dtype=np.int32)
+        assert AB.atlb_dposv_batched(count, _int_array(ns), _ptr_array(As), _int_array(ns), _ptr_array(Bs),
+                                     _int_array(ns), _int_array([nr] * count), info) == 0
+        assert np.all(info == 0)
+        for i in range(count):
+            x = Bs[i].cpu().numpy().T
+            res = np.abs(a0s[i] @ x - b0s[i]).max() / (np.abs(a0s[i]).sum(1).max() * np.abs(x).max())
+            assert res < 1e-14, (call, i, ns[i], res)
 
 
 def test_batched_getrf_only_matches_oracle(gpu):
