@@ -1,6 +1,6 @@
 // Blocked Cholesky in shared memory, for one CTA of 256 threads: the FP32
 // potrf (chol.cu) factors its diagonal blocks with it (FP64: chol_tiles.cuh).
-// Also the FP64 MMA and the leading dimension shared by the batched LU.
+// Also the FP64 MMA of the other kernels.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -47,9 +47,8 @@ __device__ __forceinline__ void syrk_lower_update(int mt, int nc, int jb, const 
     }
 }
 
-// Leading dimension for an order-n matrix in shared memory: the smallest
-// value >= n that is 8 (mod 16), so that the 8 x 4 operand fragments of the
-// FP64 MMA below (lanes: 8 rows x 4 columns) fall in distinct banks.
+// Leading dimension for an order-n matrix in shared memory: the smallest value
+// >= n that is 8 (mod 16).
 __host__ __device__ constexpr int ld_for(int n) { return (n + 7) / 16 * 16 + 8; }
 
 // d += a b on one m8n8k4 FP64 tensor-core tile (PTX mma.m8n8k4 .f64
