@@ -49,7 +49,7 @@ struct Prob {
 // 10,000 problems of orders 8..256 (mean 132) with 4 right-hand sides, B200:
 // 17.5 ms before (panels in shared memory, the trailing matrix in L2, the
 // right-hand sides solved one after another with loads of L on the chain),
-// 3.4 ms now; the bytes of A and B would take 0.3 ms, the flops 0.5 ms.
+// 2.9 ms now; the bytes of A and B would take 0.3 ms, the flops 0.5 ms.
 template <int NT, int NBMAX>
 struct PosvSmem {
   cholt::Shared<NBMAX> S;
@@ -112,7 +112,7 @@ batched_posv_kernel(const Prob *__restrict__ probs, const int *__restrict__ orde
 // 10,000 problems of orders 8..256 with one right-hand side, B200: getrf and
 // getrs kernels 14.5 + 3.0 ms before (two barriers and a shared-memory rank-1
 // update per column, interchanges and U12 as separate passes, a solve with
-// loads of the factor on its chain), 9.7 ms now for both.
+// loads of the factor on its chain), 9.6 ms now for both.
 constexpr int LU_RHS = 8;       // right-hand sides carried along
 constexpr int DLD = LPW + 1;
 
